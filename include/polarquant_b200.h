@@ -128,7 +128,9 @@ int pq_compress_rows_dynamic(const void* x, int64_t n_rows, int64_t tokens_per_r
  * wait for a tile copy gave up), bit 5 compress (pq_compress_rows_dynamic found its device-side
  * position out of range; nothing was written), bit 6 dequantise (a wait gave up), bit 7
  * pq_lse_exchange_merge (a peer's records did not arrive within about two seconds; the output rows of the
- * waiting CTAs are left unwritten).
+ * waiting CTAs are left unwritten), bit 8 the llama.cpp bridge's attention (a wait for a tile copy gave up),
+ * bit 9 the same kernel (shared-memory window unusable, nothing computed), bits 10 and 11 the same two of the
+ * bridge's compress.
  * The flags are cleared by the call.  No counterpart in the reference (its kernels report nothing). */
 int pq_poll_device_errors(unsigned int* flags_out);
 

@@ -1,0 +1,439 @@
+// Compress of the llama.cpp bridge's codec for head dims 64 and 128 and more than a few hundred vectors: rotate,
+// Euclidean norm, divide, nearest level of a device-side codebook, pack two indices per byte.
+//
+// The rotation is a [N x D] . [D x D] product of float32 operands.  On CUDA cores it is the bound (17 TFLOP at 2^20
+// vectors of 128: 0.5 ms at the FP32 peak); here it runs on the 5th-generation tensor cores with both operands as the
+// sum of three bfloat16 terms, which is exact for float32 (3 x 8 significant bits) and needs no range scaling.  Six of
+// the nine product terms are issued; the three left out are below 2^-24 of the product.  The correction terms go into
+// the accumulator before the leading one, so they are added while the accumulator is still small.
+//
+// A persistent CTA owns 128 vectors at a time:
+//   copy warp    boxes of 128 vectors x 32 floats by TMA (128-byte swizzle), a ring of them in flight;
+//   worker warps (4 per 32 dims) one thread = one vector x 32 dims: reads its row of the box, writes the three terms
+//                into tensor memory as the A operand (two buffers); one tile behind, reads its 32 accumulator columns
+//                and runs the float32 epilogue;
+//   MMA warp     6 x D/16 MMAs per tile (A from tensor memory, B = the three terms of R in shared memory), 3.1 K
+//                cycles at D = 128, which is what the tile's 74 KB take at the HBM's rate (3.2 K): the kernel is
+//                balanced between the two.
+// Index search: the reference scans the levels and keeps the first of the closest.  For a codebook in ascending order
+// that is "how many decision points lie below", with the decision points found once per CTA by bisection over the
+// float32 numbers; a coordinate's bucket (1/128 wide) holds at most one of them.  Any other codebook (unsorted, levels
+// closer than 1e-5, two decision points in a bucket) is scanned level by level as the reference does.
+// Measured (D = 128, 16 levels): 131 072 vectors 32 us = 2.36 TB/s of the 580 bytes a vector takes (the FP32 kernel before
+// it, R^T in shared memory: 226 us), 20 000 vectors 17 us (48.5).
+// All waits are bounded (bit 10 of pq_poll_device_errors).
+#include <cstring>
+
+#include "pq_bridge.cuh"
+#include "pq_tcgen05.cuh"
+
+namespace pq {
+
+static __device__ unsigned int g_bridge_compress_error = 0;
+
+constexpr int kBcVecs = 128;
+
+template <int D>
+struct BridgeCompressCfg {
+    static constexpr int WG = D / 32;
+    static constexpr int WORKERS = 128 * WG;                       // one thread per (vector, 32 dims)
+    static constexpr int THREADS = WORKERS + 64;                   // + MMA warp + copy warp
+    static constexpr uint32_t kBTerm = D * D * 2;                  // one bfloat16 term of R
+    static constexpr uint32_t kBox = kBcVecs * 32 * 4;             // 128 vectors x 32 floats
+    // A slot of the ring always serves the same 32 dims (a multiple of WG): its next box can then not be waited for
+    // before every thread that reads the slot has seen the previous one, which the parity waits rely on.
+    static constexpr int kBoxes = D == 128 ? 4 : 6;
+    static_assert(kBoxes % WG == 0, "a box slot belongs to one group of worker warps");
+    // Layout by absolute shared address: index table (257 buckets x 16 copies x 8 bytes; its address is an immediate of
+    // the lookups) | three terms of R | boxes | small buffers
+    static constexpr uint32_t kTabAddr = 4096;
+    static constexpr uint32_t kTabRows = 257;
+    static constexpr uint32_t kBAddr = (kTabAddr + kTabRows * 128 + 1023) & ~1023u;
+    static constexpr uint32_t kBoxAddr = (kBAddr + 3 * kBTerm + 1023) & ~1023u;
+    static constexpr uint32_t kSmallAddr = kBoxAddr + kBoxes * kBox;
+    static constexpr uint32_t kATerm = D / 2;                      // tensor-memory columns of one term
+    static constexpr uint32_t kABuf = 3 * kATerm;
+    static constexpr uint32_t kAcc = 2 * kABuf;
+    static constexpr uint32_t kTmemCols = D == 128 ? 512 : 256;
+    // norms [2][128][WG], codebook 16, decision points 16, barriers, tensor-memory slot, abort flag, fast flag
+    static constexpr uint32_t kSmall = 2 * kBcVecs * WG * 4 + 2 * 16 * 4 + (2 * kBoxes + 6) * 8 + 16;
+    static constexpr size_t smem_bytes() { return kSmallAddr + kSmall; }
+};
+
+// kind::f16 instruction descriptor with bfloat16 operands (both K-major), float32 accumulator, M = 128
+__host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) { return umma_idesc_f16(n) | (1u << 7) | (1u << 10); }
+
+__device__ __forceinline__ float2 bc_mul2(float2 a, float2 b) {
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;\n"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return d;
+}
+__device__ __forceinline__ float2 bc_fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
+          "l"(*reinterpret_cast<unsigned long long*>(&c)));
+    return d;
+}
+// two floats -> packed bfloat16 (first in the low half), and what the rounding left
+__device__ __forceinline__ uint32_t bc_term(float2& x) {
+    uint32_t w;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(w) : "f"(x.y), "f"(x.x));
+    const float2 neg = make_float2(__uint_as_float((w << 16) ^ 0x80000000u), __uint_as_float((w & 0xFFFF0000u) ^ 0x80000000u));
+    float2 r;
+    asm("add.rn.f32x2 %0, %1, %2;\n"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&r))
+        : "l"(*reinterpret_cast<unsigned long long*>(&x)), "l"(*reinterpret_cast<const unsigned long long*>(&neg)));
+    x = r;                                                          // exact
+    return w;
+}
+__device__ __forceinline__ void bc_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                 "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
+}
+// Bucket of a coordinate in bits 7..15: the unit in the last place of 128 v + 98432 is 2^-7, so those bits hold
+// floor(128 v + 128) after rounding to 1/128.  Monotone in v.
+__device__ __forceinline__ uint32_t bc_bucket_bits(float v) { return __float_as_uint(fmaf(v, 128.f, 98432.f)) & 0xFF80u; }
+// order-preserving integer image of a float and back
+__device__ __forceinline__ int bc_key(float x) {
+    const int b = __float_as_int(x);
+    return b >= 0 ? b : -(b & 0x7FFFFFFF);
+}
+__device__ __forceinline__ float bc_unkey(int k) {
+    return k >= 0 ? __int_as_float(k) : __uint_as_float((uint32_t)(-k) | 0x80000000u);
+}
+
+struct BridgeCompressParams {
+    const float* R;
+    const float* codebook;
+    float* radius_out;
+    uint8_t* packed_out;
+    int N, n_levels;
+};
+
+template <int D>
+__global__ void __launch_bounds__(BridgeCompressCfg<D>::THREADS, 1)
+bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUtensorMap x_map) {
+    using C = BridgeCompressCfg<D>;
+    constexpr int WG = C::WG, WORKERS = C::WORKERS, NB = C::kBoxes;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const uint32_t base = sm_addr(smem);
+    if (base > C::kTabAddr) {                                  // the window starts too high for the fixed layout
+        if (threadIdx.x == 0) atomicOr(&g_bridge_compress_error, 2u);
+        return;
+    }
+    uint8_t* zero = smem - base;                               // generic address of shared address 0
+    uint8_t* Bt = zero + C::kBAddr;
+    float* norm_s = reinterpret_cast<float*>(zero + C::kSmallAddr);          // [tile parity][vector][WG]
+    float* cb = norm_s + 2 * kBcVecs * WG;
+    float* thr = cb + 16;
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(thr + 16);
+    // [0, NB) box landed; [NB, 2 NB) box read; then A buffer 0 / 1 written; tile's MMAs done (per parity: frees the A
+    // buffer, completes the accumulator); accumulator read out (per parity)
+    uint64_t* box_full = mbar;
+    uint64_t* box_free = mbar + NB;
+    uint64_t* a_full = mbar + 2 * NB;
+    uint64_t* mma_done = a_full + 2;
+    uint64_t* acc_free = a_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_full + 6);
+    volatile uint32_t* abort_s = tmem_slot + 1;
+    uint32_t* fast_s = tmem_slot + 2;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // ---- set-up
+    if (tid == 0) {
+        for (int i = 0; i < NB; ++i) {
+            mbar_init(sm_addr(box_full + i), 1);
+            mbar_init(sm_addr(box_free + i), 128);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(sm_addr(a_full + i), WORKERS);
+            mbar_init(sm_addr(mma_done + i), 1);
+            mbar_init(sm_addr(acc_free + i), WORKERS);
+        }
+        *abort_s = 0u;
+        *fast_s = 1u;
+    }
+    if (tid < 16) cb[tid] = __ldg(p.codebook + min(tid, p.n_levels - 1));
+    // B: three bfloat16 terms of R, K-major core matrices (8 rows x 16 bytes), K chunks D / 8 * 128 bytes apart
+    for (int e = tid; e < D * (D / 8); e += C::THREADS) {
+        const int n = (e & 7) + 8 * (e / (8 * (D / 8))), kc = (e >> 3) % (D / 8);
+        float2 x[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) x[i] = __ldg(reinterpret_cast<const float2*>(p.R + (size_t)n * D + kc * 8) + i);
+        const uint32_t off = (uint32_t)(kc * (D / 8) * 128 + (n >> 3) * 128 + (n & 7) * 16);
+#pragma unroll
+        for (int t = 0; t < 3; ++t) {
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = bc_term(x[i]);
+            *reinterpret_cast<uint4*>(Bt + t * C::kBTerm + off) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    if (warp == 0) tmem_alloc(sm_addr(tmem_slot), C::kTmemCols);
+    __syncthreads();
+    // decision points: the largest v for which level i is at least as close as level i + 1 (both distances rounded to
+    // float32, as the scan rounds them)
+    if (tid < p.n_levels - 1) {
+        const float a = cb[tid], b = cb[tid + 1];
+        bool good = a > -1.f && b < 1.f && b - a > 1e-5f;
+        if (good) {
+            int lo = bc_key(a), hi = bc_key(b);                // holds at a, not at b
+            while (hi - lo > 1) {
+                const int mid = lo + (hi - lo) / 2;
+                const float v = bc_unkey(mid);
+                if (v - a <= b - v) lo = mid; else hi = mid;
+            }
+            thr[tid] = bc_unkey(lo);
+        }
+        if (!good) *fast_s = 0u;
+    }
+    __syncthreads();
+    if (tid + 1 < p.n_levels - 1 && bc_bucket_bits(thr[tid]) == bc_bucket_bits(thr[tid + 1])) *fast_s = 0u;
+    // a bucket's entry: its decision point (or a number no coordinate reaches) and the count of lower ones,
+    // replicated into every index field of a word
+    for (int e = tid; e < (int)C::kTabRows * 16; e += C::THREADS) {
+        const uint32_t bits = (uint32_t)(e >> 4) << 7;
+        float t = 3.0e38f;
+        uint32_t cnt = 0;
+        for (int i = 0; i < p.n_levels - 1; ++i) {
+            const uint32_t tb = bc_bucket_bits(thr[i]);
+            if (tb == bits) t = thr[i];
+            cnt += tb < bits ? 1u : 0u;
+        }
+        *reinterpret_cast<uint2*>(zero + C::kTabAddr + (e >> 4) * 128 + (e & 15) * 8) =
+            make_uint2(__float_as_uint(t), cnt * 0x11111111u);
+    }
+    fence_async_smem();                                        // B is read by the tensor core through the async proxy
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    const bool fast = *fast_s != 0u;
+    const int n_tiles = (p.N + kBcVecs - 1) / kBcVecs;
+    const int n_my = (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
+    bool ok = true;
+
+    if (warp == WORKERS / 32) {
+        // ---- MMA warp: every lane runs the loop, lane 0 issues
+        constexpr uint32_t idesc = umma_idesc_bf16(D);
+        constexpr uint32_t kLbo = (D / 8) * 128;
+        constexpr uint32_t b_hi = (128u >> 4) | (1u << 14);    // 8-row groups 128 B apart, no swizzle
+        const uint32_t b0 = ((C::kBAddr >> 4) & 0x3FFFu) | ((kLbo >> 4) << 16);
+        const uint32_t issue = lane == 0 ? 1u : 0u, acc = tmem_base + C::kAcc;
+        for (int i = 0; i < n_my && ok; ++i) {
+            const uint32_t b = i & 1, use = (uint32_t)i >> 1;
+            ok = mbar_wait(sm_addr(a_full + b), use & 1u, abort_s, 32) && ok;
+            if (i >= 1) ok = mbar_wait(sm_addr(acc_free + (b ^ 1)), (uint32_t)((i - 1) >> 1) & 1u, abort_s, 32) && ok;
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t a = tmem_base + b * C::kABuf;
+            // (term of x, term of R): the smallest products first
+            constexpr int ta[6] = {2, 0, 1, 1, 0, 0}, tb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+            for (int t = 0; t < 6; ++t)
+#pragma unroll
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_f16_ts_pred(acc, a + ta[t] * C::kATerm + ks * 8,
+                                     b0 + (uint32_t)((tb[t] * C::kBTerm + 2 * ks * kLbo) >> 4), b_hi, idesc,
+                                     (t || ks) ? 1u : 0u, issue);
+            umma_commit_pred(sm_addr(mma_done + b), issue);
+            __syncwarp();
+        }
+    } else if (warp == WORKERS / 32 + 1) {
+        // ---- copy warp
+        int slot = 0;
+        uint32_t round = 0;
+        for (int i = 0; i < n_my && ok; ++i) {
+            const int v0 = ((int)blockIdx.x + i * (int)gridDim.x) * kBcVecs;
+            for (int g = 0; g < WG && ok; ++g) {
+                if (round) ok = mbar_wait(sm_addr(box_free + slot), (round - 1u) & 1u, abort_s, 32) && ok;
+                if (!ok) break;
+                if (lane == 0) {
+                    mbar_expect_tx(sm_addr(box_full + slot), C::kBox);
+                    tma_load_2d(C::kBoxAddr + slot * C::kBox, &x_map, g * 32, v0, sm_addr(box_full + slot));
+                }
+                __syncwarp();
+                if (++slot == NB) { slot = 0; ++round; }
+            }
+        }
+    } else {
+        // ---- workers: vector `row` of the tile (= TMEM lane), dims 32 wg .. 32 wg + 31
+        const int wg = warp >> 2, q = warp & 3, row = 32 * q + lane;
+        const uint32_t tmem_lane = tmem_base + ((uint32_t)(32 * q) << 16);
+        const uint32_t lane_copy = (uint32_t)(lane & 15) * 8;
+        auto produce = [&](int i) {
+            const int n = i * WG + wg, slot = n % NB;
+            ok = mbar_wait(sm_addr(box_full + slot), (uint32_t)(n / NB) & 1u, abort_s) && ok;
+            float2 x[16];
+            const uint32_t r = C::kBoxAddr + slot * C::kBox + row * 128;
+#pragma unroll
+            for (int c = 0; c < 8; ++c) {
+                float4 v;
+                asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(r + ((c ^ (row & 7)) << 4)));
+                x[2 * c] = make_float2(v.x, v.y);
+                x[2 * c + 1] = make_float2(v.z, v.w);
+            }
+            mbar_arrive(sm_addr(box_free + slot));
+            const uint32_t b = i & 1;
+            if (i >= 2) {                                      // the A buffer's MMAs (tile i - 2) are done
+                ok = mbar_wait(sm_addr(mma_done + b), (uint32_t)((i >> 1) - 1) & 1u, abort_s) && ok;
+                tc_fence_after();
+            }
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                uint32_t w[16];
+#pragma unroll
+                for (int k = 0; k < 16; ++k) w[k] = bc_term(x[k]);
+                bc_tmem_st16(tmem_lane + b * C::kABuf + t * C::kATerm + wg * 16, w);
+            }
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            tc_fence_before();
+            mbar_arrive(sm_addr(a_full + b));
+        };
+        auto epilogue = [&](int i) -> bool {
+            const uint32_t b = i & 1;
+            ok = mbar_wait(sm_addr(mma_done + b), (uint32_t)(i >> 1) & 1u, abort_s) && ok;
+            tc_fence_after();
+            float2 v2[16];
+            tmem_ld32(v2, tmem_lane + C::kAcc + wg * 32);
+            tc_fence_before();
+            mbar_arrive(sm_addr(acc_free + b));
+            // squares: this thread's 32 as a tree, then the vector's WG parts
+            float2 s2[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) s2[k] = bc_mul2(v2[k], v2[k]);
+#pragma unroll
+            for (int h = 8; h; h >>= 1)
+#pragma unroll
+                for (int k = 0; k < h; ++k) { s2[k].x = __fadd_rn(s2[k].x, s2[k + h].x); s2[k].y = __fadd_rn(s2[k].y, s2[k + h].y); }
+            float* ns = norm_s + (i & 1) * kBcVecs * WG + row * WG;
+            ns[wg] = __fadd_rn(s2[0].x, s2[0].y);
+            // the barrier also votes: a wait that gave up in one of the group's warps stops all of them here
+            if (group_barrier_any(1u + q, 32u * WG, !ok || *abort_s != 0u)) {
+                ok = false;
+                *abort_s = 1u;
+                return false;
+            }
+            float ss;
+            if constexpr (WG == 4) {
+                const float4 t = *reinterpret_cast<const float4*>(ns);
+                ss = __fadd_rn(__fadd_rn(t.x, t.z), __fadd_rn(t.y, t.w));
+            } else {
+                const float2 t = *reinterpret_cast<const float2*>(ns);
+                ss = __fadd_rn(t.x, t.y);
+            }
+            const float radius = __fsqrt_rn(ss);
+            const int vec = ((int)blockIdx.x + i * (int)gridDim.x) * kBcVecs + row;
+            const bool live = radius > 1e-30f && radius < 3.4e38f;      // otherwise every direction is 0
+            const float dsafe = live ? radius : 1.f;
+            // IEEE-rounded quotient from the correctly rounded reciprocal and one residual step (Markstein 1990)
+            const float rinv = __frcp_rn(dsafe);
+            const float2 rinv2 = make_float2(rinv, rinv), negd2 = make_float2(-dsafe, -dsafe);
+            uint32_t packed[4] = {0u, 0u, 0u, 0u};
+            if (!live) {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) v2[k] = make_float2(0.f, 0.f);
+            }
+            if (fast) {
+                const float2 c128 = make_float2(128.f, 128.f), magic = make_float2(98432.f, 98432.f);
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const float2 y = bc_mul2(v2[k], rinv2);
+                    const float2 dir = bc_fma2(bc_fma2(y, negd2, v2[k]), rinv2, y);
+                    const float2 u = bc_fma2(dir, c128, magic);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int j = 2 * k + e, sh = (j * 4) & 31;
+                        const uint32_t a = (__float_as_uint(e ? u.y : u.x) & 0xFF80u) | lane_copy;
+                        uint2 be;
+                        asm volatile("ld.shared.v2.u32 {%0, %1}, [%2 + %3];\n" : "=r"(be.x), "=r"(be.y) : "r"(a), "n"(C::kTabAddr));
+                        uint32_t& pw = packed[j >> 3];
+                        pw |= be.y & (0xFu << sh);
+                        if ((e ? dir.y : dir.x) > __uint_as_float(be.x)) pw += 1u << sh;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const float dir[2] = {__fdiv_rn(v2[k].x, dsafe), __fdiv_rn(v2[k].y, dsafe)};
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        uint32_t best = 0;
+                        float dist = 1e30f;
+                        for (int l = 0; l < p.n_levels; ++l) {
+                            const float d = fabsf(dir[e] - cb[l]);
+                            if (d < dist) { dist = d; best = l; }
+                        }
+                        packed[k >> 2] |= best << (((2 * k + e) * 4) & 31);
+                    }
+                }
+            }
+            if (vec < p.N) {
+                if (wg == 0) p.radius_out[vec] = radius;
+                *reinterpret_cast<uint4*>(p.packed_out + (size_t)vec * (D / 2) + wg * 16) =
+                    make_uint4(packed[0], packed[1], packed[2], packed[3]);
+            }
+            return true;
+        };
+        bool going = true;
+        for (int i = 0; i < n_my && going; ++i) {
+            produce(i);
+            if (i >= 1) going = epilogue(i - 1);
+        }
+        if (going && n_my >= 1) epilogue(n_my - 1);
+    }
+    if (!ok && lane == 0) { *abort_s = 1u; atomicOr(&g_bridge_compress_error, 1u); }
+    if (*abort_s && tid == 0) {                                // give box copies still in flight time to land
+        const long long t0 = clock64();
+        while (clock64() - t0 < (1ll << 20)) {}
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem_base, C::kTmemCols);
+}
+
+// ------------------------------------------------------------------ host side
+bool bridge_compress_fits(int N, int D, const float* input, const float* rotation, const uint8_t* packed) {
+    // The set-up (R to three bfloat16 terms, decision points and table) is a fixed cost: 14 us at D = 128 for anything up
+    // to one tile per SM.  The CTA-per-vector kernel, which reads R from L2, takes 3.4 us for 8 vectors and 7.5 for 511
+    // and grows by 3.7 per 296 more, so it finishes first below about 1280 vectors (D = 64: 11.3 us against 5.7 at 511).
+    return (D == 64 || D == 128) && N >= kBridgeCompressMin && (reinterpret_cast<uintptr_t>(input) & 15) == 0 &&
+           (reinterpret_cast<uintptr_t>(rotation) & 7) == 0 && (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
+}
+
+template <int D>
+static cudaError_t launch_bridge_compress(const float* input, const BridgeCompressParams& p, int sms, cudaStream_t st) {
+    using C = BridgeCompressCfg<D>;
+    CUtensorMap map;
+    const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)p.N}, strides[1] = {(cuuint64_t)D * 4};
+    const cuuint32_t box[2] = {32u, (cuuint32_t)kBcVecs};
+    if (!encode_tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, input, dims, strides, box)) return cudaErrorInvalidValue;
+    auto kern = bridge_compress_kernel<D>;
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
+    if (e != cudaSuccess) return e;
+    const int n_tiles = (p.N + kBcVecs - 1) / kBcVecs;
+    kern<<<n_tiles < sms ? n_tiles : sms, C::THREADS, C::smem_bytes(), st>>>(p, map);
+    return cudaGetLastError();
+}
+
+cudaError_t bridge_compress_launch(const float* input, const float* rotation, const float* codebook, float* radius_out,
+                                   uint8_t* packed_out, int N, int D, int n_levels, int sms, cudaStream_t st) {
+    BridgeCompressParams p{rotation, codebook, radius_out, packed_out, N, n_levels};
+    return D == 64 ? launch_bridge_compress<64>(input, p, sms, st) : launch_bridge_compress<128>(input, p, sms, st);
+}
+
+int bridge_compress_error_flags(unsigned int* flags) {
+    unsigned int v = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&v, g_bridge_compress_error, sizeof(v)) != cudaSuccess) return PQ_ERR_CUDA;
+    if (v && cudaMemcpyToSymbol(g_bridge_compress_error, &zero, sizeof(zero)) != cudaSuccess) return PQ_ERR_CUDA;
+    *flags = v;
+    return PQ_OK;
+}
+
+}  // namespace pq

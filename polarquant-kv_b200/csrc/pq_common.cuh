@@ -77,5 +77,9 @@ int decode_error_flags(unsigned int* flags);
 int dequant_error_flags(unsigned int* flags);
 // pq_lse_merge.cu: bit 0 a wait for a peer's records gave up
 int exchange_error_flags(unsigned int* flags);
+// pq_bridge_attn.cu: bit 0 a wait for a tile copy gave up, bit 1 shared-memory window unusable
+int bridge_error_flags(unsigned int* flags);
+// pq_bridge_compress.cu: the same
+int bridge_compress_error_flags(unsigned int* flags);
 
 }  // namespace pq

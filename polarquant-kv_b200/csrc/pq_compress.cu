@@ -642,29 +642,12 @@ pq_compress_kernel(const CompressParams p, const __grid_constant__ CUtensorMap x
     if (warp == 0) tmem_dealloc(tmem_base, C::kTmemCols);
 }
 
-// Tensor map of x as a [n_vec][D] float16 matrix, boxes of 128 vectors x 64 halves, 128-byte swizzle.
-// The encoder is a driver entry point, fetched through the runtime so the library links to cudart only.
+// Tensor map of x as a [n_vec][D] float16 matrix, boxes of 128 vectors x 64 halves.
 static int make_x_map(const CompressParams& p, int D, CUtensorMap* map) {
-    typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    static encode_fn encode = nullptr;
-    if (!encode) {
-        void* fn = nullptr;
-        cudaDriverEntryPointQueryResult qres;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
-            qres != cudaDriverEntryPointSuccess || !fn)
-            return PQ_ERR_CUDA;
-        encode = reinterpret_cast<encode_fn>(fn);
-    }
     const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)p.n_vec};
     const cuuint64_t strides[1] = {(cuuint64_t)D * sizeof(__half)};
     const cuuint32_t box[2] = {64u, (cuuint32_t)kTileVecs};
-    const cuuint32_t estr[2] = {1u, 1u};
-    const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half*>(p.x), dims, strides, box,
-                              estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? PQ_OK : PQ_ERR_CUDA;
+    return encode_tensor_map_2d(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, p.x, dims, strides, box) ? PQ_OK : PQ_ERR_CUDA;
 }
 
 template <int D, int BITS, bool QJL>
@@ -710,7 +693,13 @@ extern "C" int pq_poll_device_errors(unsigned int* flags_out) {
     unsigned int xf = 0;
     const int sx = pq::exchange_error_flags(&xf);
     if (sx != PQ_OK) return sx;
-    *flags_out = v | pf | (df << 3) | (qf << 6) | (xf << 7);
+    unsigned int bf = 0;
+    const int sb = pq::bridge_error_flags(&bf);
+    if (sb != PQ_OK) return sb;
+    unsigned int cf = 0;
+    const int sc = pq::bridge_compress_error_flags(&cf);
+    if (sc != PQ_OK) return sc;
+    *flags_out = v | pf | (df << 3) | (qf << 6) | (xf << 7) | (bf << 8) | (cf << 10);
     return PQ_OK;
 }
 

@@ -2,14 +2,12 @@
 // decoded lines 695-763) for sm_100a: the per-vector-radius codec with nibble-packed
 // indices, as kernels laid out for a 148-SM part instead of one CTA per vector / per head.
 //
-//   compress   one warp owns four vectors at a time; Rᵀ sits in shared memory once per CTA
-//              (head dims 64 and 128), every R word read feeds four FMAs; the sum of squares
-//              is combined in the order of the reference's shared-memory tree (element t with
-//              t + 64, then + 32, ... , + 1), so the radius sees the same additions.
-//   attention  CTAs own (kv head, query group, slice of S); a warp takes 32 tokens at a time,
-//              each lane holds D/32 (rounded up) dims, the 32 partial dot products are
-//              transposed and summed with 31 shuffles so that lane t ends with token t's
-//              score; online softmax; the slices are merged by the last CTA to finish.
+//   compress   head dims 64 and 128 and more than a few hundred vectors: pq_bridge_compress.cu (tensor cores); everything
+//              else one CTA per vector, which streams R from L2.
+//   attention  head dims 64 and 128: pq_bridge_attn.cu.  Other head dims: CTAs own (kv head, query group, slice of S); a
+//              warp takes 32 tokens at a time, each lane holds D/32 (rounded up) dims, the 32 partial dot products are
+//              transposed and summed with 31 shuffles so that lane t ends with token t's score; online softmax; the
+//              slices are merged by the last CTA to finish.
 //   rotate / inverse rotate: one CTA per row (a few dozen rows per call).
 #include <cuda_runtime.h>
 
@@ -20,6 +18,7 @@
 #include <cstdlib>
 
 #include "polarquant_llama_abi.h"
+#include "pq_bridge.cuh"
 
 namespace {
 
@@ -52,36 +51,71 @@ bool launched() {
 // rows · Rᵀ and rows · R
 // ---------------------------------------------------------------------------------------------
 
-// out[n][j] = sum_k in[n][k] * R[j][k]: a warp per output element, lanes along k (coalesced).
-__global__ void __launch_bounds__(256) rotate_rows_kernel(const float* __restrict__ in, const float* __restrict__ R,
-                                                          float* __restrict__ out, int D) {
+// These run over a few dozen rows per call and are bound by the latency of R's loads from L2, so what counts is how many
+// of them a warp has in flight: a warp takes kRowBatch rows of R at once (a row per loop step, as a first version did,
+// is one round trip after another: 6 us instead of 2.5 for a token's eight vectors of 128).
+constexpr int kRowBatch = 8;
+
+// dot[u] = sum_k xs[k] * R[j0 + u][k] over the warp's lanes (every lane gets the sums); rows past D read row D - 1.
+__device__ __forceinline__ void dot_rows(const float* xs, const float* __restrict__ R, int D, int j0, int lane,
+                                         float (&dot)[kRowBatch]) {
+#pragma unroll
+    for (int u = 0; u < kRowBatch; ++u) dot[u] = 0.0f;
+#pragma unroll 4
+    for (int k = lane; k < D; k += 32) {
+        const float x = xs[k];
+        float r[kRowBatch];
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) r[u] = __ldg(R + (size_t)min(j0 + u, D - 1) * D + k);
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) dot[u] = fmaf(x, r[u], dot[u]);
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) dot[u] += __shfl_xor_sync(kFull, dot[u], o);
+}
+
+// out[n][j] = sum_k in[n][k] * R[j][k]: lanes along k (coalesced).
+__global__ void __launch_bounds__(512) rotate_rows_kernel(const float* in, const float* __restrict__ R, float* out, int D) {
     __shared__ float xs[kMaxDim];
     const int n = blockIdx.x;
     for (int k = threadIdx.x; k < D; k += blockDim.x) xs[k] = in[(size_t)n * D + k];
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int j = warp; j < D; j += blockDim.x >> 5) {
-        const float* row = R + (size_t)j * D;
-        float s = 0.0f;
-        for (int k = lane; k < D; k += 32) s = fmaf(xs[k], row[k], s);
+    for (int j0 = warp * kRowBatch; j0 < D; j0 += (blockDim.x >> 5) * kRowBatch) {
+        float dot[kRowBatch];
+        dot_rows(xs, R, D, j0, lane, dot);
 #pragma unroll
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (lane == 0) out[(size_t)n * D + j] = s;
+        for (int u = 0; u < kRowBatch; ++u)
+            if (lane == u && j0 + u < D) out[(size_t)n * D + j0 + u] = dot[u];
     }
 }
 
-// out[n][j] = sum_k in[n][k] * R[k][j]: a thread per output element, k ascending.
-__global__ void __launch_bounds__(256) inverse_rotate_rows_kernel(const float* __restrict__ in,
-                                                                  const float* __restrict__ R,
-                                                                  float* __restrict__ out, int D) {
+// out[n][j] = sum_k in[n][k] * R[k][j]: kInvCols columns at a time, k dealt to kInvParts threads of a column.  (One CTA
+// per row, which reads its input before it writes: `out` may be `in`.)
+constexpr int kInvCols = 128, kInvParts = 8;
+__global__ void __launch_bounds__(kInvCols * kInvParts) inverse_rotate_rows_kernel(const float* in, const float* __restrict__ R,
+                                                                                  float* out, int D) {
     __shared__ float xs[kMaxDim];
-    const int n = blockIdx.x;
-    for (int k = threadIdx.x; k < D; k += blockDim.x) xs[k] = in[(size_t)n * D + k];
+    __shared__ float part[kInvParts][kInvCols];
+    const int n = blockIdx.x, c = threadIdx.x, y = threadIdx.y;
+    for (int k = y * kInvCols + c; k < D; k += kInvCols * kInvParts) xs[k] = in[(size_t)n * D + k];
     __syncthreads();
-    for (int j = threadIdx.x; j < D; j += blockDim.x) {
+    for (int j0 = 0; j0 < D; j0 += kInvCols) {
+        const int j = min(j0 + c, D - 1);
         float s = 0.0f;
-        for (int k = 0; k < D; ++k) s = fmaf(xs[k], R[(size_t)k * D + j], s);
-        out[(size_t)n * D + j] = s;
+#pragma unroll 16
+        for (int k = y; k < D; k += kInvParts) s = fmaf(xs[k], __ldg(R + (size_t)k * D + j), s);
+        part[y][c] = s;
+        __syncthreads();
+        if (y == 0 && j0 + c < D) {
+            float t = 0.0f;
+#pragma unroll
+            for (int u = 0; u < kInvParts; ++u) t += part[u][c];
+            out[(size_t)n * D + j] = t;
+        }
+        __syncthreads();
     }
 }
 
@@ -99,94 +133,9 @@ __device__ __forceinline__ int nearest_level(float v, const float* cb, int n_lev
     return best;
 }
 
-constexpr int kCmpWarps = 8;
-constexpr int kCmpVecs = 4;      // vectors a warp carries through the rotation together
-constexpr int kCmpSmallN = 4096;
-
-// Head dims 64 and 128.  Lane l owns rotated elements l + 32 i.
-template <int D>
-__global__ void __launch_bounds__(kCmpWarps * 32) compress_kernel(const float* __restrict__ input,
-                                                                   const float* __restrict__ R,
-                                                                   const float* __restrict__ codebook,
-                                                                   float* __restrict__ radius_out,
-                                                                   uint8_t* __restrict__ packed_out,
-                                                                   int N, int n_levels) {
-    constexpr int DPL = D / 32;
-    constexpr int kPitch = D + 1;                       // transposed fill and row reads both conflict-free
-    extern __shared__ __align__(16) float smem[];
-    float* Rt = smem;                                   // Rt[k][j] = R[j][k]
-    float* xs = smem + D * kPitch;                      // [warp][k][kCmpVecs]
-    __shared__ float cb[16];
-    if (threadIdx.x < n_levels) cb[threadIdx.x] = codebook[threadIdx.x];
-    for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
-        const int j = e / D, k = e - j * D;
-        Rt[k * kPitch + j] = R[e];
-    }
-    __syncthreads();
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float4* xw = reinterpret_cast<float4*>(xs + warp * D * kCmpVecs);
-    const int n_groups = (N + kCmpVecs - 1) / kCmpVecs;
-    for (int grp = blockIdx.x * kCmpWarps + warp; grp < n_groups; grp += gridDim.x * kCmpWarps) {
-        const int v0 = grp * kCmpVecs;
-        // stage the four inputs interleaved: xw[k] = {x0[k], x1[k], x2[k], x3[k]}
-        for (int k = lane; k < D; k += 32) {
-            float4 x;
-            x.x = input[(size_t)v0 * D + k];
-            x.y = v0 + 1 < N ? input[(size_t)(v0 + 1) * D + k] : 0.0f;
-            x.z = v0 + 2 < N ? input[(size_t)(v0 + 2) * D + k] : 0.0f;
-            x.w = v0 + 3 < N ? input[(size_t)(v0 + 3) * D + k] : 0.0f;
-            xw[k] = x;
-        }
-        __syncwarp();
-        float acc[kCmpVecs][DPL];
-#pragma unroll
-        for (int v = 0; v < kCmpVecs; ++v)
-#pragma unroll
-            for (int i = 0; i < DPL; ++i) acc[v][i] = 0.0f;
-#pragma unroll 4
-        for (int k = 0; k < D; ++k) {
-            const float4 x = xw[k];
-#pragma unroll
-            for (int i = 0; i < DPL; ++i) {
-                const float r = Rt[k * kPitch + lane + 32 * i];
-                acc[0][i] = fmaf(x.x, r, acc[0][i]);
-                acc[1][i] = fmaf(x.y, r, acc[1][i]);
-                acc[2][i] = fmaf(x.z, r, acc[2][i]);
-                acc[3][i] = fmaf(x.w, r, acc[3][i]);
-            }
-        }
-        __syncwarp();
-#pragma unroll
-        for (int v = 0; v < kCmpVecs; ++v) {
-            // sum of squares: element t pairs with t + D/2, then + D/4, ... down to + 1
-            float sq[DPL];
-#pragma unroll
-            for (int i = 0; i < DPL; ++i) sq[i] = __fmul_rn(acc[v][i], acc[v][i]);   // no contraction into the adds
-#pragma unroll
-            for (int h = DPL / 2; h; h >>= 1)
-#pragma unroll
-                for (int i = 0; i < h; ++i) sq[i] = __fadd_rn(sq[i], sq[i + h]);
-            float s = sq[0];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-            const float radius = sqrtf(s);
-            const bool live = v0 + v < N;
-            if (live && lane == 0) radius_out[v0 + v] = radius;
-#pragma unroll
-            for (int i = 0; i < DPL; ++i) {
-                const float dir = radius > 1e-30f ? acc[v][i] / radius : 0.0f;
-                const int idx = nearest_level(dir, cb, n_levels);
-                const int up = __shfl_down_sync(kFull, idx, 1);
-                if (live && !(lane & 1))
-                    packed_out[(size_t)(v0 + v) * (D / 2) + (lane >> 1) + 16 * i] = (uint8_t)(idx | (up << 4));
-            }
-        }
-    }
-}
-
 // Any even head dim up to 1024: one CTA per vector.
-__global__ void __launch_bounds__(256) compress_any_dim_kernel(const float* __restrict__ input,
+constexpr int kSmallWarps = 16;
+__global__ void __launch_bounds__(kSmallWarps * 32) compress_any_dim_kernel(const float* __restrict__ input,
                                                                const float* __restrict__ R,
                                                                const float* __restrict__ codebook,
                                                                float* __restrict__ radius_out,
@@ -195,27 +144,28 @@ __global__ void __launch_bounds__(256) compress_any_dim_kernel(const float* __re
     __shared__ float xs[kMaxDim];
     __shared__ float rot[kMaxDim];
     __shared__ float cb[16];
-    __shared__ float part[8];
+    __shared__ float part[kSmallWarps];
     const int n = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < n_levels) cb[threadIdx.x] = codebook[threadIdx.x];
     for (int k = threadIdx.x; k < D; k += blockDim.x) xs[k] = input[(size_t)n * D + k];
     __syncthreads();
     float sq = 0.0f;
-    for (int j = warp; j < D; j += 8) {
-        const float* row = R + (size_t)j * D;
-        float s = 0.0f;
-        for (int k = lane; k < D; k += 32) s = fmaf(xs[k], row[k], s);
+    for (int j0 = warp * kRowBatch; j0 < D; j0 += kSmallWarps * kRowBatch) {
+        float dot[kRowBatch];
+        dot_rows(xs, R, D, j0, lane, dot);
 #pragma unroll
-        for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-        if (lane == 0) rot[j] = s;
-        sq = fmaf(s, s, sq);
+        for (int u = 0; u < kRowBatch; ++u) {
+            if (j0 + u >= D) continue;
+            if (lane == u) rot[j0 + u] = dot[u];
+            sq = fmaf(dot[u], dot[u], sq);
+        }
     }
     if (lane == 0) part[warp] = sq;
     __syncthreads();
     float total = 0.0f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) total += part[w];
+    for (int w = 0; w < kSmallWarps; ++w) total += part[w];
     const float radius = sqrtf(total);
     if (threadIdx.x == 0) radius_out[n] = radius;
     for (int b = threadIdx.x; b < D / 2; b += blockDim.x) {
@@ -234,20 +184,7 @@ constexpr int kAttWarps = 4;
 constexpr int kTile = 32;                     // tokens a warp takes at a time (lane t <-> token t)
 constexpr float kLowest = -1e30f;
 
-struct AttnParams {
-    const float* q;
-    const uint8_t* pk;
-    const float* kr;
-    const uint8_t* pv;
-    const float* vr;
-    const float* codebook;
-    float* out;
-    float* partials;          // [total_q_heads][n_split][2 + 32*DPL], used when n_split > 1
-    unsigned* tickets;        // [total_kv_heads * groups], zero between launches
-    int gqa, S, D, n_levels, n_split, tiles_per_split;
-    float scale;
-    int vector_loads;         // rows start on a multiple of the lane's byte count
-};
+using AttnParams = pq::BridgeAttnParams;
 
 // DPL/2 packed bytes of one row for this lane, zero beyond the row.
 template <int DPL>
@@ -551,6 +488,16 @@ __global__ void __launch_bounds__(kAttWarps * 32, 3) attention_kernel(const Attn
     }
 }
 
+// Device addresses of the workspace on the current device.
+bool workspace(AttnParams& p) {
+    if (cudaGetSymbolAddress((void**)&p.partials, g_partials) == cudaSuccess &&
+        cudaGetSymbolAddress((void**)&p.tickets, g_tickets) == cudaSuccess)
+        return true;
+    fail(kErrCuda, "attention: workspace symbol lookup failed");
+    cudaGetLastError();
+    return false;
+}
+
 template <int DPL, int G>
 bool launch_attention(const AttnParams& p, dim3 grid, cudaStream_t stream) {
     attention_kernel<DPL, G><<<grid, kAttWarps * 32, 0, stream>>>(p);
@@ -607,7 +554,7 @@ void polarquant_rotate_query_cuda_c(const float* q_input, const float* rotation,
     if (total_q_heads <= 0 || D <= 0) return;
     if (!q_input || !rotation || !q_rotated) { fail(kErrNull, "rotate_query: NULL pointer"); return; }
     if (D > kMaxDim) { fail(kErrDim, "rotate_query: head dim above 1024"); return; }
-    rotate_rows_kernel<<<total_q_heads, 256, 0, (cudaStream_t)stream>>>(q_input, rotation, q_rotated, D);
+    rotate_rows_kernel<<<total_q_heads, 512, 0, (cudaStream_t)stream>>>(q_input, rotation, q_rotated, D);
     launched();
 }
 
@@ -616,7 +563,7 @@ void polarquant_inverse_rotate_cuda_c(const float* input, const float* rotation,
     if (total_q_heads <= 0 || D <= 0) return;
     if (!input || !rotation || !output) { fail(kErrNull, "inverse_rotate: NULL pointer"); return; }
     if (D > kMaxDim) { fail(kErrDim, "inverse_rotate: head dim above 1024"); return; }
-    inverse_rotate_rows_kernel<<<total_q_heads, 256, 0, (cudaStream_t)stream>>>(input, rotation, output, D);
+    inverse_rotate_rows_kernel<<<total_q_heads, dim3(kInvCols, kInvParts), 0, (cudaStream_t)stream>>>(input, rotation, output, D);
     launched();
 }
 
@@ -628,31 +575,15 @@ void polarquant_compress_cuda_c(const float* input, const float* rotation, const
     if (!dim_ok(D)) { fail(kErrDim, "compress: head dim must be even and at most 1024"); return; }
     if (n_levels < 1 || n_levels > 16) { fail(kErrLevels, "compress: n_levels outside [1, 16]"); return; }
     cudaStream_t st = (cudaStream_t)stream;
-    // The shared-memory transpose of R costs a fixed 20-odd microseconds per launch; below a few
-    // thousand vectors the CTA-per-vector kernel, which streams R from L2, finishes first.
-    if ((D == 64 || D == 128) && N >= kCmpSmallN) {
+    if (pq::bridge_compress_fits(N, D, input, rotation, packed_out)) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const int n_groups = (N + kCmpVecs - 1) / kCmpVecs;
-        const int ctas = std::min((n_groups + kCmpWarps - 1) / kCmpWarps, (D == 64 ? 4 : 2) * sms);
-        const size_t smem = ((size_t)D * (D + 1) + (size_t)kCmpWarps * D * kCmpVecs) * sizeof(float);
-        cudaError_t e;
-        if (D == 64) {
-            e = cudaFuncSetAttribute(compress_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e == cudaSuccess)
-                compress_kernel<64><<<ctas, kCmpWarps * 32, smem, st>>>(input, rotation, codebook, radius_out,
-                                                                         packed_out, N, n_levels);
-        } else {
-            e = cudaFuncSetAttribute(compress_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e == cudaSuccess)
-                compress_kernel<128><<<ctas, kCmpWarps * 32, smem, st>>>(input, rotation, codebook, radius_out,
-                                                                          packed_out, N, n_levels);
-        }
-        if (e != cudaSuccess) { fail(kErrCuda, cudaGetErrorString(e)); return; }
-    } else {
-        compress_any_dim_kernel<<<N, 256, 0, st>>>(input, rotation, codebook, radius_out, packed_out, D, n_levels);
+        const cudaError_t e = pq::bridge_compress_launch(input, rotation, codebook, radius_out, packed_out, N, D, n_levels, sms, st);
+        if (e != cudaSuccess) fail(kErrCuda, cudaGetErrorString(e));
+        return;
     }
+    compress_any_dim_kernel<<<N, kSmallWarps * 32, 0, st>>>(input, rotation, codebook, radius_out, packed_out, D, n_levels);
     launched();
 }
 
@@ -674,27 +605,36 @@ void polarquant_fused_attention_cuda_c(const float* q_rotated, const uint8_t* pa
     }
     cudaStream_t st = (cudaStream_t)stream;
     const int gqa = total_q_heads / total_kv_heads;
-    int DPL = 2;
-    while (32 * DPL < D) DPL *= 2;
-    int G = 8;
-    while (G > 1 && (gqa % G || G * DPL > 32)) G >>= 1;
-    const int groups = gqa / G;
-
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const int n_tiles = (S + kTile - 1) / kTile;
-    const int base = total_kv_heads * groups;
-    // two CTAs per SM with at least two tiles per warp (three CTAs per SM measured slower:
-    // 192 against 150 microseconds at 8 kv heads x 65536 tokens)
-    int n_split = std::max(1, std::min((2 * sms + base - 1) / base, n_tiles / (2 * kAttWarps)));
-    int tiles_per_split = (n_tiles + n_split - 1) / n_split;
-    n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
 
     AttnParams p{};
     p.q = q_rotated; p.pk = packed_k; p.kr = k_radius; p.pv = packed_v; p.vr = v_radius;
     p.codebook = codebook; p.out = output;
     p.gqa = gqa; p.S = S; p.D = D; p.n_levels = n_levels; p.scale = scale;
+
+    // Head dims 64 and 128 on 16-byte boundaries (the bridge's own buffers are) have a kernel of their own.  It masks
+    // indices with n_levels - 1 like the general one, so other table sizes than powers of two behave alike.
+    if (pq::bridge_attention_fits(D, packed_k, packed_v) && (reinterpret_cast<uintptr_t>(q_rotated) & 7) == 0) {
+        const int groups = pq::bridge_attention_plan(p, total_kv_heads, sms, kWsFloats, kWsTickets, total_q_heads);
+        if (p.n_split > 1 && !workspace(p)) return;
+        const cudaError_t e = pq::bridge_attention_launch(p, total_kv_heads, groups, st);
+        if (e != cudaSuccess) fail(kErrCuda, cudaGetErrorString(e));
+        return;
+    }
+
+    int DPL = 2;
+    while (32 * DPL < D) DPL *= 2;
+    int G = 8;
+    while (G > 1 && (gqa % G || G * DPL > 32)) G >>= 1;
+    const int groups = gqa / G;
+    const int n_tiles = (S + kTile - 1) / kTile;
+    const int base = total_kv_heads * groups;
+    // two CTAs per SM with at least two tiles per warp (three CTAs per SM measured slower)
+    int n_split = std::max(1, std::min((2 * sms + base - 1) / base, n_tiles / (2 * kAttWarps)));
+    int tiles_per_split = (n_tiles + n_split - 1) / n_split;
+    n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
     const int bpl = DPL / 2;
     p.vector_loads = ((D / 2) % bpl == 0) && (reinterpret_cast<uintptr_t>(packed_k) % bpl == 0) &&
                      (reinterpret_cast<uintptr_t>(packed_v) % bpl == 0);
@@ -708,13 +648,7 @@ void polarquant_fused_attention_cuda_c(const float* q_rotated, const uint8_t* pa
         }
         tiles_per_split = (n_tiles + n_split - 1) / n_split;
         n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
-        if (n_split > 1 &&
-            (cudaGetSymbolAddress((void**)&p.partials, g_partials) != cudaSuccess ||
-             cudaGetSymbolAddress((void**)&p.tickets, g_tickets) != cudaSuccess)) {
-            fail(kErrCuda, "attention: workspace symbol lookup failed");
-            cudaGetLastError();
-            return;
-        }
+        if (n_split > 1 && !workspace(p)) return;
     }
     p.n_split = n_split;
     p.tiles_per_split = tiles_per_split;

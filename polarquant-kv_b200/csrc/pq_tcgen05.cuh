@@ -1,5 +1,7 @@
 // tcgen05 / TMEM / TMA / mbarrier wrappers shared by the tensor-core kernels (inline PTX, sm_100a).
 #pragma once
+#include <atomic>
+
 #include <cuda.h>   // CUtensorMap and its enums only; the encoder is looked up at run time
 
 #include "pq_common.cuh"
@@ -193,6 +195,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, const 
         }
     }
     return false;
+}
+
+// Tensor map of a row-major matrix, 128-byte swizzle, zeros outside.  The encoder is a driver entry point, fetched through
+// the runtime so the library links to cudart only (the lookup is thread-safe: every thread stores the same address).
+inline bool encode_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, const void* base, const cuuint64_t (&dims)[2],
+                                 const cuuint64_t (&strides)[1], const cuuint32_t (&box)[2]) {
+    typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static std::atomic<void*> entry{nullptr};
+    void* fn = entry.load(std::memory_order_acquire);
+    if (!fn) {
+        cudaDriverEntryPointQueryResult qres;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres) != cudaSuccess ||
+            qres != cudaDriverEntryPointSuccess || !fn)
+            return false;
+        entry.store(fn, std::memory_order_release);
+    }
+    const cuuint32_t estr[2] = {1u, 1u};
+    return reinterpret_cast<encode_fn>(fn)(map, type, 2, const_cast<void*>(base), dims, strides, box, estr,
+                                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 }  // namespace pq

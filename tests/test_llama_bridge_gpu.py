@@ -185,3 +185,48 @@ def test_arguments_the_bridge_cannot_serve_are_reported():
         LB.fused_attention(q, pk, r, pk, r, torch.zeros(16, device="cuda"), 1.0)
     with pytest.raises(ValueError, match="n_levels"):
         LB.fused_attention(torch.zeros(4, 64, device="cuda"), pk, r, pk, r, torch.zeros(17, device="cuda"), 1.0)
+
+
+# edges of the tensor-core compress kernel: its smallest size, several tiles per CTA with a ragged last one, and
+# codebooks its bucket table cannot hold (descending, levels in one bucket), which are scanned
+@pytest.mark.parametrize("d,n,book", [(128, 1280, "normal"), (64, 1281, "normal"), (128, 60_011, "normal"),
+                                      (64, 130_049, "normal"), (128, 1500, "descending"), (64, 1500, "narrow")])
+def test_compress_tensor_core_edges_vs_oracle(d, n, book):
+    from polarquant_kv import _ext
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(n + d)
+    x = (rng.standard_normal((n, d)) * np.exp(rng.uniform(-30, 30, (n, 1)))).astype(np.float32)
+    x[1] = 0.0
+    R, cb = orthogonal(d, rng), codebook_for(16, rng)
+    if book == "descending":
+        cb = cb[::-1].copy()
+    elif book == "narrow":
+        cb = np.sort((0.02 * rng.standard_normal(16)).astype(np.float32))
+    radius, packed = LB.compress(torch.from_numpy(x).cuda(), torch.from_numpy(R).cuda(), torch.from_numpy(cb).cuda())
+    want_radius, want_packed, direction = LO.compress(x, R, cb)
+    # six bfloat16 product terms (2^-24 each dropped) and a few truncating float32 accumulations: a few units of 2^-23
+    np.testing.assert_allclose(radius.cpu().numpy(), want_radius, rtol=2e-6, atol=1e-30)
+    got, want = LO.unpack(packed.cpu().numpy(), 16), LO.unpack(want_packed, 16)
+    n_bad, n_unexplained, worst = explained(direction, cb.astype(np.float64), got, want)
+    assert n_unexplained == 0 and n_bad <= max(2, got.size // 2000), (n_bad, n_unexplained, worst)
+    assert _ext.poll_device_errors() == 0
+
+
+# edges of the kernel for head dims 64 and 128: every group width (missing heads masked), tiles of one token, slices
+@pytest.mark.parametrize("hq,hkv,s", [(1, 1, 31), (2, 2, 32), (6, 3, 129), (3, 1, 64), (7, 1, 1000), (10, 2, 513),
+                                      (20, 1, 300), (5, 5, 4099), (2, 1, 70_001)])
+@pytest.mark.parametrize("d", [64, 128])
+def test_fused_attention_group_widths_vs_oracle(hq, hkv, s, d):
+    from polarquant_kv import _ext
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(hq * 7 + hkv + s + d)
+    cb = codebook_for(16, rng)
+    pk, kr = random_cache(hkv, s, d, 16, rng)
+    pv, vr = random_cache(hkv, s, d, 16, rng)
+    q = (rng.standard_normal((hq, d)) * 1.5).astype(np.float32)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    out = LB.fused_attention(dev(q), dev(pk), dev(kr), dev(pv), dev(vr), dev(cb), 0.1).cpu().numpy()
+    want = LO.fused_attention(q, pk, kr, pv, vr, cb, 16, 0.1)
+    # float32 throughout: scores of a few tens carry about 1e-5, which the weights inherit
+    assert np.abs(out - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
+    assert _ext.poll_device_errors() == 0
