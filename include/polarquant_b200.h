@@ -204,7 +204,11 @@ int pq_dequant(const void* blocks, int64_t n_vec, int head_dim, int n_bits,
  *              q_heads and kv_heads on the same stream reuse the buffer as it is; before a
  *              call with another batch or other head counts clear the first
  *              4 * batch * q_heads bytes (rounded up to 256) again, because the records of
- *              a call with fewer counters lie where a larger call keeps its counters
+ *              a call with fewer counters lie where a larger call keeps its counters.  When
+ *              scratch_bytes is at least pq_decode_attn_counter_bytes() more than needed, the
+ *              records start at pq_decode_attn_counter_bytes() instead: calls of any shapes
+ *              with at most that many bytes of counters, all made that way, share a buffer
+ *              without a clear in between
  *              (concurrent calls need separate scratch buffers)
  */
 int pq_decode_attn(const void* q, const void* k_blocks, const void* v_blocks,
@@ -218,6 +222,9 @@ int pq_decode_attn(const void* q, const void* k_blocks, const void* v_blocks,
 /* Bytes of scratch pq_decode_attn needs for this shape (n_splits == 0: library default). */
 size_t pq_decode_attn_scratch_bytes(int batch, int q_heads, int kv_heads, int64_t seq_len,
                                     int head_dim, int n_splits);
+
+/* Bytes at the start of the scratch that only ever hold counters (65536). */
+size_t pq_decode_attn_counter_bytes(void);
 
 /* The number of splits the library would choose for n_splits == 0 on the current device. */
 int pq_decode_attn_default_splits(int batch, int q_heads, int kv_heads, int64_t seq_len, int head_dim);

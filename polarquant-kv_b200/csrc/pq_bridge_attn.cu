@@ -438,7 +438,8 @@ template <int D, int G>
 static cudaError_t launch_bridge(const BridgeAttnParams& p, int total_kv_heads, int groups, cudaStream_t st) {
     auto kern = bridge_attn_kernel<D, G>;
     const size_t smem = BridgeAttnCfg<D, G>::smem_bytes();
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static std::atomic<uint64_t> allowed{0};
+    const cudaError_t e = allow_shared(kern, smem, allowed);
     if (e != cudaSuccess) return e;
     kern<<<dim3(p.n_split, groups, total_kv_heads), BridgeAttnCfg<D, G>::WARPS * 32, smem, st>>>(p);
     return cudaGetLastError();

@@ -21,6 +21,10 @@
 // closer than 1e-5, two decision points in a bucket) is scanned level by level as the reference does.
 // Measured (D = 128, 16 levels): 131 072 vectors 32 us = 2.36 TB/s of the 580 bytes a vector takes (the FP32 kernel before
 // it, R^T in shared memory: 226 us), 20 000 vectors 17 us (48.5).
+// The rotation's last bits depend on the order of its additions, and a coordinate within them of a decision point gets one
+// index or the other.  So that stored bytes do not depend on which kernel wrote them, a block with a coordinate closer
+// than kBcNear to a decision point (one in 500 at 16 levels) is put on a list and done again at the end in the order of
+// an FP32 chain, k ascending per output.  R's fp32 words are the exact sums of their three terms in shared memory.
 // All waits are bounded (bit 10 of pq_poll_device_errors).
 #include <cstring>
 
@@ -32,6 +36,8 @@ namespace pq {
 static __device__ unsigned int g_bridge_compress_error = 0;
 
 constexpr int kBcVecs = 128;
+constexpr float kBcNear = 6e-7f;               // ten times the typical difference between two summation orders
+constexpr int kBcList = 480;                   // (vector, block) entries a CTA keeps for the second pass
 
 template <int D>
 struct BridgeCompressCfg {
@@ -47,7 +53,7 @@ struct BridgeCompressCfg {
     // Layout by absolute shared address: index table (257 buckets x 16 copies x 8 bytes; its address is an immediate of
     // the lookups) | three terms of R | boxes | small buffers
     static constexpr uint32_t kTabAddr = 4096;
-    static constexpr uint32_t kTabRows = 257;
+    static constexpr uint32_t kTabRows = 258;
     static constexpr uint32_t kBAddr = (kTabAddr + kTabRows * 128 + 1023) & ~1023u;
     static constexpr uint32_t kBoxAddr = (kBAddr + 3 * kBTerm + 1023) & ~1023u;
     static constexpr uint32_t kSmallAddr = kBoxAddr + kBoxes * kBox;
@@ -56,7 +62,7 @@ struct BridgeCompressCfg {
     static constexpr uint32_t kAcc = 2 * kABuf;
     static constexpr uint32_t kTmemCols = D == 128 ? 512 : 256;
     // norms [2][128][WG], codebook 16, decision points 16, barriers, tensor-memory slot, abort flag, fast flag
-    static constexpr uint32_t kSmall = 2 * kBcVecs * WG * 4 + 2 * 16 * 4 + (2 * kBoxes + 6) * 8 + 16;
+    static constexpr uint32_t kSmall = 2 * kBcVecs * WG * 4 + 2 * 16 * 4 + (2 * kBoxes + 6) * 8 + 32 + kBcList * 4;
     static constexpr size_t smem_bytes() { return kSmallAddr + kSmall; }
 };
 
@@ -97,8 +103,9 @@ __device__ __forceinline__ void bc_tmem_st16(uint32_t taddr, const uint32_t (&v)
                  : "memory");
 }
 // Bucket of a coordinate in bits 7..15: the unit in the last place of 128 v + 98432 is 2^-7, so those bits hold
-// floor(128 v + 128) after rounding to 1/128.  Monotone in v.
-__device__ __forceinline__ uint32_t bc_bucket_bits(float v) { return __float_as_uint(fmaf(v, 128.f, 98432.f)) & 0xFF80u; }
+// floor(128 v + 128 + shift) after rounding to 1/128.  Monotone in v.  `magic` = 98432 + shift; the shift (below 1) keeps
+// every decision point away from the edges of its bucket, so that a coordinate near one shares its bucket.
+__device__ __forceinline__ uint32_t bc_bucket_bits(float v, float magic) { return __float_as_uint(fmaf(v, 128.f, magic)) & 0xFF80u; }
 // order-preserving integer image of a float and back
 __device__ __forceinline__ int bc_key(float x) {
     const int b = __float_as_int(x);
@@ -113,8 +120,79 @@ struct BridgeCompressParams {
     const float* codebook;
     float* radius_out;
     uint8_t* packed_out;
+    const float* x;
     int N, n_levels;
 };
+
+// One block of one vector once more, by a whole warp (lane l: elements l + 32 i): k ascending per output as on CUDA cores,
+// squares as a tree over i and the lanes, then level by level.  Its 16 bytes were stored before.  (Out of line and with
+// real loops: it runs for a few blocks per CTA, and straight-line code would spend its time on instruction fetches.)
+template <int D>
+__device__ __noinline__ void bc_again(const float* input, uint8_t* packed_out, const float* cb, int n_levels, int vec, int block) {
+    using C = BridgeCompressCfg<D>;
+    constexpr int WG = C::WG;
+    const int lane = threadIdx.x & 31;
+    const float* x = input + (size_t)vec * D;
+    float acc[WG], xl[WG];
+#pragma unroll
+    for (int m = 0; m < WG; ++m) { xl[m] = __ldg(x + lane + 32 * m); acc[m] = 0.f; }
+#pragma unroll 1
+    for (int kc = 0; kc < D / 8; ++kc) {
+        float xv[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) xv[k] = __shfl_sync(0xffffffffu, xl[0], ((kc & 3) * 8 + k) & 31);
+        if ((kc & 3) == 3) {
+#pragma unroll
+            for (int m = 0; m + 1 < WG; ++m) xl[m] = xl[m + 1];
+        }
+#pragma unroll
+        for (int i = 0; i < WG; ++i) {
+            // R[n][8 kc .. 8 kc + 7]: the sum of the three terms, exact in any order
+            const int n = lane + 32 * i;
+            const uint32_t a = C::kBAddr + (uint32_t)(kc * (D / 8) * 128 + (n >> 3) * 128 + (n & 7) * 16);
+            float r[8];
+#pragma unroll
+            for (int t = 2; t >= 0; --t) {
+                uint32_t w[4];
+                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(a + t * C::kBTerm));
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
+                    r[2 * k] = t == 2 ? lo : r[2 * k] + lo;
+                    r[2 * k + 1] = t == 2 ? hi : r[2 * k + 1] + hi;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[i] = fmaf(xv[k], r[k], acc[i]);
+        }
+    }
+    float sq[WG];
+#pragma unroll
+    for (int i = 0; i < WG; ++i) sq[i] = __fmul_rn(acc[i], acc[i]);
+#pragma unroll
+    for (int h = WG / 2; h; h >>= 1)
+#pragma unroll
+        for (int i = 0; i < h; ++i) sq[i] = __fadd_rn(sq[i], sq[i + h]);
+    float t = sq[0];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const float radius = __fsqrt_rn(t);
+    float v = acc[0];
+#pragma unroll
+    for (int i = 1; i < WG; ++i)
+        if (i == block) v = acc[i];
+    const float dir = radius > 1e-30f ? __fdiv_rn(v, radius) : 0.f;
+    uint32_t best = 0;
+    float dist = 1e30f;
+#pragma unroll 1
+    for (int l = 0; l < n_levels; ++l) {
+        const float d = fabsf(dir - cb[l]);
+        if (d < dist) { dist = d; best = l; }
+    }
+    const uint32_t up = __shfl_down_sync(0xffffffffu, best, 1);
+    __syncwarp();
+    if (!(lane & 1)) packed_out[(size_t)vec * (D / 2) + block * 16 + (lane >> 1)] = (uint8_t)(best | (up << 4));
+}
 
 template <int D>
 __global__ void __launch_bounds__(BridgeCompressCfg<D>::THREADS, 1)
@@ -143,6 +221,9 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_full + 6);
     volatile uint32_t* abort_s = tmem_slot + 1;
     uint32_t* fast_s = tmem_slot + 2;
+    float* magic_s = reinterpret_cast<float*>(tmem_slot + 3);
+    int* n_list = reinterpret_cast<int*>(tmem_slot + 4);
+    int* list = reinterpret_cast<int*>(tmem_slot + 8);          // vector * WG + block
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // ---- set-up
@@ -158,6 +239,7 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
         }
         *abort_s = 0u;
         *fast_s = 1u;
+        *n_list = 0;
     }
     if (tid < 16) cb[tid] = __ldg(p.codebook + min(tid, p.n_levels - 1));
     // B: three bfloat16 terms of R, K-major core matrices (8 rows x 16 bytes), K chunks D / 8 * 128 bytes apart
@@ -194,7 +276,24 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
         if (!good) *fast_s = 0u;
     }
     __syncthreads();
-    if (tid + 1 < p.n_levels - 1 && bc_bucket_bits(thr[tid]) == bc_bucket_bits(thr[tid + 1])) *fast_s = 0u;
+    if (warp == 0) {
+        // the first shift for which every decision point lies alone in its bucket and off its edges
+        const bool mine = lane < p.n_levels - 1;
+        const float t = mine ? thr[lane] : 0.f;
+        bool found = false;
+        for (int k = 0; k < 16 && !found; ++k) {
+            const float magic = 98432.f + (float)k * 0.0625f;
+            const uint32_t b = bc_bucket_bits(t, magic);
+            const uint32_t next = __shfl_down_sync(0xffffffffu, b, 1);
+            const bool bad = mine && (bc_bucket_bits(t - 4e-6f, magic) != b || bc_bucket_bits(t + 4e-6f, magic) != b ||
+                                      (lane + 1 < p.n_levels - 1 && next == b));
+            found = !__any_sync(0xffffffffu, bad);
+            if (found && lane == 0) *magic_s = magic;
+        }
+        if (!found && lane == 0) { *fast_s = 0u; *magic_s = 98432.f; }
+    }
+    __syncthreads();
+    const float magic1 = *magic_s;
     // a bucket's entry: its decision point (or a number no coordinate reaches) and the count of lower ones,
     // replicated into every index field of a word
     for (int e = tid; e < (int)C::kTabRows * 16; e += C::THREADS) {
@@ -202,7 +301,7 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
         float t = 3.0e38f;
         uint32_t cnt = 0;
         for (int i = 0; i < p.n_levels - 1; ++i) {
-            const uint32_t tb = bc_bucket_bits(thr[i]);
+            const uint32_t tb = bc_bucket_bits(thr[i], magic1);
             if (tb == bits) t = thr[i];
             cnt += tb < bits ? 1u : 0u;
         }
@@ -336,12 +435,13 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
             const float rinv = __frcp_rn(dsafe);
             const float2 rinv2 = make_float2(rinv, rinv), negd2 = make_float2(-dsafe, -dsafe);
             uint32_t packed[4] = {0u, 0u, 0u, 0u};
+            float near = 1.f;                              // smallest distance of a coordinate to a decision point
             if (!live) {
 #pragma unroll
                 for (int k = 0; k < 16; ++k) v2[k] = make_float2(0.f, 0.f);
             }
             if (fast) {
-                const float2 c128 = make_float2(128.f, 128.f), magic = make_float2(98432.f, 98432.f);
+                const float2 c128 = make_float2(128.f, 128.f), magic = make_float2(magic1, magic1);
 #pragma unroll
                 for (int k = 0; k < 16; ++k) {
                     const float2 y = bc_mul2(v2[k], rinv2);
@@ -355,7 +455,13 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
                         asm volatile("ld.shared.v2.u32 {%0, %1}, [%2 + %3];\n" : "=r"(be.x), "=r"(be.y) : "r"(a), "n"(C::kTabAddr));
                         uint32_t& pw = packed[j >> 3];
                         pw |= be.y & (0xFu << sh);
-                        if ((e ? dir.y : dir.x) > __uint_as_float(be.x)) pw += 1u << sh;
+                        const float off = (e ? dir.y : dir.x) - __uint_as_float(be.x);       // its sign is exact
+                        near = fminf(near, fabsf(off));
+                        asm("{\n\t.reg .pred p;\n\t"
+                            "setp.gt.f32 p, %1, 0f00000000;\n\t"
+                            "@p add.u32 %0, %0, %2;\n\t}\n"
+                            : "+r"(pw)
+                            : "f"(off), "r"(1u << sh));
                     }
                 }
             } else {
@@ -365,11 +471,12 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         uint32_t best = 0;
-                        float dist = 1e30f;
+                        float dist = 1e30f, second = 1e30f;
                         for (int l = 0; l < p.n_levels; ++l) {
                             const float d = fabsf(dir[e] - cb[l]);
-                            if (d < dist) { dist = d; best = l; }
+                            if (d < dist) { second = dist; dist = d; best = l; } else { second = fminf(second, d); }
                         }
+                        near = fminf(near, 0.5f * (second - dist));
                         packed[k >> 2] |= best << (((2 * k + e) * 4) & 31);
                     }
                 }
@@ -379,6 +486,20 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
                 *reinterpret_cast<uint4*>(p.packed_out + (size_t)vec * (D / 2) + wg * 16) =
                     make_uint4(packed[0], packed[1], packed[2], packed[3]);
             }
+            uint32_t todo = __ballot_sync(0xffffffffu, near < kBcNear && live && vec < p.N);
+            if (todo) {
+                int at = 0;
+                if (lane == 0) at = atomicAdd(n_list, __popc(todo));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                const int mine = at + __popc(todo & ((1u << lane) - 1u));
+                if ((todo >> lane & 1u) && mine < kBcList) list[mine] = vec * WG + wg;
+                todo = __ballot_sync(0xffffffffu, (todo >> lane & 1u) && mine >= kBcList);
+                while (todo) {                                 // the list is full: at once
+                    const int v = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    bc_again<D>(p.x, p.packed_out, cb, p.n_levels, vec - lane + v, wg);
+                }
+            }
             return true;
         };
         bool going = true;
@@ -387,6 +508,9 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
             if (i >= 1) going = epilogue(i - 1);
         }
         if (going && n_my >= 1) epilogue(n_my - 1);
+        asm volatile("bar.sync 9, %0;\n" ::"r"(WORKERS) : "memory");       // the list is complete, its blocks are stored
+        const int n = min(*n_list, kBcList);
+        for (int e = warp; e < n; e += WORKERS / 32) bc_again<D>(p.x, p.packed_out, cb, p.n_levels, list[e] / WG, list[e] % WG);
     }
     if (!ok && lane == 0) { *abort_s = 1u; atomicOr(&g_bridge_compress_error, 1u); }
     if (*abort_s && tid == 0) {                                // give box copies still in flight time to land
@@ -400,9 +524,8 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
 
 // ------------------------------------------------------------------ host side
 bool bridge_compress_fits(int N, int D, const float* input, const float* rotation, const uint8_t* packed) {
-    // The set-up (R to three bfloat16 terms, decision points and table) is a fixed cost: 14 us at D = 128 for anything up
-    // to one tile per SM.  The CTA-per-vector kernel, which reads R from L2, takes 3.4 us for 8 vectors and 7.5 for 511
-    // and grows by 3.7 per 296 more, so it finishes first below about 1280 vectors (D = 64: 11.3 us against 5.7 at 511).
+    // Below kBridgeCompressMin the kernel with a few vectors per CTA, which reads R from L2, is about as fast (the set-up
+    // and the second pass here are a fixed cost of 17 us at D = 128), and its summation order settles near ties there.
     return (D == 64 || D == 128) && N >= kBridgeCompressMin && (reinterpret_cast<uintptr_t>(input) & 15) == 0 &&
            (reinterpret_cast<uintptr_t>(rotation) & 7) == 0 && (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
 }
@@ -415,7 +538,8 @@ static cudaError_t launch_bridge_compress(const float* input, const BridgeCompre
     const cuuint32_t box[2] = {32u, (cuuint32_t)kBcVecs};
     if (!encode_tensor_map_2d(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, input, dims, strides, box)) return cudaErrorInvalidValue;
     auto kern = bridge_compress_kernel<D>;
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::smem_bytes());
+    static std::atomic<uint64_t> allowed{0};
+    const cudaError_t e = allow_shared(kern, C::smem_bytes(), allowed);
     if (e != cudaSuccess) return e;
     const int n_tiles = (p.N + kBcVecs - 1) / kBcVecs;
     kern<<<n_tiles < sms ? n_tiles : sms, C::THREADS, C::smem_bytes(), st>>>(p, map);
@@ -424,7 +548,7 @@ static cudaError_t launch_bridge_compress(const float* input, const BridgeCompre
 
 cudaError_t bridge_compress_launch(const float* input, const float* rotation, const float* codebook, float* radius_out,
                                    uint8_t* packed_out, int N, int D, int n_levels, int sms, cudaStream_t st) {
-    BridgeCompressParams p{rotation, codebook, radius_out, packed_out, N, n_levels};
+    BridgeCompressParams p{rotation, codebook, radius_out, packed_out, input, N, n_levels};
     return D == 64 ? launch_bridge_compress<64>(input, p, sms, st) : launch_bridge_compress<128>(input, p, sms, st);
 }
 

@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "polarquant_b200.h"
 
 namespace pq {
@@ -67,6 +69,20 @@ __device__ __forceinline__ float fast_exp2(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;\n" : "=f"(y) : "f"(x));
     return y;
+}
+
+// Raises a kernel's dynamic shared-memory limit, once per device (the driver call costs a few hundred nanoseconds, a
+// fifth of a launch).  `done` belongs to the kernel: a bit per device; racing first calls repeat the same setting.
+template <typename Kernel>
+inline cudaError_t allow_shared(Kernel kern, size_t bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+    if (bit & done.load(std::memory_order_relaxed)) return cudaSuccess;
+    const cudaError_t s = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (s == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+    return s;
 }
 
 // Device error flags of the prefill kernel, read and cleared (defined in pq_prefill_attn.cu).

@@ -660,8 +660,8 @@ static int launch_compress(const CompressParams& p, cudaStream_t stream) {
         return PQ_ERR_CUDA;
     const size_t smem = C::smem_bytes();
     auto kern = pq_compress_kernel<D, BITS, QJL>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return PQ_ERR_CUDA;
+    static std::atomic<uint64_t> allowed{0};
+    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
     const int64_t n_tiles = (p.n_vec + kTileVecs - 1) / kTileVecs;
     // one CTA per SM: a CTA holds up to all 512 tensor-memory columns of its SM
     const int grid = (int)(n_tiles < sm_count ? n_tiles : sm_count);
@@ -751,17 +751,31 @@ static int compress_rows_impl(const void* x, int64_t n_rows, int64_t tokens_per_
     for (int i = 0; i < 16; ++i) p.cb[i] = i < nlev ? codebook[i] : 0.f;
     // bucket(y), evaluated exactly as the kernel does (one fused multiply-add, then mantissa bits):
     // floor(64 y + 64) after rounding to 1/128
-    for (int k = 0; k < 132; ++k) { p.bucket_t[k] = 3.0e38f; p.bucket_base[k] = 0; }
-    for (int i = 0; i < nlev - 1; ++i) {
-        const float u = fmaf(thresholds[i], 64.f, 98368.f);
-        uint32_t bits;
-        memcpy(&bits, &u, sizeof(bits));
-        const int kb = (int)((bits >> 7) & 0xFFu);
-        if (!(thresholds[i] > -1.0f && thresholds[i] < 1.0f) || kb > 130 || p.bucket_t[kb] != 3.0e38f)
-            return PQ_ERR_BAD_SHAPE;      // thresholds out of range or two of them in one bucket
-        p.bucket_t[kb] = thresholds[i];
-        for (int k = kb + 1; k < 132; ++k) p.bucket_base[k] += 1;
+    // (the last table of the thread is kept: building it costs as much host time as a launch)
+    struct Buckets {
+        int nlev = 0;
+        float thresholds[16], t[132];
+        uint32_t base[132];
+    };
+    static thread_local Buckets kept;
+    if (kept.nlev != nlev || memcmp(kept.thresholds, thresholds, sizeof(float) * (nlev - 1)) != 0) {
+        kept.nlev = 0;
+        for (int k = 0; k < 132; ++k) { kept.t[k] = 3.0e38f; kept.base[k] = 0; }
+        for (int i = 0; i < nlev - 1; ++i) {
+            const float u = fmaf(thresholds[i], 64.f, 98368.f);
+            uint32_t bits;
+            memcpy(&bits, &u, sizeof(bits));
+            const int kb = (int)((bits >> 7) & 0xFFu);
+            if (!(thresholds[i] > -1.0f && thresholds[i] < 1.0f) || kb > 130 || kept.t[kb] != 3.0e38f)
+                return PQ_ERR_BAD_SHAPE;      // thresholds out of range or two of them in one bucket
+            kept.t[kb] = thresholds[i];
+            for (int k = kb + 1; k < 132; ++k) kept.base[k] += 1;
+        }
+        memcpy(kept.thresholds, thresholds, sizeof(float) * (nlev - 1));
+        kept.nlev = nlev;
     }
+    memcpy(p.bucket_t, kept.t, sizeof(kept.t));
+    memcpy(p.bucket_base, kept.base, sizeof(kept.base));
 
 #define PQ_DISPATCH(DD, BB)                                                         \
     if (head_dim == DD && n_bits == BB)                                             \

@@ -1130,6 +1130,12 @@ static int device_sms() {
     return sms;
 }
 
+// Where the records start.  Tight: right behind the call's counters.  When the caller's buffer is kCounterBytes larger
+// than the call needs they start at kCounterBytes whatever the shape, so that calls of different shapes share the buffer
+// without a clear in between (each leaves its counters at zero, and no record ever lies where a counter may).
+constexpr size_t kCounterBytes = 65536;
+static size_t tight_counter_bytes(size_t groups) { return (groups * sizeof(unsigned int) + 255) & ~size_t(255); }
+
 // query heads per CTA: 4 (one MMA n-tile holds 4 heads x {hi, lo}) or 8 (a hi and a lo tile)
 static int heads_per_cta(int G) { return G <= 4 ? 4 : 8; }
 
@@ -1225,8 +1231,8 @@ static int launch_decode(const DecodeParams& p, int rows, cudaStream_t st) {
     using C = DecodeCfg<D, KBITS, VBITS, NH, QJL>;
     const size_t smem = C::smem_bytes(p.jl_dim);
     auto kern = pq_decode_attn_kernel<D, KBITS, VBITS, NH, QJL>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return PQ_ERR_CUDA;
+    static std::atomic<uint64_t> allowed{0};
+    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
     int sms = device_sms();
     if (sms <= 0) sms = 148;
     static_assert(C::kTeams <= kMaxTeams, "balanced_plan bounds the segments of a row with kMaxTeams");
@@ -1263,9 +1269,10 @@ extern "C" size_t pq_decode_attn_scratch_bytes(int batch, int q_heads, int kv_he
         int n_cta = 0;
         pq::balanced_plan((int64_t)groups, (seq_len + pq::kTileTok - 1) / pq::kTileTok, pq::device_sms(), &n_cta, &segs);
     }
-    const size_t tickets = (groups * sizeof(unsigned int) + 255) & ~size_t(255);
-    return tickets + groups * segs * pq::kRecHeads * (head_dim + 2) * sizeof(float);
+    return pq::tight_counter_bytes(groups) + groups * segs * pq::kRecHeads * (head_dim + 2) * sizeof(float);
 }
+
+extern "C" size_t pq_decode_attn_counter_bytes(void) { return pq::kCounterBytes; }
 
 // Argument checks shared by pq_decode_attn and pq_decode_attn_static.  Returns PQ_OK when a launch (or
 // the empty-input shortcut) may proceed; *n_splits_io is clamped to [0, tiles].
@@ -1331,8 +1338,8 @@ static int decode_attn_impl(const void* q, const void* k_blocks, const void* v_b
     }
     if (reinterpret_cast<uintptr_t>(scratch) & 255) return PQ_ERR_MISALIGNED;
     const int64_t tiles = (seq_len + kTileTok - 1) / kTileTok;
-    if (scratch_bytes < pq_decode_attn_scratch_bytes(batch, q_heads, kv_heads, seq_len, head_dim, n_splits))
-        return PQ_ERR_SCRATCH_TOO_SMALL;
+    const size_t need = pq_decode_attn_scratch_bytes(batch, q_heads, kv_heads, seq_len, head_dim, n_splits);
+    if (scratch_bytes < need) return PQ_ERR_SCRATCH_TOO_SMALL;
     const int rows = batch * kv_heads;
 
     DecodeParams p{};
@@ -1371,8 +1378,9 @@ static int decode_attn_impl(const void* q, const void* k_blocks, const void* v_b
         p.cbv[i] = i < (1 << v_bits) ? codebook_v[i] : 0.f;
     }
     const size_t groups = (size_t)rows * p.HG;
+    const bool roomy = tight_counter_bytes(groups) <= kCounterBytes && scratch_bytes >= need + kCounterBytes;
     p.tickets = static_cast<unsigned int*>(scratch);
-    p.records = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + ((groups * sizeof(unsigned int) + 255) & ~size_t(255)));
+    p.records = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + (roomy ? kCounterBytes : tight_counter_bytes(groups)));
 
     const bool wide = heads_per_cta(p.G) == 8;
 #define PQ_DEC(DD, KB, VB)                                                                            \

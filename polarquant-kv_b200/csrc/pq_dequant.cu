@@ -341,8 +341,8 @@ static int launch_dequant(const DequantParams& p, cudaStream_t st) {
     using C = DequantCfg<D>;
     const size_t smem = C::smem_bytes();
     auto kern = pq_dequant_kernel<D, BITS>;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return PQ_ERR_CUDA;
+    static std::atomic<uint64_t> allowed{0};
+    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)

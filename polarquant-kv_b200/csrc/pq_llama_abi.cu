@@ -56,39 +56,47 @@ bool launched() {
 // is one round trip after another: 6 us instead of 2.5 for a token's eight vectors of 128).
 constexpr int kRowBatch = 8;
 
-// dot[u] = sum_k xs[k] * R[j0 + u][k] over the warp's lanes (every lane gets the sums); rows past D read row D - 1.
-__device__ __forceinline__ void dot_rows(const float* xs, const float* __restrict__ R, int D, int j0, int lane,
-                                         float (&dot)[kRowBatch]) {
+// dot[v][u] = sum_k xs[v][k] * R[j0 + u][k] over the warp's lanes (every lane gets the sums); rows past D read row D - 1.
+template <int V>
+__device__ __forceinline__ void dot_rows(const float (*xs)[kMaxDim], const float* __restrict__ R, int D, int j0, int lane,
+                                         float (&dot)[V][kRowBatch]) {
 #pragma unroll
-    for (int u = 0; u < kRowBatch; ++u) dot[u] = 0.0f;
-#pragma unroll 4
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int u = 0; u < kRowBatch; ++u) dot[v][u] = 0.0f;
+#pragma unroll (V == 1 ? 4 : 2)
     for (int k = lane; k < D; k += 32) {
-        const float x = xs[k];
         float r[kRowBatch];
 #pragma unroll
         for (int u = 0; u < kRowBatch; ++u) r[u] = __ldg(R + (size_t)min(j0 + u, D - 1) * D + k);
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) dot[u] = fmaf(x, r[u], dot[u]);
+        for (int v = 0; v < V; ++v) {
+            const float x = xs[v][k];
+#pragma unroll
+            for (int u = 0; u < kRowBatch; ++u) dot[v][u] = fmaf(x, r[u], dot[v][u]);
+        }
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1)
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) dot[u] += __shfl_xor_sync(kFull, dot[u], o);
+        for (int v = 0; v < V; ++v)
+#pragma unroll
+            for (int u = 0; u < kRowBatch; ++u) dot[v][u] += __shfl_xor_sync(kFull, dot[v][u], o);
 }
 
 // out[n][j] = sum_k in[n][k] * R[j][k]: lanes along k (coalesced).
 __global__ void __launch_bounds__(512) rotate_rows_kernel(const float* in, const float* __restrict__ R, float* out, int D) {
-    __shared__ float xs[kMaxDim];
+    __shared__ float xs[1][kMaxDim];
     const int n = blockIdx.x;
-    for (int k = threadIdx.x; k < D; k += blockDim.x) xs[k] = in[(size_t)n * D + k];
+    for (int k = threadIdx.x; k < D; k += blockDim.x) xs[0][k] = in[(size_t)n * D + k];
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int j0 = warp * kRowBatch; j0 < D; j0 += (blockDim.x >> 5) * kRowBatch) {
-        float dot[kRowBatch];
-        dot_rows(xs, R, D, j0, lane, dot);
+        float dot[1][kRowBatch];
+        dot_rows<1>(xs, R, D, j0, lane, dot);
 #pragma unroll
         for (int u = 0; u < kRowBatch; ++u)
-            if (lane == u && j0 + u < D) out[(size_t)n * D + j0 + u] = dot[u];
+            if (lane == u && j0 + u < D) out[(size_t)n * D + j0 + u] = dot[0][u];
     }
 }
 
@@ -133,46 +141,63 @@ __device__ __forceinline__ int nearest_level(float v, const float* cb, int n_lev
     return best;
 }
 
-// Any even head dim up to 1024: one CTA per vector.
+// Any even head dim up to 1024: V vectors per CTA.  One, so that a token's few vectors spread over the SMs; four once there
+// are more vectors than SMs can hold, because every CTA streams the whole of R from L2 (1024 vectors of 128: 12.3 us at
+// one, where L2 delivers 64 KB per vector).
 constexpr int kSmallWarps = 16;
+template <int V>
 __global__ void __launch_bounds__(kSmallWarps * 32) compress_any_dim_kernel(const float* __restrict__ input,
                                                                const float* __restrict__ R,
                                                                const float* __restrict__ codebook,
                                                                float* __restrict__ radius_out,
                                                                uint8_t* __restrict__ packed_out,
-                                                               int D, int n_levels) {
-    __shared__ float xs[kMaxDim];
-    __shared__ float rot[kMaxDim];
+                                                               int N, int D, int n_levels) {
+    __shared__ float xs[V][kMaxDim];
+    __shared__ float rot[V][kMaxDim];
     __shared__ float cb[16];
-    __shared__ float part[kSmallWarps];
-    const int n = blockIdx.x;
+    __shared__ float part[V][8];
+    const int n0 = blockIdx.x * V;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x < n_levels) cb[threadIdx.x] = codebook[threadIdx.x];
-    for (int k = threadIdx.x; k < D; k += blockDim.x) xs[k] = input[(size_t)n * D + k];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+        for (int k = threadIdx.x; k < D; k += blockDim.x) xs[v][k] = input[(size_t)min(n0 + v, N - 1) * D + k];
     __syncthreads();
-    float sq = 0.0f;
     for (int j0 = warp * kRowBatch; j0 < D; j0 += kSmallWarps * kRowBatch) {
-        float dot[kRowBatch];
-        dot_rows(xs, R, D, j0, lane, dot);
+        float dot[V][kRowBatch];
+        dot_rows<V>(xs, R, D, j0, lane, dot);
 #pragma unroll
-        for (int u = 0; u < kRowBatch; ++u) {
-            if (j0 + u >= D) continue;
-            if (lane == u) rot[j0 + u] = dot[u];
-            sq = fmaf(dot[u], dot[u], sq);
-        }
+        for (int u = 0; u < kRowBatch; ++u)
+#pragma unroll
+            for (int v = 0; v < V; ++v)
+                if (lane == u && j0 + u < D) rot[v][j0 + u] = dot[v][u];
     }
-    if (lane == 0) part[warp] = sq;
     __syncthreads();
-    float total = 0.0f;
+    // squares in eight chains (j mod 8), added in order: stored indices at a decision point depend on the order
+    if (threadIdx.x < 8 * V) {
+        const int v = threadIdx.x >> 3, w = threadIdx.x & 7;
+        float sq = 0.0f;
+#pragma unroll 8
+        for (int j = w; j < D; j += 8) sq = fmaf(rot[v][j], rot[v][j], sq);
+        part[v][w] = sq;
+    }
+    __syncthreads();
 #pragma unroll
-    for (int w = 0; w < kSmallWarps; ++w) total += part[w];
-    const float radius = sqrtf(total);
-    if (threadIdx.x == 0) radius_out[n] = radius;
-    for (int b = threadIdx.x; b < D / 2; b += blockDim.x) {
-        const float d0 = radius > 1e-30f ? rot[2 * b] / radius : 0.0f;
-        const float d1 = radius > 1e-30f ? rot[2 * b + 1] / radius : 0.0f;
-        packed_out[(size_t)n * (D / 2) + b] =
-            (uint8_t)(nearest_level(d0, cb, n_levels) | (nearest_level(d1, cb, n_levels) << 4));
+    for (int v = 0; v < V; ++v) {
+        if (n0 + v >= N) break;
+        float total = 0.0f;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) total += part[v][w];
+        const float radius = sqrtf(total);
+        if (threadIdx.x == 0) radius_out[n0 + v] = radius;
+        // a quarter of the threads per vector when there are four
+        for (int b = (int)threadIdx.x - v * (kSmallWarps * 32 / V); b < D / 2; b += kSmallWarps * 32) {
+            if (b < 0) continue;
+            const float d0 = radius > 1e-30f ? rot[v][2 * b] / radius : 0.0f;
+            const float d1 = radius > 1e-30f ? rot[v][2 * b + 1] / radius : 0.0f;
+            packed_out[(size_t)(n0 + v) * (D / 2) + b] =
+                (uint8_t)(nearest_level(d0, cb, n_levels) | (nearest_level(d1, cb, n_levels) << 4));
+        }
     }
 }
 
@@ -583,7 +608,10 @@ void polarquant_compress_cuda_c(const float* input, const float* rotation, const
         if (e != cudaSuccess) fail(kErrCuda, cudaGetErrorString(e));
         return;
     }
-    compress_any_dim_kernel<<<N, kSmallWarps * 32, 0, st>>>(input, rotation, codebook, radius_out, packed_out, D, n_levels);
+    if (N < 512)
+        compress_any_dim_kernel<1><<<N, kSmallWarps * 32, 0, st>>>(input, rotation, codebook, radius_out, packed_out, N, D, n_levels);
+    else
+        compress_any_dim_kernel<4><<<(N + 3) / 4, kSmallWarps * 32, 0, st>>>(input, rotation, codebook, radius_out, packed_out, N, D, n_levels);
     launched();
 }
 

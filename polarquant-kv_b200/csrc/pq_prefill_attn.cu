@@ -907,13 +907,13 @@ static int launch_prefill(const PrefillParams& p, int rows, uint8_t* ws, cudaStr
         pq_prefill_expand_kernel<D, KBITS, VBITS><<<dim3(n_tiles, rows, 1), kPfDeqThreads, 0, st>>>(p, ws, n_tiles);
         if (cudaGetLastError() != cudaSuccess) return PQ_ERR_CUDA;
         auto kern = pq_prefill_attn_kernel<D, 4, 4, true>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return PQ_ERR_CUDA;
+        static std::atomic<uint64_t> allowed{0};
+    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
         kern<<<grid, pf_threads(true), smem, st>>>(p);
     } else {
         auto kern = pq_prefill_attn_kernel<D, KBITS, VBITS, false>;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return PQ_ERR_CUDA;
+        static std::atomic<uint64_t> allowed{0};
+    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
         kern<<<grid, pf_threads(false), smem, st>>>(p);
     }
     return cudaGetLastError() == cudaSuccess ? PQ_OK : PQ_ERR_CUDA;

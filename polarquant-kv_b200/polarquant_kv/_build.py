@@ -17,6 +17,8 @@ PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(PKG_DIR), "csrc")
 INCLUDE = os.path.join(os.path.dirname(os.path.dirname(PKG_DIR)), "include")
 LIB_PATH = os.path.join(PKG_DIR, "libpolarquant_b200.so")
+HOST_PATH = os.path.join(PKG_DIR, "_host.so")         # native host path of the Python package (CPython extension)
+HOST_SOURCE = os.path.join(CSRC, "pq_host.cpp")
 
 SOURCES = ["pq_compress.cu", "pq_dequant.cu", "pq_decode_attn.cu", "pq_prefill_attn.cu", "pq_lse_merge.cu", "pq_qjl.cu",
            "pq_llama_abi.cu", "pq_bridge_attn.cu", "pq_bridge_compress.cu"]
@@ -31,17 +33,51 @@ def _nvcc() -> str:
     raise RuntimeError("nvcc not found; set NVCC or put /usr/local/cuda/bin on PATH")
 
 
-def _stale() -> bool:
-    if not os.path.exists(LIB_PATH):
+def _older(target: str, deps) -> bool:
+    if not os.path.exists(target):
         return True
-    built = os.path.getmtime(LIB_PATH)
-    deps = [os.path.join(CSRC, s) for s in SOURCES] + [h if os.path.isabs(h) else os.path.join(CSRC, h) for h in HEADERS]
+    built = os.path.getmtime(target)
     return any(os.path.getmtime(d) > built for d in deps if os.path.exists(d))
 
 
+def _stale() -> bool:
+    deps = [os.path.join(CSRC, s) for s in SOURCES] + [h if os.path.isabs(h) else os.path.join(CSRC, h) for h in HEADERS]
+    return _older(LIB_PATH, deps)
+
+
+def _start_host_build(force: bool):
+    """The compiler process for _host.so, or None when it is up to date.  Plain C++ (no device code): torch's headers,
+    the C ABI's headers; libraries are found beside the module and in torch's own lib folder."""
+    headers = [h for h in HEADERS if os.path.isabs(h)]
+    if not force and not _older(HOST_PATH, [HOST_SOURCE] + headers):
+        return None
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for inc in cpp_extension.include_paths() + [cuda, sysconfig.get_paths()["include"], INCLUDE]:
+        cmd += ["-isystem" if inc != INCLUDE else "-I", inc]
+    cmd += [HOST_SOURCE, "-o", HOST_PATH, "-L", PKG_DIR, "-l:libpolarquant_b200.so", "-L", torch_lib, "-lc10", "-lc10_cuda",
+            "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-L", os.path.join(os.path.dirname(cuda), "lib64"), "-lcudart",
+            "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"]
+    return subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+
+
+def _finish_host_build(proc) -> None:
+    if proc is not None:
+        out, _ = proc.communicate()
+        if proc.returncode != 0:
+            raise RuntimeError(f"building _host.so failed:\n{out}")
+
+
 def build_library(force: bool = False, verbose: bool = False) -> str:
-    """Compile every kernel for sm_100a and link the shared library; returns its path."""
+    """Compile every kernel for sm_100a, link the shared library and build the host module; returns the library's path."""
     if not force and not _stale():
+        _finish_host_build(_start_host_build(False))
         return LIB_PATH
     nvcc = _nvcc()
     objs = []
@@ -71,6 +107,7 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     res = subprocess.run(link, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link failed:\n{res.stdout}")
+    _finish_host_build(_start_host_build(force))
     return LIB_PATH
 
 

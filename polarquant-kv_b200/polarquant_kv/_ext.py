@@ -44,6 +44,7 @@ SIGNATURES = {
                                       c_void_p, c_int, c_void_p, c_int, c_void_p]),
     "pq_decode_attn_static_scratch_capacity": (c_size_t, []),
     "pq_decode_attn_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int64, c_int, c_int]),
+    "pq_decode_attn_counter_bytes": (c_size_t, []),
     "pq_decode_attn_default_splits": (c_int, [c_int, c_int, c_int, c_int64, c_int]),
     "pq_lse_merge": (c_int, [c_void_p, c_int, c_int64, c_int, c_void_p, c_void_p, c_int, c_void_p]),
     "pq_lse_exchange_bytes": (c_size_t, [c_int, c_int64, c_int]),
@@ -67,6 +68,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class PQError(RuntimeError):
@@ -97,6 +99,23 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = handle
     return _lib
+
+
+def host():
+    """The native host path (csrc/pq_host.cpp), set up on first use; raises when it has not been built."""
+    global _host
+    if _host is None:
+        lib()                                        # its own, clearer error comes first
+        try:
+            from . import _host as module
+        except ImportError as exc:
+            raise ImportError(f"polarquant_kv._host cannot be loaded ({exc}): build it with "
+                              "`python -m polarquant_kv._build`; there is no fallback path") from exc
+        from .rotation import DevicePlan
+        from .types import CompressedKV
+        module.register(CompressedKV, DevicePlan, check)
+        _host = module
+    return _host
 
 
 def check(status: int, where: str) -> None:

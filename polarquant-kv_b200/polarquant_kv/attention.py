@@ -20,10 +20,12 @@ from .rotation import device_plan
 from .types import CompressedKV
 
 _SCRATCH: dict = {}
+_OUT_TYPES = (torch.float32, torch.float16)
 
 
 def _scratch(device, nbytes: int, batch: int, q_heads: int, kv_heads: int) -> torch.Tensor:
-    """Scratch for pq_decode_attn, one per (device, stream); grown on demand.
+    """Scratch for the pq_decode_attn calls made from Python (the ordinary ones go through the native host path,
+    which has its own), one per (device, stream); grown on demand.
 
     The buffer starts with one ticket counter per (batch, kv head, head group), which must read zero when
     a launch starts; the segment records follow.  A kernel leaves its own counters at zero, so consecutive
@@ -71,6 +73,10 @@ def decode_attention(query: torch.Tensor, ck: CompressedKV, cv: CompressedKV, pl
     ``seq_range`` restricts attention to tokens [begin, end) of the cache.  With ``seq_len_tensor``
     (one int64 on the device) the kernel reads the number of tokens when it runs, up to the cache's
     capacity (pq_decode_attn_dynamic): the launch can be replayed from a CUDA graph as the cache grows."""
+    if not partial and seq_range is None and n_splits <= 0 and query.dim() == 3 and out_dtype in _OUT_TYPES:
+        done = _ext.host().decode(query, ck, cv, plan, None, scale, bool(enable_qjl), out_dtype == torch.float16, seq_len_tensor)
+        if done is not None:
+            return done
     _require_cuda(query, "query")
     B, Hq, D = query.shape
     Hkv = ck.blocks.shape[1]
@@ -156,36 +162,33 @@ class PreparedDecode:
         else:
             self.out = torch.empty((B, Hq, D), dtype=out_dtype, device=self.dev)
         lib = _ext.lib()
-        self._fn = lib.pq_decode_attn
         self.seq_len_tensor = seq_len_tensor
         if seq_len_tensor is not None:
             if seq_len_tensor.dtype != torch.int64 or seq_len_tensor.numel() != 1 or seq_len_tensor.device != self.dev:
                 raise ValueError("seq_len_tensor must be a one-element int64 tensor on the query's device")
-            self._fn = lib.pq_decode_attn_dynamic
         need = lib.pq_decode_attn_scratch_bytes(B, Hq, Hkv, ck.max_seq_len, D, max(0, n_splits))
         self.scratch = torch.zeros(max(need, 256), dtype=torch.uint8, device=self.dev)   # private: no sharing
         cbk, cbv = tables(ck.n_bits)[0], tables(cv.n_bits)[0]
         use_qjl = bool(enable_qjl and plan.jl is not None and ck.qjl_signs is not None)
         if use_qjl and (not ck.qjl_signs.is_contiguous() or not ck.residual_norms.is_contiguous()):
             raise ValueError("sketch tensors must be contiguous")
-        self._head = (query.data_ptr(), ck.blocks.data_ptr(), cv.blocks.data_ptr(), B, Hq, Hkv)
-        self._tail = (ck.max_seq_len, D, ck.n_bits, cv.n_bits, cbk, cbv, plan.rot.data_ptr(),
-                      ctypes.c_float(scale if scale is not None else 1.0 / math.sqrt(D)),
-                      plan.jl.data_ptr() if use_qjl else None, plan.jl_dim if use_qjl else 0,
-                      ck.qjl_signs.data_ptr() if use_qjl else None,
-                      ck.residual_norms.data_ptr() if use_qjl else None,
-                      None if partial else self.out.data_ptr(), 1 if out_dtype == torch.float16 else 0,
-                      self.out.data_ptr() if partial else None,
-                      max(0, n_splits), self.scratch.data_ptr(), self.scratch.numel())
+        ptr = lambda t: t.data_ptr() if t is not None else 0                    # noqa: E731
+        self._tables = (cbk, cbv)
+        self._prepared = _ext.host().prepare(
+            query.data_ptr(), ck.blocks.data_ptr(), cv.blocks.data_ptr(), B, Hq, Hkv, ck.max_seq_len, D, ck.n_bits, cv.n_bits,
+            ctypes.addressof(cbk), ctypes.addressof(cbv), plan.rot.data_ptr(), ptr(plan.jl) if use_qjl else 0,
+            plan.jl_dim if use_qjl else 0, ck.qjl_signs.data_ptr() if use_qjl else 0,
+            ck.residual_norms.data_ptr() if use_qjl else 0, 0 if partial else self.out.data_ptr(),
+            1 if out_dtype == torch.float16 else 0, self.out.data_ptr() if partial else 0, max(0, n_splits),
+            self.scratch.data_ptr(), self.scratch.numel(), ptr(seq_len_tensor),
+            float(scale if scale is not None else 1.0 / math.sqrt(D)))
+        self._run = _ext.host().run_prepared
         self._stream = torch.cuda.current_stream(self.dev)
+        self._stream_handle = self._stream.cuda_stream
 
     def __call__(self, stream: torch.cuda.Stream | None = None) -> torch.Tensor:
         """Enqueue on the stream the object was prepared on, or on `stream`."""
-        if self.seq_len_tensor is not None:
-            st = self._fn(*self._head, self.ck.max_seq_len, self.seq_len_tensor.data_ptr(), *self._tail,
-                          (stream or self._stream).cuda_stream)
-        else:
-            st = self._fn(*self._head, self.ck.seq_len, *self._tail, (stream or self._stream).cuda_stream)
+        st = self._run(self._prepared, self.ck, stream.cuda_stream if stream is not None else self._stream_handle)
         if st:
             _ext.check(st, "pq_decode_attn")
         return self.out
@@ -235,6 +238,10 @@ def prefill_attention(query: torch.Tensor, ck: CompressedKV, cv: CompressedKV, p
     K/V tile once into a device workspace first (1 KB per token and KV head at D = 128), False
     dequantises inside the attention kernel; None picks the workspace when more than one 128-row
     query tile shares a KV head and the workspace stays below PREFILL_WORKSPACE_LIMIT."""
+    if use_workspace is None and out_dtype in _OUT_TYPES:
+        done = _ext.host().prefill(query, ck, cv, plan, None, scale, bool(causal), out_dtype == torch.float16, PREFILL_WORKSPACE_LIMIT)
+        if done is not None:
+            return done
     _require_cuda(query, "query")
     B, Hq, Sq, D = query.shape
     Hkv = ck.blocks.shape[1]
@@ -277,6 +284,13 @@ def compressed_attention(query: torch.Tensor, compressed_keys, compressed_values
     {"output", "scores"} like the reference's 2-D form (attention.py:157-160); the pre-softmax
     scores [.., Sq, S] come from a checking path (pq_dequant + a float32 matmul + the sketch
     correction in torch), not from the attention kernels."""
+    if not return_scores and num_kv_heads is None and out_dtype in _OUT_TYPES and isinstance(query, torch.Tensor) \
+            and query.dim() == 4 and query.shape[2] == 1:
+        # one position over finished caches: the native path; it declines everything else
+        done = _ext.host().decode(query, compressed_keys, compressed_values, rotation_matrix,
+                                  jl_matrix if enable_qjl else None, None, bool(enable_qjl), out_dtype == torch.float16, None)
+        if done is not None:
+            return done
     _require_cuda(query, "query")
     if query.dim() == 2:                       # reference 2-D form: one head, n_q query rows
         def lift(x):

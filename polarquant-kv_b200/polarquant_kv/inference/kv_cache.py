@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import torch
 
-from .. import quantizer
+from .. import _ext, quantizer
 from ..attention import decode_attention, prefill_attention
 from ..qjl import generate_jl_matrix
 from ..rotation import device_plan, generate_rotation_matrix
@@ -73,6 +73,13 @@ class KVCacheManager:
         the host-side length is left alone: a decode step recorded once as a CUDA graph appends at a
         position that advances on the device; call ``advance`` afterwards for the bookkeeping."""
         new_seq = key.shape[2]
+        if self.config.enable_compression and (position is not None or self._seq_len + new_seq <= self.max_seq_len):
+            # both tensors in one native call; it declines what is not the ordinary form (then the checks below speak)
+            if _ext.host().append(key, value, self._compressed_keys, self._compressed_values, self.plan, self.plan_v,
+                                  self._seq_len if position is None else position):
+                if position is None:
+                    self._seq_len += new_seq
+                return
         if position is not None:
             if not self.config.enable_compression:
                 raise ValueError("a device-side position needs the compressed cache")
@@ -113,6 +120,11 @@ class KVCacheManager:
         positions: with ``causal`` query i sees tokens [0, seq_len - seq_q + i].  ``seq_len_tensor``
         (one int64 on the device, seq_q == 1): the number of tokens is read by the kernel when it runs."""
         B, Hq, Sq, D = query.shape
+        if self.config.enable_compression and Sq == 1:
+            done = _ext.host().decode(query, self._compressed_keys, self._compressed_values, self.plan, None, None,
+                                      self.config.enable_qjl, False, seq_len_tensor)
+            if done is not None:
+                return done
         if seq_len_tensor is not None:
             if Sq != 1 or not self.config.enable_compression:
                 raise ValueError("a device-side length serves single-token steps over the compressed cache")

@@ -31,13 +31,17 @@ def _f32(t: torch.Tensor, name: str) -> torch.Tensor:
 
 
 def _raise_on_error(where: str) -> None:
-    code = _ext.lib().polarquant_last_error_c()
+    code = _ext.host().bridge_error()
     if code:
         raise ValueError(f"{where}: {ERRORS.get(code, code)}")
 
 
 def compress(x: torch.Tensor, rotation: torch.Tensor, codebook: torch.Tensor):
     """x [N, D] float32 -> (radius float32 [N], packed uint8 [N, D/2])."""
+    done = _ext.host().bridge_compress(x, rotation, codebook)
+    if done is not None:
+        _raise_on_error("polarquant_compress_cuda_c")
+        return done
     x, rotation, codebook = _f32(x, "x"), _f32(rotation, "rotation"), _f32(codebook, "codebook")
     n, d = x.shape
     radius = torch.empty(n, dtype=torch.float32, device=x.device)
@@ -52,6 +56,10 @@ def compress(x: torch.Tensor, rotation: torch.Tensor, codebook: torch.Tensor):
 
 def rotate_query(q: torch.Tensor, rotation: torch.Tensor) -> torch.Tensor:
     """q [Hq, D] · Rᵀ."""
+    done = _ext.host().bridge_rotate(q, rotation, False)
+    if done is not None:
+        _raise_on_error("polarquant_rotate_query_cuda_c")
+        return done
     q, rotation = _f32(q, "q"), _f32(rotation, "rotation")
     out = torch.empty_like(q)
     with torch.cuda.device(q.device):
@@ -63,6 +71,10 @@ def rotate_query(q: torch.Tensor, rotation: torch.Tensor) -> torch.Tensor:
 
 def inverse_rotate(y: torch.Tensor, rotation: torch.Tensor) -> torch.Tensor:
     """y [Hq, D] · R."""
+    done = _ext.host().bridge_rotate(y, rotation, True)
+    if done is not None:
+        _raise_on_error("polarquant_inverse_rotate_cuda_c")
+        return done
     y, rotation = _f32(y, "y"), _f32(rotation, "rotation")
     out = torch.empty_like(y)
     with torch.cuda.device(y.device):
@@ -76,6 +88,11 @@ def fused_attention(q_rot: torch.Tensor, packed_k: torch.Tensor, k_radius: torch
                     packed_v: torch.Tensor, v_radius: torch.Tensor, codebook: torch.Tensor,
                     scale: float, out: torch.Tensor | None = None) -> torch.Tensor:
     """q_rot [Hq, D]; packed_* uint8 [Hkv, S, D/2]; *_radius [Hkv, S] -> [Hq, D] (rotated space)."""
+    if out is None:
+        done = _ext.host().bridge_attention(q_rot, packed_k, k_radius, packed_v, v_radius, codebook, scale)
+        if done is not None:
+            _raise_on_error("polarquant_fused_attention_cuda_c")
+            return done
     q_rot, k_radius, v_radius, codebook = (_f32(q_rot, "q_rot"), _f32(k_radius, "k_radius"),
                                            _f32(v_radius, "v_radius"), _f32(codebook, "codebook"))
     if packed_k.dtype != torch.uint8 or packed_v.dtype != torch.uint8:

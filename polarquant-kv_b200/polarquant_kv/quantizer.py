@@ -42,6 +42,7 @@ def tables(n_bits: int):
     if t is None:
         cb = block_codebook(n_bits)
         t = (_ext.float_array(cb), _ext.float_array(decision_thresholds(cb)), cb)
+        _ext.host().set_tables(n_bits, ctypes.addressof(t[0]), ctypes.addressof(t[1]))
         _TABLES[n_bits] = t
     return t
 
@@ -66,6 +67,9 @@ def compress(kv: torch.Tensor, rotation_matrix, n_bits: int = 4, group_size: int
     (pq_compress_rows_dynamic), which lets a decode step be recorded once as a CUDA graph.
     An empty input returns an empty cache (compress_kernel.py:108-124).
     """
+    done = _ext.host().compress(kv, rotation_matrix, n_bits, group_size, jl_matrix, out, position)
+    if done is not None:
+        return done
     _require_cuda(kv, "kv")
     if kv.dim() < 1:
         raise ValueError("kv needs at least one dimension")
@@ -125,6 +129,10 @@ def compress(kv: torch.Tensor, rotation_matrix, n_bits: int = 4, group_size: int
 def decompress(cache: CompressedKV, rotation_matrix, dtype: torch.dtype = torch.float32) -> torch.Tensor:
     """CompressedKV -> [batch, heads, seq_len, head_dim] in ``dtype`` (float32 like the numpy
     reference, or float16 like decompress_gpu, clamped to the float16 range)."""
+    if dtype in (torch.float32, torch.float16):
+        done = _ext.host().decompress(cache, rotation_matrix, dtype == torch.float16)
+        if done is not None:
+            return done
     if dtype not in (torch.float32, torch.float16):
         raise ValueError("dtype must be float32 or float16")
     blocks = cache.blocks

@@ -9,6 +9,8 @@ import numpy as np
 import torch
 from scipy.stats import ortho_group
 
+from . import _ext
+
 ROT_SCALE = 4096.0   # power of two applied before the float16 split of R
 JL_SCALE = 1024.0    # same for the folded JL matrix P @ R^T
 
@@ -83,6 +85,12 @@ class DevicePlan:
             self.jl_dim = P.shape[0]
             self.jl = torch.from_numpy(P.astype(np.float32)).contiguous().to(self.device)
             self.jl_split = torch.from_numpy(split_fp16(P @ R.T, JL_SCALE)).contiguous().to(self.device)
+        self._native = None
+        if self.device.type == "cuda":
+            self.device = self.rot.device                    # with its index
+            ptr = lambda t: t.data_ptr() if t is not None else 0                # noqa: E731
+            self._native = _ext.host().plan_handle(self.head_dim, self.device.index, ptr(self.rot), ptr(self.rot_split),
+                                                   ptr(self.jl), ptr(self.jl_split), self.jl_dim)
 
 
 _PLANS: dict = {}
@@ -95,48 +103,23 @@ def _digest(m) -> str:
     return hashlib.blake2b(a.tobytes(), digest_size=16).hexdigest() + str(a.shape)
 
 
-_QUICK: dict = {}
-_QUICK_LIMIT = 64
-
-
-def _quick_key(m):
-    """Identity of a matrix object without reading it: the object, where its data lives and, for arrays,
-    three probe values (for tensors the version counter) - enough to notice the in-place edits that the
-    content digest would notice, at no cost per call.  None when the object offers no such handle."""
-    if m is None:
-        return ("-",)
-    if isinstance(m, np.ndarray):
-        if m.size == 0:
-            return None
-        flat = m.reshape(-1) if m.flags.c_contiguous else None
-        if flat is None:
-            return None
-        return ("np", id(m), m.shape, m.dtype.str, m.ctypes.data, float(flat[0]), float(flat[m.size // 2]), float(flat[-1]))
-    if isinstance(m, torch.Tensor):
-        return ("pt", id(m), tuple(m.shape), str(m.dtype), m.data_ptr(), m._version)
-    return None
-
-
 def device_plan(rotation_matrix, device, jl_matrix=None) -> DevicePlan:
     """Cached DevicePlan for (R, P, device).  The same matrix OBJECTS are recognised without being read
-    (the usual case: a caller passes its R and P on every call); otherwise the plan is looked up by a digest
-    of the contents.  Callers on a hot loop can also hold the plan and pass it instead of R."""
+    (the usual case: a caller passes its R and P on every call) by where their data lives and three probe values
+    (tensors: the version counter), enough to notice the in-place edits that the digest would notice; otherwise the
+    plan is looked up by a digest of the contents.  Callers on a hot loop can also hold the plan and pass it instead of R."""
     if isinstance(rotation_matrix, DevicePlan):
         return rotation_matrix
-    dev = str(torch.device(device))
-    qr, qp = _quick_key(rotation_matrix), _quick_key(jl_matrix)
-    quick = (qr, qp, dev) if qr is not None and qp is not None else None
-    if quick is not None:
-        hit = _QUICK.get(quick)
-        if hit is not None:
-            return hit[0]
-    key = (_digest(rotation_matrix), _digest(jl_matrix), dev)
+    dev = torch.device(device)
+    index = -1 if dev.type != "cuda" else torch.cuda.current_device() if dev.index is None else dev.index
+    hit = _ext.host().plan_get(rotation_matrix, index, jl_matrix) if index >= 0 else None
+    if hit is not None:
+        return hit
+    key = (_digest(rotation_matrix), _digest(jl_matrix), index)
     plan = _PLANS.get(key)
     if plan is None:
         plan = DevicePlan(rotation_matrix, device, jl_matrix)
         _PLANS[key] = plan
-    if quick is not None:
-        if len(_QUICK) >= _QUICK_LIMIT:
-            _QUICK.pop(next(iter(_QUICK)))
-        _QUICK[quick] = (plan, rotation_matrix, jl_matrix)      # the references keep the ids from being reused
+    if index >= 0:
+        _ext.host().plan_put(rotation_matrix, index, jl_matrix, plan)
     return plan

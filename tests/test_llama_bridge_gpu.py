@@ -189,8 +189,8 @@ def test_arguments_the_bridge_cannot_serve_are_reported():
 
 # edges of the tensor-core compress kernel: its smallest size, several tiles per CTA with a ragged last one, and
 # codebooks its bucket table cannot hold (descending, levels in one bucket), which are scanned
-@pytest.mark.parametrize("d,n,book", [(128, 1280, "normal"), (64, 1281, "normal"), (128, 60_011, "normal"),
-                                      (64, 130_049, "normal"), (128, 1500, "descending"), (64, 1500, "narrow")])
+@pytest.mark.parametrize("d,n,book", [(128, 4095, "normal"), (64, 513, "normal"), (128, 4096, "normal"), (64, 4097, "normal"), (128, 60_011, "normal"),
+                                      (64, 130_049, "normal"), (128, 4500, "descending"), (64, 4500, "narrow")])
 def test_compress_tensor_core_edges_vs_oracle(d, n, book):
     from polarquant_kv import _ext
     from polarquant_kv import llama_bridge as LB
