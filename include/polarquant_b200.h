@@ -130,7 +130,7 @@ int pq_compress_rows_dynamic(const void* x, int64_t n_rows, int64_t tokens_per_r
  * pq_lse_exchange_merge (a peer's records did not arrive within about two seconds; the output rows of the
  * waiting CTAs are left unwritten), bit 8 the llama.cpp bridge's attention (a wait for a tile copy gave up),
  * bit 9 the same kernel (shared-memory window unusable, nothing computed), bits 10 and 11 the same two of the
- * bridge's compress.
+ * bridge's compress, bit 12 dequantise (shared-memory window unusable).
  * The flags are cleared by the call.  No counterpart in the reference (its kernels report nothing). */
 int pq_poll_device_errors(unsigned int* flags_out);
 

@@ -699,7 +699,7 @@ extern "C" int pq_poll_device_errors(unsigned int* flags_out) {
     unsigned int cf = 0;
     const int sc = pq::bridge_compress_error_flags(&cf);
     if (sc != PQ_OK) return sc;
-    *flags_out = v | pf | (df << 3) | (qf << 6) | (xf << 7) | (bf << 8) | (cf << 10);
+    *flags_out = v | pf | (df << 3) | ((qf & 1u) << 6) | ((qf >> 1) << 12) | (xf << 7) | (bf << 8) | (cf << 10);
     return PQ_OK;
 }
 

@@ -1,70 +1,102 @@
-// pq_dequant: stored block_pq4 blocks -> centroid[idx] * float(d) (rotated space) ->
-// inverse rotation v @ R -> float32 or float16.
+// pq_dequant: stored block_pq4 blocks -> centroid[idx] * float(d) (rotated space) -> inverse rotation v @ R -> float32
+// or float16; and the same with another end, the expanded tiles of the prefill kernel (pq_expand.cuh).
 //
-// Follows dequantize_with_codebook (src/polarquant_kv_cuda/lloyd_max.py:93-98), the radius
-// restore of quantizer.decompress (python/polarquant_kv/quantizer.py:151) and
-// inverse_rotate (python/polarquant_kv/rotation.py:61); the float16 output is clamped to
-// +-65504 like decompress_gpu (src/polarquant_kv_cuda/decompress_kernel.py:47-51).
+// Follows dequantize_with_codebook (src/polarquant_kv_cuda/lloyd_max.py:93-98), the radius restore of
+// quantizer.decompress (python/polarquant_kv/quantizer.py:151) and inverse_rotate (python/polarquant_kv/rotation.py:61);
+// the float16 output is clamped to +-65504 like decompress_gpu (src/polarquant_kv_cuda/decompress_kernel.py:47-51).
 //
-// The inverse rotation is a [vectors x D] . [D x D] contraction on the 5th-generation tensor cores
-// (tcgen05.mma kind::f16, M = 128, accumulators in tensor memory) with both operands as two float16
-// terms and three product terms (hi*hi + hi*lo + lo*hi), which keeps float32-level accuracy (2e-6 of
-// a vector's largest component against the float64 reference).  A persistent CTA owns 128 vectors at a
-// time and runs the compress pipeline backwards:
-//   worker warps (4 per 32-dim block)  a thread dequantises one block of one vector - centroid * radius
-//       in float32 exactly as the reference, times a power of two per vector (so tiny vectors keep their
-//       precision) - and writes its hi and lo float16 terms as four 16-byte chunks each into the K-major
-//       A tiles in shared memory (two pairs of tiles: tile i+1 is produced while tile i is contracted);
-//       the stored bytes of the next tile are loaded before the epilogue so they are in flight;
-//   MMA warp  one lane issues, per tile, D/16 MMAs A_hi x [R_hi ; R_lo] (N = 2D: columns [0, D) receive
-//       hi*hi, [D, 2D) hi*lo) and D/16 MMAs A_lo x R_hi on top of the first D columns; tcgen05.commit
-//       releases the A tiles and hands the accumulator (one of two) to the epilogue;
-//   the same worker warps, one tile behind, read their 32 output columns of both halves from tensor
-//       memory (thread = vector), add, rescale and store 64 or 128 contiguous bytes per vector.
-// R is split into the two float16 terms of 4096 R and laid out as the B operand once per CTA.
+// The inverse rotation is a [vectors x D] . [D x D] contraction on the 5th-generation tensor cores (tcgen05.mma kind::f16,
+// M = 128) with both operands as two float16 terms and three product terms (lo*hi, hi*lo, then hi*hi into the same
+// float32 accumulator), which keeps float32-level accuracy (2e-6 of a vector's largest component).
+//
+// Bound: HBM, 72 bytes in and 256 or 512 out per vector of 128 (4-bit).  A persistent CTA owns 128 vectors at a time:
+//   copy warp     the tile's stored bytes (contiguous), by bulk copy, four tiles in flight (by 4- or 8-byte asynchronous
+//                 copies where a row does not start on a 16-byte boundary);
+//   worker warps  (4 per 32-dim block) a thread owns one vector x one block: a stored byte is one lookup of its centroids'
+//                 hi and lo float16 terms (256-byte table rows at a fixed shared address, 16 private copies, so a byte
+//                 becomes an address with one byte-permute and lookups never conflict), times the radius as an error-free
+//                 float16 product (hi = h x d, lo = l x d + (h x d - hi)), and goes into tensor memory as the A operand
+//                 (two buffers) - nothing is staged through shared memory;
+//   MMA warp      3 x D/16 MMAs per tile (1.5 K cycles at D = 128; HBM needs 1.8 K for the float16 output);
+//   the same worker warps, one tile behind, read their vector's 32 accumulator columns, scale, and send the results off
+//                 through swizzled shared memory by TMA (stores straight from the threads, one vector's 32 bytes per lane,
+//                 took two thirds of the load-store pipe: 136 us against the figure below).
+// A power of two per vector keeps the largest radius in [1, 2) inside, so tiny vectors keep their precision.
 // All waits are bounded (a lost completion sets an error flag instead of hanging).
-// Bound: 72 B in + 256 or 512 B out per vector (HBM).
+#include <cstring>
+
+#include "pq_expand.cuh"
 #include "pq_tcgen05.cuh"
 
 namespace pq {
 
 constexpr int kDqVecs = 128;
+constexpr float kDqCbScale = 64.0f;          // centroids sit x64 in the table (keeps the lo terms normal)
 
-// bit 0: a bounded wait gave up (read and cleared through pq_poll_device_errors, bit 6 there)
+// bit 0: a bounded wait gave up; bit 1: shared-memory window unusable (pq_poll_device_errors, bits 6 and 12 there)
 static __device__ unsigned int g_dequant_error = 0;
 
 struct DequantParams {
-    const uint8_t* blocks;
+    const uint8_t* blocks[2];    // expand: K and V; else the one tensor
     const float* rot;
     void* out;
-    int64_t n_vec;
+    int64_t n_vec;               // plain: vectors
+    int64_t n_items;             // tiles of 128 vectors (expand: of both operands)
     int out_is_fp16;
+    int aligned;                 // rows start on 16-byte boundaries
+    // expand: tokens per row, row capacity, 128-token tiles per row, items per operand, first operand
+    int64_t S, Scap;
+    int row_tiles, operand_items, operand0;
+    float score_scale;
     float cb[16];
 };
 
 template <int D>
 struct DequantCfg {
     static constexpr int NBLK = D / 32;
-    static constexpr int kWorkers = 32 * 4 * NBLK;                // one thread per (vector, block)
-    static constexpr int kThreads = kWorkers + 32;                // + the MMA warp
-    static constexpr int kATile = kDqVecs * D * 2;                // one float16 term of a 128-vector tile
-    static constexpr int kBBytes = 2 * D * D * 2;                 // [R_hi ; R_lo] as the stacked B operand
-    static constexpr int kAccCols = 2 * D;                        // accumulator columns per buffer
-    static constexpr int kWarpSegMax = (32 / NBLK) * NBLK * 18;   // packed bytes of a warp's vectors, 4-bit (576)
-    // A tiles (2 buffers x 2 terms) | B | codebook copies | per-vector scales (4 tiles) | the warps' packed
-    // bytes | barriers | alignment
-    static constexpr size_t smem_bytes() {
-        return 4 * (size_t)kATile + kBBytes + 16 * 32 * 4 + 4 * kDqVecs * 4 + (kWorkers / 32) * kWarpSegMax + 128 + 128;
-    }
+    static constexpr int kWorkers = 128 * NBLK;                   // one thread per (vector, block)
+    static constexpr int kThreads = kWorkers + 64;                // + MMA warp + copy warp
+    static constexpr int kRing = 4;                               // tiles of stored bytes in flight or in use
+    static constexpr uint32_t kSlot = kDqVecs * NBLK * 18;        // stored bytes of a tile at 4 bits
+    // [window start: ring, barriers][0x10000: table rows of 256 bytes, their upper halves hold the core matrices of R_hi]
+    // [0x20000: R_lo][results on their way out]
+    static constexpr uint32_t kTabAddr = 0x10000u, kBLoAddr = 0x20000u, kBTerm = 2u * D * D;
+    static constexpr uint32_t kOutAddr = kBLoAddr + kBTerm, kOutBytes = kDqVecs * D * 4;
+    static constexpr uint32_t kLow = kRing * kSlot + 256 + 128;
+    static constexpr size_t smem_bytes() { return (size_t)kOutAddr + kOutBytes; }
+    static constexpr uint32_t kTmemCols = 4 * D;                  // A 2 x D, accumulators 2 x D
 };
 
-// Byte offset of 16-byte chunk `kc` of row `r` in a K-major operand tile with `rows` rows (8-row x 16-byte
-// core matrices, 128 bytes each; consecutive 8-row groups 128 bytes apart, consecutive K chunks rows/8 * 128).
-__device__ __forceinline__ uint32_t dq_chunk_off(int rows, int r, int kc) {
-    return (uint32_t)(kc * (rows / 8) * 128 + (r >> 3) * 128 + (r & 7) * 16);
+__device__ __forceinline__ void dq_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};\n" ::"r"(taddr),
+                 "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+                 "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+                 : "memory");
 }
-
-// packed float32x2 arithmetic: two round-to-nearest operations per instruction
+// Two float16 terms of (h + l) x d per half: the product h x d is split without error.
+__device__ __forceinline__ void dq_scaled(uint32_t h, uint32_t l, __half2 d, uint32_t& hi, uint32_t& lo) {
+    const __half2 H = *reinterpret_cast<const __half2*>(&h), L = *reinterpret_cast<const __half2*>(&l);
+    const __half2 p = __hmul2(H, d);
+    const __half2 q = __hfma2(L, d, __hfma2(H, d, __hneg2(p)));
+    hi = *reinterpret_cast<const uint32_t*>(&p);
+    lo = *reinterpret_cast<const uint32_t*>(&q);
+}
+__device__ __forceinline__ uint32_t dq_lds_u16(uint32_t a) {
+    uint32_t v;
+    asm volatile("{ .reg .u16 t; ld.shared.u16 t, [%1]; cvt.u32.u16 %0, t; }\n" : "=r"(v) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ uint32_t dq_lds_u32(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a));
+    return v;
+}
+// pack two floats as float16, values outside the range clamped to +-65504
+__device__ __forceinline__ uint32_t dq_pack_sat(float lo, float hi) {
+    uint32_t w;
+    asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;\n" : "=r"(w) : "f"(hi), "f"(lo));
+    return w;
+}
 __device__ __forceinline__ float2 dq_mul2(float2 a, float2 b) {
     float2 d;
     asm("mul.rn.f32x2 %0, %1, %2;\n"
@@ -72,259 +104,362 @@ __device__ __forceinline__ float2 dq_mul2(float2 a, float2 b) {
         : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
     return d;
 }
-__device__ __forceinline__ float2 dq_fma2(float2 a, float2 b, float2 c) {
+__device__ __forceinline__ float2 dq_sub2(float2 a, float2 b) {            // a - b
     float2 d;
+    const float2 m = make_float2(-1.f, -1.f);
     asm("fma.rn.f32x2 %0, %1, %2, %3;\n"
         : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)),
-          "l"(*reinterpret_cast<unsigned long long*>(&c)));
+        : "l"(*reinterpret_cast<unsigned long long*>(&b)), "l"(*reinterpret_cast<const unsigned long long*>(&m)),
+          "l"(*reinterpret_cast<unsigned long long*>(&a)));
     return d;
 }
-
-// 32 bytes to global memory at a 32-byte boundary in one instruction
-__device__ __forceinline__ void stg_256(void* dst, const uint32_t (&w)[8]) {
-    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};\n" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]),
-                 "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                 : "memory");
+__device__ __forceinline__ void dq_sts4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-template <int D, int BITS>
-__global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(const DequantParams p) {
+// EXPAND: the output is the prefill kernel's records instead of vectors.
+template <int D, int BITS, bool EXPAND>
+__global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(const DequantParams p, const __grid_constant__ CUtensorMap out_map) {
     using C = DequantCfg<D>;
-    constexpr int NBLK = C::NBLK;
-    constexpr int BB = block_bytes(BITS);
-    constexpr int VB = NBLK * BB;
-    constexpr int WORKERS = C::kWorkers;
+    constexpr int NBLK = C::NBLK, WORKERS = C::kWorkers, RING = C::kRing;
+    constexpr int BB = block_bytes(BITS), VB = NBLK * BB;
     extern __shared__ __align__(128) uint8_t smem_raw[];
-    uint8_t* sp = smem_raw + ((128u - (sm_addr(smem_raw) & 127u)) & 127u);
-    uint8_t* a_tiles = sp;                      sp += 4 * C::kATile;      // [buffer][term]
-    uint8_t* b_tile = sp;                       sp += C::kBBytes;
-    float* cbs = reinterpret_cast<float*>(sp);  sp += 16 * 32 * 4;        // a copy of the codebook per lane
-    // [tile & 3][vector] power-of-two scale.  A worker may already produce tile i + 1 while another still
-    // reads the scales of tile i - 2 in its epilogue (tile i + 2 cannot start before that: its A tiles are
-    // free only after the MMAs of tile i, which need every worker's tile i), hence four slots.
-    float* vscale = reinterpret_cast<float*>(sp); sp += 4 * kDqVecs * 4;
-    uint8_t* segs = sp;                         sp += (C::kWorkers / 32) * C::kWarpSegMax;   // [warp] packed bytes
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(sp);
-    // [0], [1]: A tiles of buffer b written; [2], [3]: A tiles of buffer b consumed by their MMAs;
-    // [4], [5]: accumulator b complete; [6], [7]: accumulator b read out by every worker
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(mbar + 8);
-    volatile uint32_t* abort_s = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
-
+    const uint32_t base = (sm_addr(smem_raw) + 127u) & ~127u;
+    uint8_t* zero = smem_raw - sm_addr(smem_raw);                  // generic address of shared address 0
+    if (base + C::kLow > C::kTabAddr) {
+        if (threadIdx.x == 0) atomicOr(&g_dequant_error, 2u);
+        return;
+    }
+    const uint32_t ring = base;
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(zero + base + RING * C::kSlot);
+    // stored bytes landed / read, per ring slot; A buffer written; its MMAs done (A free, accumulator complete);
+    // accumulator read out
+    uint64_t *in_full = mbar, *in_free = mbar + RING, *a_full = mbar + 2 * RING, *mma_done = a_full + 2, *acc_free = a_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_full + 6);
+    volatile uint32_t* abort_s = tmem_slot + 1;
+    uint32_t* cs = tmem_slot + 4;                                  // 16 split centroids
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 
-    // ---- set-up: B = [R_hi ; R_lo] with B[n][k] = 4096 R[k][n] (out[v][n] = sum_k x[v][k] R[k][n])
-    for (int e = tid; e < D * D; e += C::kThreads) {
-        const int k = e / D, n = e - k * D;                               // coalesced along n
-        const float v = p.rot[e] * 4096.f;
-        const __half h = __float2half_rn(v);
-        const __half l = __float2half_rn(v - __half2float(h));
-        const uint32_t off = dq_chunk_off(2 * D, n, k >> 3) + (k & 7) * 2;
-        *reinterpret_cast<__half*>(b_tile + off) = h;
-        *reinterpret_cast<__half*>(b_tile + off + dq_chunk_off(2 * D, D, 0)) = l;      // rows D .. 2D-1
-    }
-    for (int e = tid; e < 16 * 32; e += C::kThreads) cbs[e] = p.cb[e >> 5];
+    // ---- set-up
     if (tid == 0) {
-        for (int i = 0; i < 2; ++i) mbar_init(sm_addr(mbar + i), WORKERS);
-        for (int i = 2; i < 6; ++i) mbar_init(sm_addr(mbar + i), 1);
-        for (int i = 6; i < 8; ++i) mbar_init(sm_addr(mbar + i), WORKERS);
+        for (int i = 0; i < RING; ++i) {
+            mbar_init(sm_addr(in_full + i), 32);                   // every lane of the copy warp
+            mbar_init(sm_addr(in_free + i), WORKERS);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(sm_addr(a_full + i), WORKERS);
+            mbar_init(sm_addr(mma_done + i), 1);
+            mbar_init(sm_addr(acc_free + i), WORKERS);
+        }
         *abort_s = 0u;
     }
-    if (warp == 0) tmem_alloc(sm_addr(tmem_slot), 2 * C::kAccCols);
-    fence_async_smem();          // B is read by the tensor core through the async proxy
+    if (tid < 16) {
+        __half h, l;
+        split_half(p.cb[tid] * kDqCbScale, h, l);
+        cs[tid] = (uint32_t)__half_as_ushort(h) | ((uint32_t)__half_as_ushort(l) << 16);
+    }
+    // B terms, K-major core matrices: B[n][k] = 4096 R[k][n]  (out[v][n] = sum_k x[v][k] R[k][n]); lanes along n
+    for (int e = tid; e < D * (D / 8); e += C::kThreads) {
+        const int n = e % D, kc = e / D;
+        uint32_t h[4], l[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const float x0 = __ldg(p.rot + (size_t)(kc * 8 + 2 * u) * D + n) * 4096.f;
+            const float x1 = __ldg(p.rot + (size_t)(kc * 8 + 2 * u + 1) * D + n) * 4096.f;
+            const __half2 hh = __floats2half2_rn(x0, x1);
+            const float2 f = __half22float2(hh);
+            h[u] = *reinterpret_cast<const uint32_t*>(&hh);
+            l[u] = pack_half2(x0 - f.x, x1 - f.y);
+        }
+        const uint32_t m = (uint32_t)(kc * (D / 8) + (n >> 3)), in = (uint32_t)(n & 7) * 16;     // core matrix, row
+        *reinterpret_cast<uint4*>(zero + C::kTabAddr + m * 256 + 128 + in) = make_uint4(h[0], h[1], h[2], h[3]);
+        *reinterpret_cast<uint4*>(zero + C::kBLoAddr + m * 128 + in) = make_uint4(l[0], l[1], l[2], l[3]);
+    }
+    if (warp == 0) tmem_alloc(sm_addr(tmem_slot), C::kTmemCols);
+    __syncthreads();
+    // table: row r (256 bytes) = the centroid pairs of byte r, {hi pair, lo pair}
+    if (BITS == 4) {
+        for (int e = tid; e < 256 * 16; e += C::kThreads) {
+            const int b = e >> 4;
+            const uint32_t c0 = cs[b & 15], c1 = cs[b >> 4];
+            *reinterpret_cast<uint2*>(zero + C::kTabAddr + b * 256 + (e & 15) * 8) =
+                make_uint2(__byte_perm(c0, c1, 0x5410), __byte_perm(c0, c1, 0x7632));
+        }
+    } else {
+        for (int e = tid; e < 256 * 8; e += C::kThreads) {
+            const int b = e >> 3;
+            const uint32_t c0 = cs[b & 3], c1 = cs[(b >> 2) & 3], c2 = cs[(b >> 4) & 3], c3 = cs[b >> 6];
+            *reinterpret_cast<uint4*>(zero + C::kTabAddr + b * 256 + (e & 7) * 16) =
+                make_uint4(__byte_perm(c0, c1, 0x5410), __byte_perm(c0, c1, 0x7632),
+                           __byte_perm(c2, c3, 0x5410), __byte_perm(c2, c3, 0x7632));
+        }
+    }
+    fence_async_smem();                                            // B is read by the tensor core through the async proxy
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-
-    const int64_t n_tiles = (p.n_vec + kDqVecs - 1) / kDqVecs;
-    const int64_t n_my = (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x;      // tiles of this CTA
+    const int n_my = (int)((p.n_items - blockIdx.x + gridDim.x - 1) / gridDim.x);
     bool ok = true;
+    // first stored byte and number of vectors of the i-th tile of this CTA
+    struct Item { int64_t at; int n; int operand, row, tile; };
+    auto item = [&](int i) -> Item {
+        const int64_t it = (int64_t)blockIdx.x + (int64_t)i * gridDim.x;
+        Item r;
+        if (EXPAND) {
+            const int op = it >= p.operand_items ? 1 : 0, k = (int)(it - (int64_t)op * p.operand_items);
+            r.operand = p.operand0 + op;
+            r.row = k / p.row_tiles;
+            r.tile = k - r.row * p.row_tiles;
+            const int64_t tok = (int64_t)r.tile * kDqVecs;
+            r.at = ((int64_t)r.row * p.Scap + tok) * VB;
+            r.n = (int)min((int64_t)kDqVecs, p.S - tok);
+        } else {
+            r.operand = r.row = r.tile = 0;
+            r.at = it * kDqVecs * VB;
+            r.n = (int)min((int64_t)kDqVecs, p.n_vec - it * kDqVecs);
+        }
+        return r;
+    };
 
     if (warp == WORKERS / 32) {
-        // ---- MMA warp: every lane runs the loop (uniform waits and descriptor arithmetic), lane 0 issues
-        constexpr uint32_t idesc_full = umma_idesc_f16(2 * D), idesc_half = umma_idesc_f16(D);
-        constexpr uint32_t kLboA = (kDqVecs / 8) * 128, kLboB = (2 * D / 8) * 128;   // K-chunk strides
-        constexpr uint32_t d_hi = (128u >> 4) | (1u << 14);                         // 8-row groups 128 B apart, no swizzle
-        const uint32_t b_lo0 = ((sm_addr(b_tile) >> 4) & 0x3FFFu) | ((kLboB >> 4) << 16);
+        // ---- MMA warp: every lane runs the loop, lane 0 issues
+        constexpr uint32_t idesc = umma_idesc_f16(D);
+        // no swizzle; core matrices 256 B apart (R_hi, between the table rows) or 128 B (R_lo), K chunks D / 8 of them
+        constexpr uint32_t hi_step = (D / 8) * 256, lo_step = (D / 8) * 128;
+        constexpr uint32_t hi_d = (256u >> 4) | (1u << 14), lo_d = (128u >> 4) | (1u << 14);
+        const uint32_t hi0 = (((C::kTabAddr + 128) >> 4) & 0x3FFFu) | ((hi_step >> 4) << 16);
+        const uint32_t lo0 = ((C::kBLoAddr >> 4) & 0x3FFFu) | ((lo_step >> 4) << 16);
         const uint32_t issue = lane == 0 ? 1u : 0u;
-        for (int64_t i = 0; i < n_my && ok; ++i) {
-            const uint32_t b = (uint32_t)(i & 1), use = (uint32_t)(i >> 1);
-            ok = mbar_wait(sm_addr(mbar + b), use & 1u, abort_s, 32) && ok;                       // A written
-            if (i >= 2) ok = mbar_wait(sm_addr(mbar + 6 + b), (use - 1u) & 1u, abort_s, 32) && ok;   // accumulator free
+        for (int i = 0; i < n_my && ok; ++i) {
+            const uint32_t b = i & 1, use = (uint32_t)i >> 1;
+            ok = mbar_wait(sm_addr(a_full + b), use & 1u, abort_s, 32) && ok;
+            if (i >= 2) ok = mbar_wait(sm_addr(acc_free + b), (use - 1u) & 1u, abort_s, 32) && ok;
             if (!ok) break;
             tc_fence_after();
-            const uint32_t acc = tmem_base + b * C::kAccCols;
-            const uint32_t ah0 = ((sm_addr(a_tiles + (2 * b) * C::kATile) >> 4) & 0x3FFFu) | ((kLboA >> 4) << 16);
-            const uint32_t al0 = ((sm_addr(a_tiles + (2 * b + 1) * C::kATile) >> 4) & 0x3FFFu) | ((kLboA >> 4) << 16);
+            const uint32_t a = tmem_base + b * D, acc = tmem_base + 2 * D + b * D;
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks)          // a k-step is two 16-byte chunks
-                umma_f16_split_pred(acc, ah0 + ks * ((2 * kLboA) >> 4), d_hi, b_lo0 + ks * ((2 * kLboB) >> 4), d_hi,
-                                    idesc_full, ks ? 1u : 0u, issue);
+            for (int t = 0; t < 3; ++t)                            // lo x hi, hi x lo, hi x hi
 #pragma unroll
-            for (int ks = 0; ks < D / 16; ++ks)          // lo term of the vectors x hi term of R: the first D rows of B
-                umma_f16_split_pred(acc, al0 + ks * ((2 * kLboA) >> 4), d_hi, b_lo0 + ks * ((2 * kLboB) >> 4), d_hi,
-                                    idesc_half, 1u, issue);
-            umma_commit_pred(sm_addr(mbar + 2 + b), issue);      // the A tiles may be overwritten
-            umma_commit_pred(sm_addr(mbar + 4 + b), issue);      // the accumulator is complete
+                for (int ks = 0; ks < D / 16; ++ks)
+                    umma_f16_ts_pred(acc, a + (t == 0 ? D / 2 : 0) + ks * 8,
+                                     t == 1 ? lo0 + ((2 * ks * lo_step) >> 4) : hi0 + ((2 * ks * hi_step) >> 4),
+                                     t == 1 ? lo_d : hi_d, idesc, (t || ks) ? 1u : 0u, issue);
+            umma_commit_pred(sm_addr(mma_done + b), issue);
+            __syncwarp();
         }
-        if (!ok && lane == 0) { *abort_s = 1u; atomicOr(&g_dequant_error, 1u); }
-    } else {
-        // ---- worker warps
-        // produce: this thread's (vector, block).  Eight neighbouring lanes own eight neighbouring vectors
-        // of the same block, so that their 16-byte chunk stores into the A tiles fill 128 contiguous bytes
-        // (a quarter warp per shared-memory wavefront, no bank conflicts); the blocks of a vector sit
-        // 32 / NBLK lanes apart.
-        constexpr int VPW = 32 / NBLK;                            // vectors per warp
-        const int vec = warp * VPW + (lane % VPW), blk = lane / VPW;
-        const int q = warp & 3, cc = warp >> 2;                   // epilogue: TMEM lane quarter, 32-column chunk
-        const int row = 32 * q + lane;
-        const uint32_t tmem_lane = tmem_base + ((uint32_t)(32 * q) << 16);
-        // The stored bytes of a warp's VPW vectors are one contiguous segment of VPW * VB bytes (576 or 320):
-        // the warp loads it as 16-byte pieces, one or two per lane, a tile ahead, and passes it through a
-        // shared-memory slot from which every thread picks its block (18 or 10 bytes at a 2-byte boundary).
-        constexpr int kSeg = VPW * VB;                            // a multiple of 16
-        constexpr int kPieces = kSeg / 16;                        // 36 or 20
-        const int64_t total_bytes = p.n_vec * VB;
-        uint4 piece0 = make_uint4(0u, 0u, 0u, 0u), piece1 = make_uint4(0u, 0u, 0u, 0u);
-        auto load_piece = [&](int64_t byte0) -> uint4 {           // 16 bytes at a 16-byte boundary, zeros past the end
-            uint4 r = make_uint4(0u, 0u, 0u, 0u);
-            if (byte0 + 16 <= total_bytes) {
-                r = __ldg(reinterpret_cast<const uint4*>(p.blocks + byte0));
-            } else if (byte0 < total_bytes) {                     // the last piece of the tensor: 2-byte loads
-                uint32_t w[4] = {0u, 0u, 0u, 0u};
-                for (int h = 0; h < 8 && byte0 + 2 * h < total_bytes; ++h)
-                    w[h >> 1] |= (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(p.blocks + byte0) + h) << (16 * (h & 1));
-                r = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-            return r;
-        };
-        auto fetch = [&](int64_t tile) {
-            const int64_t seg0 = (tile * kDqVecs + (int64_t)warp * VPW) * VB;
-            piece0 = lane < kPieces ? load_piece(seg0 + 16 * lane) : make_uint4(0u, 0u, 0u, 0u);
-            piece1 = 32 + lane < kPieces ? load_piece(seg0 + 16 * (32 + lane)) : make_uint4(0u, 0u, 0u, 0u);
-        };
-        uint8_t* seg = segs + warp * C::kWarpSegMax;
-        uint32_t words[BITS];                                     // 32 packed indices of this thread's block
-        float d_cur = 0.f;
-        auto unpack_block = [&]() {                               // registers -> slot -> this thread's block
-            __syncwarp();
-            if (lane < kPieces) *reinterpret_cast<uint4*>(seg + 16 * lane) = piece0;
-            if (32 + lane < kPieces) *reinterpret_cast<uint4*>(seg + 16 * (32 + lane)) = piece1;
-            __syncwarp();
-            const int off = (lane % VPW) * VB + blk * BB;         // 2-byte aligned; 4-byte aligned for even blocks
-            const uint32_t* w32 = reinterpret_cast<const uint32_t*>(seg + (off & ~3));
-            uint32_t w[BITS + 1];
-#pragma unroll
-            for (int k = 0; k <= BITS; ++k) w[k] = w32[k];
-            if (off & 2) {
-                d_cur = __half2float(__ushort_as_half((unsigned short)(w[0] >> 16)));
-#pragma unroll
-                for (int k = 0; k < BITS; ++k) words[k] = w[k + 1];
-            } else {
-                d_cur = __half2float(__ushort_as_half((unsigned short)(w[0] & 0xFFFFu)));
-#pragma unroll
-                for (int k = 0; k < BITS; ++k) words[k] = __funnelshift_r(w[k], w[k + 1], 16);
-            }
-        };
-        auto epilogue = [&](int64_t i) {                          // tile number i of this CTA
-            const uint32_t b = (uint32_t)(i & 1), use = (uint32_t)(i >> 1);
-            ok = mbar_wait(sm_addr(mbar + 4 + b), use & 1u, abort_s) && ok;
-            if (!ok) return;
-            tc_fence_after();
-            float hi[32], lo[32];
-            tmem_ld32(hi, tmem_lane + b * C::kAccCols + cc * 32);
-            tmem_ld32(lo, tmem_lane + b * C::kAccCols + D + cc * 32);
-            tc_fence_before();
-            mbar_arrive(sm_addr(mbar + 6 + b));                   // this thread's part of the accumulator is in registers
-            const int64_t tile = (int64_t)blockIdx.x + i * gridDim.x;
-            const int64_t v = tile * kDqVecs + row;
-            if (v >= p.n_vec) return;
-            const float s = vscale[(i & 3) * kDqVecs + row] * (1.0f / 4096.f);
-            const size_t off = (size_t)v * D + cc * 32;
-            // 32-byte stores: every store instruction of a thread fills a whole sector
-            if (p.out_is_fp16) {
-                __half* dst = static_cast<__half*>(p.out) + off;
-#pragma unroll
-                for (int j = 0; j < 32; j += 16) {
-                    uint32_t w[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const float a = (hi[j + 2 * u] + lo[j + 2 * u]) * s, c = (hi[j + 2 * u + 1] + lo[j + 2 * u + 1]) * s;
-                        w[u] = pack_half2(fminf(fmaxf(a, -65504.f), 65504.f), fminf(fmaxf(c, -65504.f), 65504.f));
-                    }
-                    stg_256(dst + j, w);
-                }
-            } else {
-                float* dst = static_cast<float*>(p.out) + off;
-#pragma unroll
-                for (int j = 0; j < 32; j += 8) {
-                    uint32_t w[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) w[u] = __float_as_uint((hi[j + u] + lo[j + u]) * s);
-                    stg_256(dst + j, w);
-                }
-            }
-        };
-        fetch(blockIdx.x);
-        for (int64_t i = 0; i < n_my && ok; ++i) {
-            const uint32_t b = (uint32_t)(i & 1), use = (uint32_t)(i >> 1);
-            // ---- produce tile i: its A tiles must have been consumed by the MMAs of tile i - 2
-            if (i >= 2) ok = mbar_wait(sm_addr(mbar + 2 + b), (use - 1u) & 1u, abort_s) && ok;
+    } else if (warp == WORKERS / 32 + 1) {
+        // ---- copy warp
+        int slot = 0;
+        uint32_t round = 0;
+        for (int i = 0; i < n_my && ok; ++i) {
+            if (round) ok = mbar_wait(sm_addr(in_free + slot), (round - 1u) & 1u, abort_s, 32) && ok;
             if (!ok) break;
+            const Item it = item(i);
+            const uint8_t* src = p.blocks[EXPAND ? it.operand : 0] + it.at;
+            const uint32_t dst = ring + slot * C::kSlot, bar = sm_addr(in_full + slot);
+            if (p.aligned && it.n == kDqVecs) {
+                if (lane == 0) {
+                    mbar_expect_tx(bar, kDqVecs * VB);
+                    bulk_load(dst, src, kDqVecs * VB, bar);
+                } else {
+                    mbar_arrive(bar);
+                }
+            } else {
+                // 4-byte asynchronous copies (vectors are multiples of 4 bytes); the barrier counts every lane's
+                for (int c = lane; c < it.n * VB / 4; c += 32)
+                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + 4 * c), "l"(src + 4 * c));
+                asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];\n" ::"r"(bar) : "memory");
+            }
+            __syncwarp();
+            if (++slot == RING) { slot = 0; ++round; }
+        }
+    } else {
+        // ---- workers: vector `row` of the tile (= TMEM lane), block `wg`
+        const int wg = warp >> 2, q = warp & 3, row = 32 * q + lane;
+        const uint32_t tmem_lane = tmem_base + ((uint32_t)(32 * q) << 16);
+        const uint32_t tab_lane = C::kTabAddr | (BITS == 4 ? (lane & 15) * 8 : (lane & 7) * 16);
+        float scale = 0.f;                                         // of the tile produced last
+        auto produce = [&](int i) {
+            const int slot = i % RING;
+            ok = mbar_wait(sm_addr(in_full + slot), (uint32_t)(i / RING) & 1u, abort_s) && ok;
+            const uint32_t vec = ring + slot * C::kSlot + row * VB, blk = vec + wg * BB;
+            uint32_t words[BITS], dbits, dmax = 0u;
             {
-                unpack_block();
-                const float d = d_cur;
-                // one power of two per vector: largest block radius -> [1, 2)
-                float dmax = d;
+                uint32_t w[BITS + 1];
+                const uint32_t a = blk & ~3u;
 #pragma unroll
-                for (int o = VPW; o < 32; o <<= 1) dmax = fmaxf(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-                const uint32_t be = __float_as_uint(dmax) >> 23;
-                const bool normal = be > 0 && be < 255;
-                const float sc = normal ? __uint_as_float((254u - be) << 23) : 1.0f;
-                if (blk == 0) vscale[(i & 3) * kDqVecs + vec] = normal ? __uint_as_float(be << 23) : 1.0f;
-                uint8_t* ah = a_tiles + (2 * b) * C::kATile;
-                uint8_t* al = ah + C::kATile;
-                const float2 ds2 = make_float2(d * sc, d * sc), neg1 = make_float2(-1.f, -1.f);
+                for (int k = 0; k <= BITS; ++k) w[k] = dq_lds_u32(a + 4 * k);
+                if (wg & 1) {                                      // the block starts in the upper half of a word
+                    dbits = w[0] >> 16;
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {                     // four 16-byte chunks of 8 elements
-                    uint32_t wh[4], wl[4];
+                    for (int k = 0; k < BITS; ++k) words[k] = w[k + 1];
+                } else {
+                    dbits = w[0] & 0xFFFFu;
+#pragma unroll
+                    for (int k = 0; k < BITS; ++k) words[k] = __funnelshift_r(w[k], w[k + 1], 16);
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < NBLK; ++j) dmax = max(dmax, dq_lds_u16(vec + j * BB));      // radii are not negative
+            mbar_arrive(sm_addr(in_free + slot));
+            // largest radius -> [1, 2)
+            const uint32_t be = __float_as_uint(__half2float(__ushort_as_half((unsigned short)dmax))) >> 23;
+            const bool normal = be > 0 && be < 255;
+            scale = normal ? __uint_as_float(be << 23) : 1.0f;
+            const float ds = __half2float(__ushort_as_half((unsigned short)dbits)) * (normal ? __uint_as_float((254u - be) << 23) : 1.0f);
+            const __half2 d2 = __float2half2_rn(ds);               // exact but for radii 2^-14 below the largest
+            uint32_t hi[16], lo[16];
+#pragma unroll
+            for (int k = 0; k < BITS; ++k)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t a = __byte_perm(words[k], tab_lane, 0x7604u | (j << 4));
+                    if (BITS == 4) {
+                        uint32_t h, l;
+                        asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];\n" : "=r"(h), "=r"(l) : "r"(a));
+                        dq_scaled(h, l, d2, hi[4 * k + j], lo[4 * k + j]);
+                    } else {
+                        uint32_t h0, l0, h1, l1;
+                        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(h0), "=r"(l0), "=r"(h1), "=r"(l1) : "r"(a));
+                        dq_scaled(h0, l0, d2, hi[8 * k + 2 * j], lo[8 * k + 2 * j]);
+                        dq_scaled(h1, l1, d2, hi[8 * k + 2 * j + 1], lo[8 * k + 2 * j + 1]);
+                    }
+                }
+            const uint32_t b = i & 1;
+            if (i >= 2) {                                          // the A buffer's MMAs (tile i - 2) are done
+                ok = mbar_wait(sm_addr(mma_done + b), (uint32_t)((i >> 1) - 1) & 1u, abort_s) && ok;
+                tc_fence_after();
+            }
+            dq_tmem_st16(tmem_lane + b * D + wg * 16, hi);
+            dq_tmem_st16(tmem_lane + b * D + D / 2 + wg * 16, lo);
+            asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+            tc_fence_before();
+            mbar_arrive(sm_addr(a_full + b));
+        };
+        auto epilogue = [&](int i, float sc) {                     // (every thread of the warp runs all of it)
+            const uint32_t b = i & 1;
+            ok = mbar_wait(sm_addr(mma_done + b), (uint32_t)(i >> 1) & 1u, abort_s) && ok;
+            tc_fence_after();
+            float2 v[16];
+            tmem_ld32(v, tmem_lane + 2 * D + b * D + wg * 32);
+            tc_fence_before();
+            mbar_arrive(sm_addr(acc_free + b));
+            const Item it = item(i);
+            if constexpr (EXPAND) {
+                // K: per 64 dims 64 hi rows then 64 lo rows of 128 bytes; V: the hi rows of all dims, then the lo rows
+                using E = ExpandRec<D>;
+                const int half = row >> 6, r = row & 63, pair = wg >> 1;
+                const bool in = row < it.n;                        // tokens past the end: zeros
+                const float s = in ? kExpScale / (kDqCbScale * 4096.f) : 0.f;
+                const uint32_t piece = C::kOutAddr + (uint32_t)(((half * (D / 64) + pair) * 2) * kExpTok * 128);
+                const uint32_t hi_row = piece + r * 128, lo_row = hi_row + kExpTok * 128;
+                const bool leader = !(wg & 1) && lane == 0;
+                const uint32_t bar = 1u + (uint32_t)(q * (D / 64) + pair);      // the two warps that share 32 rows of 64 dims
+                if (leader) bulk_wait_read();                      // its last stores have read the buffer
+                asm volatile("bar.sync %0, 64;\n" ::"r"(bar) : "memory");
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {                      // chunks of 8 dims
+                    uint32_t h[4], l[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        const int j = 8 * c + 2 * u;
-                        uint32_t i0, i1;
-                        if (BITS == 4) {
-                            i0 = (words[j >> 3] >> ((j & 7) * 4)) & 0xFu;
-                            i1 = (words[j >> 3] >> ((j & 7) * 4 + 4)) & 0xFu;
-                        } else {
-                            i0 = (words[j >> 4] >> ((j & 15) * 2)) & 0x3u;
-                            i1 = (words[j >> 4] >> ((j & 15) * 2 + 2)) & 0x3u;
-                        }
-                        // centroid * radius rounded once to float32 as the reference does; the power of two
-                        // rides on the radius (it commutes with that rounding)
-                        const float2 x = dq_mul2(make_float2(cbs[i0 * 32 + lane], cbs[i1 * 32 + lane]), ds2);
-                        const __half2 h = __floats2half2_rn(x.x, x.y);
-                        const float2 lo = dq_fma2(__half22float2(h), neg1, x);     // exact: x - float(h)
-                        wh[u] = *reinterpret_cast<const uint32_t*>(&h);
-                        wl[u] = pack_half2(lo.x, lo.y);
+                        float2 x = dq_mul2(v[4 * c + u], make_float2(s, s));
+                        if (!in) x = make_float2(0.f, 0.f);
+                        const __half2 hh = __floats2half2_rn(x.x, x.y);
+                        const float2 f = dq_sub2(x, __half22float2(hh));
+                        h[u] = *reinterpret_cast<const uint32_t*>(&hh);
+                        l[u] = pack_half2(f.x, f.y);
                     }
-                    const uint32_t off = dq_chunk_off(kDqVecs, vec, blk * 4 + c);
-                    *reinterpret_cast<uint4*>(ah + off) = make_uint4(wh[0], wh[1], wh[2], wh[3]);
-                    *reinterpret_cast<uint4*>(al + off) = make_uint4(wl[0], wl[1], wl[2], wl[3]);
+                    const uint32_t at = (uint32_t)((((wg & 1) * 4 + c) ^ (r & 7)) << 4);
+                    dq_sts4(hi_row + at, h[0], h[1], h[2], h[3]);
+                    dq_sts4(lo_row + at, l[0], l[1], l[2], l[3]);
+                }
+                fence_async_smem();
+                asm volatile("bar.sync %0, 64;\n" ::"r"(bar) : "memory");
+                const int tile64 = 2 * it.tile + half;
+                if (tile64 * kExpTok < p.S) {                      // (the second half of the last tile may not exist)
+                    const int n64 = (int)((p.S + kExpTok - 1) / kExpTok);
+                    uint8_t* rec = static_cast<uint8_t*>(p.out) + ((size_t)it.row * n64 + tile64) * E::kBytes;
+                    const uint32_t r0 = (uint32_t)(q & 1) * 32 * 128;
+                    if (leader) {
+                        uint8_t* dst = it.operand == 0 ? rec + pair * (2 * kExpTok * 128) : rec + 2 * E::kTerm + pair * (kExpTok * 128);
+                        bulk_store(dst + r0, piece + r0, 32 * 128);
+                        bulk_store(dst + (it.operand == 0 ? (uint32_t)kExpTok * 128 : E::kTerm) + r0, piece + kExpTok * 128 + r0, 32 * 128);
+                    }
+                    if (wg == 0) {
+                        float* f = reinterpret_cast<float*>(rec + E::kFactors);
+                        const float w = in ? sc : 0.f;
+                        if (it.operand == 0) {
+                            f[r] = w * (p.score_scale / kExpScale);
+                        } else {
+                            f[kExpTok + r] = w;
+                            const uint32_t mx = __reduce_max_sync(0xffffffffu, __float_as_uint(w));       // not negative
+                            if (lane == 0) f[2 * kExpTok + (q & 1)] = __uint_as_float(mx);
+                        }
+                    }
+                }
+            } else {
+                const float s = sc * (1.0f / (kDqCbScale * 4096.f));
+                const float2 s2 = make_float2(s, s);
+                const int64_t v0 = ((int64_t)blockIdx.x + (int64_t)i * gridDim.x) * kDqVecs + 32 * q;
+                // 32 vectors: rows of 128 bytes, 16-byte chunks swizzled as the tensor map says
+                if (p.out_is_fp16) {
+                    // 64 dims = rows of 128 bytes, shared by two warps (boxes of 64-byte rows are limited by the number of
+                    // rows a TMA unit stores: 98 us for 2^20 vectors)
+                    const uint32_t piece = C::kOutAddr + b * (C::kOutBytes / 2) + (uint32_t)((wg >> 1) * kDqVecs + 32 * q) * 128;
+                    const bool leader = !(wg & 1) && lane == 0;
+                    const uint32_t bar = 1u + (uint32_t)(q * (D / 64) + (wg >> 1));
+                    // (the pair's barrier of the tile in between orders this wait before the partner's writes too)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        uint32_t w[4];
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            const float2 x = dq_mul2(v[4 * c + u], s2);
+                            w[u] = dq_pack_sat(x.x, x.y);
+                        }
+                        dq_sts4(piece + lane * 128 + ((((wg & 1) * 4 + c) ^ (lane & 7)) << 4), w[0], w[1], w[2], w[3]);
+                    }
+                    fence_async_smem();
+                    if (leader) bulk_wait_read();                  // the store of the other buffer: free for the next tile
+                    asm volatile("bar.sync %0, 64;\n" ::"r"(bar) : "memory");
+                    if (leader && v0 < p.n_vec) tma_store_2d(&out_map, (wg >> 1) * 64, (int)v0, piece);
+                } else {
+                    const uint32_t piece = C::kOutAddr + (uint32_t)(wg * kDqVecs + 32 * q) * 128;
+                    if (lane == 0) bulk_wait_read();
+                    __syncwarp();
+#pragma unroll
+                    for (int c = 0; c < 8; ++c) {
+                        const float2 x = dq_mul2(v[2 * c], s2), y = dq_mul2(v[2 * c + 1], s2);
+                        dq_sts4(piece + lane * 128 + ((c ^ (lane & 7)) << 4), __float_as_uint(x.x), __float_as_uint(x.y),
+                                __float_as_uint(y.x), __float_as_uint(y.y));
+                    }
+                    fence_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && v0 < p.n_vec) tma_store_2d(&out_map, wg * 32, (int)v0, piece);
                 }
             }
-            fence_async_smem();                                   // the tensor core reads the tiles through the async proxy
-            mbar_arrive(sm_addr(mbar + b));
-            fetch((int64_t)blockIdx.x + (i + 1) * gridDim.x);     // in flight during the epilogue below
-            // ---- epilogue of the tile before
-            if (i >= 1) epilogue(i - 1);
+        };
+        float before = 0.f;                                        // scale of the tile in the epilogue
+        // (a wait that gave up lets the rest of the loop run through on garbage, waits returning at once, so that the two
+        // warps of a barrier stay together)
+        for (int i = 0; i < n_my; ++i) {
+            before = scale;
+            produce(i);
+            if (i >= 1) epilogue(i - 1, before);
+            if (!ok && lane == 0) *abort_s = 1u;
         }
-        if (ok && n_my >= 1) epilogue(n_my - 1);
-        if (!ok && lane == 0) { *abort_s = 1u; atomicOr(&g_dequant_error, 1u); }
+        if (n_my >= 1) epilogue(n_my - 1, scale);
+        if (lane == 0) bulk_wait_all();                            // stores in flight read shared memory
+    }
+    if (!ok && lane == 0) { *abort_s = 1u; atomicOr(&g_dequant_error, 1u); }
+    if (*abort_s && tid == 0) {                                    // give copies still in flight time to land
+        const long long t0 = clock64();
+        while (clock64() - t0 < (1ll << 20)) {}
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_base, 2 * C::kAccCols);
+    if (warp == 0) tmem_dealloc(tmem_base, C::kTmemCols);
 }
 
 // Read and clear this file's device error flag (for pq_poll_device_errors).
@@ -336,21 +471,64 @@ int dequant_error_flags(unsigned int* flags) {
     return PQ_OK;
 }
 
-template <int D, int BITS>
+template <int D, int BITS, bool EXPAND>
 static int launch_dequant(const DequantParams& p, cudaStream_t st) {
     using C = DequantCfg<D>;
-    const size_t smem = C::smem_bytes();
-    auto kern = pq_dequant_kernel<D, BITS>;
+    auto kern = pq_dequant_kernel<D, BITS, EXPAND>;
     static std::atomic<uint64_t> allowed{0};
-    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
+    if (allow_shared(kern, C::smem_bytes(), allowed) != cudaSuccess) return PQ_ERR_CUDA;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return PQ_ERR_CUDA;
-    const int64_t n_tiles = (p.n_vec + kDqVecs - 1) / kDqVecs;
-    const int grid = (int)(n_tiles < sms ? n_tiles : sms);          // persistent: one CTA per SM (tensor memory)
-    kern<<<grid, C::kThreads, smem, st>>>(p);
+    const int grid = (int)(p.n_items < sms ? p.n_items : sms);      // persistent: one CTA per SM (tensor memory)
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    if (!EXPAND) {
+        const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)p.n_vec}, strides[1] = {(cuuint64_t)D * (p.out_is_fp16 ? 2 : 4)};
+        const cuuint32_t box[2] = {p.out_is_fp16 ? 64u : 32u, 32u};
+        if (!encode_tensor_map_2d(&map, p.out_is_fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.out,
+                                  dims, strides, box))
+            return PQ_ERR_CUDA;
+    }
+    kern<<<grid, C::kThreads, C::smem_bytes(), st>>>(p, map);
     return cudaGetLastError() == cudaSuccess ? PQ_OK : PQ_ERR_CUDA;
+}
+
+template <int D>
+static int launch_expand(const DequantParams& p, int bits, cudaStream_t st) {
+    return bits == 4 ? launch_dequant<D, 4, true>(p, st) : launch_dequant<D, 2, true>(p, st);
+}
+
+int expand_launch(const ExpandArgs& a, int head_dim, int k_bits, int v_bits, cudaStream_t st) {
+    DequantParams p{};
+    p.blocks[0] = a.kb;
+    p.blocks[1] = a.vb;
+    p.rot = a.rot;
+    p.out = a.ws;
+    p.S = a.S;
+    p.Scap = a.Scap;
+    p.row_tiles = (int)((a.S + kDqVecs - 1) / kDqVecs);
+    p.operand_items = a.rows * p.row_tiles;
+    p.score_scale = a.score_scale;
+    const int nblk = head_dim / 32;
+    auto row_aligned = [&](const uint8_t* b, int bits) {
+        return ((reinterpret_cast<uintptr_t>(b) | (uintptr_t)(a.Scap * nblk * block_bytes(bits))) & 15) == 0;
+    };
+    const bool ka = row_aligned(a.kb, k_bits), va = row_aligned(a.vb, v_bits);
+    // one launch when the operands share a table
+    bool same = k_bits == v_bits;
+    for (int i = 0; same && i < (1 << k_bits); ++i) same = a.codebook_k[i] == a.codebook_v[i];
+    for (int op = 0; op < (same ? 1 : 2); ++op) {
+        const int bits = op ? v_bits : k_bits;
+        p.operand0 = op;
+        p.n_items = (int64_t)p.operand_items * (same ? 2 : 1);
+        p.aligned = same ? ka && va : op ? va : ka;
+        for (int i = 0; i < 16; ++i) p.cb[i] = i < (1 << bits) ? (op ? a.codebook_v : a.codebook_k)[i] : 0.f;
+        const int s = head_dim == 64 ? launch_expand<64>(p, bits, st) : launch_expand<128>(p, bits, st);
+        if (s != PQ_OK) return s;
+    }
+    return PQ_OK;
 }
 
 }  // namespace pq
@@ -363,18 +541,21 @@ extern "C" int pq_dequant(const void* blocks, int64_t n_vec, int head_dim, int n
     if (head_dim != 64 && head_dim != 128) return PQ_ERR_BAD_HEAD_DIM;
     if (n_bits != 2 && n_bits != 4) return PQ_ERR_BAD_BITS;
     if (n_vec == 0) return PQ_OK;
+    if (n_vec > (int64_t)0x7FFFFF00) return PQ_ERR_TOO_LARGE;      // tile coordinates are 32-bit
     if (!blocks || !codebook || !rot || !out) return PQ_ERR_NULL_POINTER;
     if ((reinterpret_cast<uintptr_t>(blocks) & 15) || (reinterpret_cast<uintptr_t>(rot) & 15) ||
         (reinterpret_cast<uintptr_t>(out) & 31))
         return PQ_ERR_MISALIGNED;
     DequantParams p{};
-    p.blocks = static_cast<const uint8_t*>(blocks);
+    p.blocks[0] = static_cast<const uint8_t*>(blocks);
+    p.n_items = (n_vec + kDqVecs - 1) / kDqVecs;
+    p.aligned = 1;
     p.rot = rot;
     p.out = out;
     p.n_vec = n_vec;
     p.out_is_fp16 = out_is_fp16;
     for (int i = 0; i < 16; ++i) p.cb[i] = i < (1 << n_bits) ? codebook[i] : 0.f;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (head_dim == 64) return n_bits == 4 ? launch_dequant<64, 4>(p, st) : launch_dequant<64, 2>(p, st);
-    return n_bits == 4 ? launch_dequant<128, 4>(p, st) : launch_dequant<128, 2>(p, st);
+    if (head_dim == 64) return n_bits == 4 ? launch_dequant<64, 4, false>(p, st) : launch_dequant<64, 2, false>(p, st);
+    return n_bits == 4 ? launch_dequant<128, 4, false>(p, st) : launch_dequant<128, 2, false>(p, st);
 }

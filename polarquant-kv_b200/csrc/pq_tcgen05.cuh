@@ -41,6 +41,13 @@ __device__ __forceinline__ void bulk_store(void* gdst, uint32_t smem_src, uint32
                  : "memory");
     asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
 }
+// One box from shared memory through a 2-D tensor map (rows past the end are not written); commits its own group.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t smem_src) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];\n" ::"l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(x), "r"(y), "r"(smem_src)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;\n" ::: "memory");
+}
 __device__ __forceinline__ void mbar_arrive(uint32_t mbar_addr) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(mbar_addr) : "memory");
 }
@@ -215,8 +222,7 @@ inline bool encode_tensor_map_2d(CUtensorMap* map, CUtensorMapDataType type, con
     }
     const cuuint32_t estr[2] = {1u, 1u};
     return reinterpret_cast<encode_fn>(fn)(map, type, 2, const_cast<void*>(base), dims, strides, box, estr,
-                                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
