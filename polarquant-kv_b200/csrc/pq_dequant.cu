@@ -1,5 +1,5 @@
 // pq_dequant: stored block_pq4 blocks -> centroid[idx] * float(d) (rotated space) -> inverse rotation v @ R -> float32
-// or float16; and the same with another end, the expanded tiles of the prefill kernel (pq_expand.cuh).
+// or float16.
 //
 // Follows dequantize_with_codebook (src/polarquant_kv_cuda/lloyd_max.py:93-98), the radius restore of
 // quantizer.decompress (python/polarquant_kv/quantizer.py:151) and inverse_rotate (python/polarquant_kv/rotation.py:61);
@@ -10,8 +10,8 @@
 // float32 accumulator), which keeps float32-level accuracy (2e-6 of a vector's largest component).
 //
 // Bound: HBM, 72 bytes in and 256 or 512 out per vector of 128 (4-bit).  A persistent CTA owns 128 vectors at a time:
-//   copy warp     the tile's stored bytes (contiguous), by bulk copy, four tiles in flight (by 4- or 8-byte asynchronous
-//                 copies where a row does not start on a 16-byte boundary);
+//   copy warp     the tile's stored bytes (contiguous), by bulk copy, four tiles in flight (the last one, if partial, by
+//                 4-byte asynchronous copies);
 //   worker warps  (4 per 32-dim block) a thread owns one vector x one block: a stored byte is one lookup of its centroids'
 //                 hi and lo float16 terms (256-byte table rows at a fixed shared address, 16 private copies, so a byte
 //                 becomes an address with one byte-permute and lookups never conflict), times the radius as an error-free
@@ -23,9 +23,9 @@
 //                 took two thirds of the load-store pipe: 136 us against the figure below).
 // A power of two per vector keeps the largest radius in [1, 2) inside, so tiny vectors keep their precision.
 // All waits are bounded (a lost completion sets an error flag instead of hanging).
-#include <cstring>
+#include <atomic>
 
-#include "pq_expand.cuh"
+#include "pq_common.cuh"
 #include "pq_tcgen05.cuh"
 
 namespace pq {
@@ -37,17 +37,12 @@ constexpr float kDqCbScale = 64.0f;          // centroids sit x64 in the table (
 static __device__ unsigned int g_dequant_error = 0;
 
 struct DequantParams {
-    const uint8_t* blocks[2];    // expand: K and V; else the one tensor
+    const uint8_t* blocks;
     const float* rot;
     void* out;
-    int64_t n_vec;               // plain: vectors
-    int64_t n_items;             // tiles of 128 vectors (expand: of both operands)
+    int64_t n_vec;
+    int64_t n_items;             // tiles of 128 vectors
     int out_is_fp16;
-    int aligned;                 // rows start on 16-byte boundaries
-    // expand: tokens per row, row capacity, 128-token tiles per row, items per operand, first operand
-    int64_t S, Scap;
-    int row_tiles, operand_items, operand0;
-    float score_scale;
     float cb[16];
 };
 
@@ -104,21 +99,11 @@ __device__ __forceinline__ float2 dq_mul2(float2 a, float2 b) {
         : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
     return d;
 }
-__device__ __forceinline__ float2 dq_sub2(float2 a, float2 b) {            // a - b
-    float2 d;
-    const float2 m = make_float2(-1.f, -1.f);
-    asm("fma.rn.f32x2 %0, %1, %2, %3;\n"
-        : "=l"(*reinterpret_cast<unsigned long long*>(&d))
-        : "l"(*reinterpret_cast<unsigned long long*>(&b)), "l"(*reinterpret_cast<const unsigned long long*>(&m)),
-          "l"(*reinterpret_cast<unsigned long long*>(&a)));
-    return d;
-}
 __device__ __forceinline__ void dq_sts4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-// EXPAND: the output is the prefill kernel's records instead of vectors.
-template <int D, int BITS, bool EXPAND>
+template <int D, int BITS>
 __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(const DequantParams p, const __grid_constant__ CUtensorMap out_map) {
     using C = DequantCfg<D>;
     constexpr int NBLK = C::NBLK, WORKERS = C::kWorkers, RING = C::kRing;
@@ -201,26 +186,8 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
     const uint32_t tmem_base = *tmem_slot;
     const int n_my = (int)((p.n_items - blockIdx.x + gridDim.x - 1) / gridDim.x);
     bool ok = true;
-    // first stored byte and number of vectors of the i-th tile of this CTA
-    struct Item { int64_t at; int n; int operand, row, tile; };
-    auto item = [&](int i) -> Item {
-        const int64_t it = (int64_t)blockIdx.x + (int64_t)i * gridDim.x;
-        Item r;
-        if (EXPAND) {
-            const int op = it >= p.operand_items ? 1 : 0, k = (int)(it - (int64_t)op * p.operand_items);
-            r.operand = p.operand0 + op;
-            r.row = k / p.row_tiles;
-            r.tile = k - r.row * p.row_tiles;
-            const int64_t tok = (int64_t)r.tile * kDqVecs;
-            r.at = ((int64_t)r.row * p.Scap + tok) * VB;
-            r.n = (int)min((int64_t)kDqVecs, p.S - tok);
-        } else {
-            r.operand = r.row = r.tile = 0;
-            r.at = it * kDqVecs * VB;
-            r.n = (int)min((int64_t)kDqVecs, p.n_vec - it * kDqVecs);
-        }
-        return r;
-    };
+    // first vector of the i-th tile of this CTA
+    auto first = [&](int i) -> int64_t { return ((int64_t)blockIdx.x + (int64_t)i * gridDim.x) * kDqVecs; };
 
     if (warp == WORKERS / 32) {
         // ---- MMA warp: every lane runs the loop, lane 0 issues
@@ -255,10 +222,11 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
         for (int i = 0; i < n_my && ok; ++i) {
             if (round) ok = mbar_wait(sm_addr(in_free + slot), (round - 1u) & 1u, abort_s, 32) && ok;
             if (!ok) break;
-            const Item it = item(i);
-            const uint8_t* src = p.blocks[EXPAND ? it.operand : 0] + it.at;
+            const int64_t v0 = first(i);
+            const int n = (int)min((int64_t)kDqVecs, p.n_vec - v0);
+            const uint8_t* src = p.blocks + v0 * VB;
             const uint32_t dst = ring + slot * C::kSlot, bar = sm_addr(in_full + slot);
-            if (p.aligned && it.n == kDqVecs) {
+            if (n == kDqVecs) {
                 if (lane == 0) {
                     mbar_expect_tx(bar, kDqVecs * VB);
                     bulk_load(dst, src, kDqVecs * VB, bar);
@@ -267,7 +235,7 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
                 }
             } else {
                 // 4-byte asynchronous copies (vectors are multiples of 4 bytes); the barrier counts every lane's
-                for (int c = lane; c < it.n * VB / 4; c += 32)
+                for (int c = lane; c < n * VB / 4; c += 32)
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(dst + 4 * c), "l"(src + 4 * c));
                 asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];\n" ::"r"(bar) : "memory");
             }
@@ -345,99 +313,44 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
             tmem_ld32(v, tmem_lane + 2 * D + b * D + wg * 32);
             tc_fence_before();
             mbar_arrive(sm_addr(acc_free + b));
-            const Item it = item(i);
-            if constexpr (EXPAND) {
-                // K: per 64 dims 64 hi rows then 64 lo rows of 128 bytes; V: the hi rows of all dims, then the lo rows
-                using E = ExpandRec<D>;
-                const int half = row >> 6, r = row & 63, pair = wg >> 1;
-                const bool in = row < it.n;                        // tokens past the end: zeros
-                const float s = in ? kExpScale / (kDqCbScale * 4096.f) : 0.f;
-                const uint32_t piece = C::kOutAddr + (uint32_t)(((half * (D / 64) + pair) * 2) * kExpTok * 128);
-                const uint32_t hi_row = piece + r * 128, lo_row = hi_row + kExpTok * 128;
+            const float s = sc * (1.0f / (kDqCbScale * 4096.f));
+            const float2 s2 = make_float2(s, s);
+            const int64_t v0 = first(i) + 32 * q;
+            // 32 vectors: rows of 128 bytes, 16-byte chunks swizzled as the tensor map says
+            if (p.out_is_fp16) {
+                // 64 dims = rows of 128 bytes, shared by two warps (boxes of 64-byte rows are limited by the number of
+                // rows a TMA unit stores: 98 us for 2^20 vectors)
+                const uint32_t piece = C::kOutAddr + b * (C::kOutBytes / 2) + (uint32_t)((wg >> 1) * kDqVecs + 32 * q) * 128;
                 const bool leader = !(wg & 1) && lane == 0;
-                const uint32_t bar = 1u + (uint32_t)(q * (D / 64) + pair);      // the two warps that share 32 rows of 64 dims
-                if (leader) bulk_wait_read();                      // its last stores have read the buffer
-                asm volatile("bar.sync %0, 64;\n" ::"r"(bar) : "memory");
+                const uint32_t bar = 1u + (uint32_t)(q * (D / 64) + (wg >> 1));
+                // (the pair's barrier of the tile in between orders this wait before the partner's writes too)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) {                      // chunks of 8 dims
-                    uint32_t h[4], l[4];
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t w[4];
 #pragma unroll
                     for (int u = 0; u < 4; ++u) {
-                        float2 x = dq_mul2(v[4 * c + u], make_float2(s, s));
-                        if (!in) x = make_float2(0.f, 0.f);
-                        const __half2 hh = __floats2half2_rn(x.x, x.y);
-                        const float2 f = dq_sub2(x, __half22float2(hh));
-                        h[u] = *reinterpret_cast<const uint32_t*>(&hh);
-                        l[u] = pack_half2(f.x, f.y);
+                        const float2 x = dq_mul2(v[4 * c + u], s2);
+                        w[u] = dq_pack_sat(x.x, x.y);
                     }
-                    const uint32_t at = (uint32_t)((((wg & 1) * 4 + c) ^ (r & 7)) << 4);
-                    dq_sts4(hi_row + at, h[0], h[1], h[2], h[3]);
-                    dq_sts4(lo_row + at, l[0], l[1], l[2], l[3]);
+                    dq_sts4(piece + lane * 128 + ((((wg & 1) * 4 + c) ^ (lane & 7)) << 4), w[0], w[1], w[2], w[3]);
                 }
                 fence_async_smem();
+                if (leader) bulk_wait_read();                  // the store of the other buffer: free for the next tile
                 asm volatile("bar.sync %0, 64;\n" ::"r"(bar) : "memory");
-                const int tile64 = 2 * it.tile + half;
-                if (tile64 * kExpTok < p.S) {                      // (the second half of the last tile may not exist)
-                    const int n64 = (int)((p.S + kExpTok - 1) / kExpTok);
-                    uint8_t* rec = static_cast<uint8_t*>(p.out) + ((size_t)it.row * n64 + tile64) * E::kBytes;
-                    const uint32_t r0 = (uint32_t)(q & 1) * 32 * 128;
-                    if (leader) {
-                        uint8_t* dst = it.operand == 0 ? rec + pair * (2 * kExpTok * 128) : rec + 2 * E::kTerm + pair * (kExpTok * 128);
-                        bulk_store(dst + r0, piece + r0, 32 * 128);
-                        bulk_store(dst + (it.operand == 0 ? (uint32_t)kExpTok * 128 : E::kTerm) + r0, piece + kExpTok * 128 + r0, 32 * 128);
-                    }
-                    if (wg == 0) {
-                        float* f = reinterpret_cast<float*>(rec + E::kFactors);
-                        const float w = in ? sc : 0.f;
-                        if (it.operand == 0) {
-                            f[r] = w * (p.score_scale / kExpScale);
-                        } else {
-                            f[kExpTok + r] = w;
-                            const uint32_t mx = __reduce_max_sync(0xffffffffu, __float_as_uint(w));       // not negative
-                            if (lane == 0) f[2 * kExpTok + (q & 1)] = __uint_as_float(mx);
-                        }
-                    }
-                }
+                if (leader && v0 < p.n_vec) tma_store_2d(&out_map, (wg >> 1) * 64, (int)v0, piece);
             } else {
-                const float s = sc * (1.0f / (kDqCbScale * 4096.f));
-                const float2 s2 = make_float2(s, s);
-                const int64_t v0 = ((int64_t)blockIdx.x + (int64_t)i * gridDim.x) * kDqVecs + 32 * q;
-                // 32 vectors: rows of 128 bytes, 16-byte chunks swizzled as the tensor map says
-                if (p.out_is_fp16) {
-                    // 64 dims = rows of 128 bytes, shared by two warps (boxes of 64-byte rows are limited by the number of
-                    // rows a TMA unit stores: 98 us for 2^20 vectors)
-                    const uint32_t piece = C::kOutAddr + b * (C::kOutBytes / 2) + (uint32_t)((wg >> 1) * kDqVecs + 32 * q) * 128;
-                    const bool leader = !(wg & 1) && lane == 0;
-                    const uint32_t bar = 1u + (uint32_t)(q * (D / 64) + (wg >> 1));
-                    // (the pair's barrier of the tile in between orders this wait before the partner's writes too)
+                const uint32_t piece = C::kOutAddr + (uint32_t)(wg * kDqVecs + 32 * q) * 128;
+                if (lane == 0) bulk_wait_read();
+                __syncwarp();
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        uint32_t w[4];
-#pragma unroll
-                        for (int u = 0; u < 4; ++u) {
-                            const float2 x = dq_mul2(v[4 * c + u], s2);
-                            w[u] = dq_pack_sat(x.x, x.y);
-                        }
-                        dq_sts4(piece + lane * 128 + ((((wg & 1) * 4 + c) ^ (lane & 7)) << 4), w[0], w[1], w[2], w[3]);
-                    }
-                    fence_async_smem();
-                    if (leader) bulk_wait_read();                  // the store of the other buffer: free for the next tile
-                    asm volatile("bar.sync %0, 64;\n" ::"r"(bar) : "memory");
-                    if (leader && v0 < p.n_vec) tma_store_2d(&out_map, (wg >> 1) * 64, (int)v0, piece);
-                } else {
-                    const uint32_t piece = C::kOutAddr + (uint32_t)(wg * kDqVecs + 32 * q) * 128;
-                    if (lane == 0) bulk_wait_read();
-                    __syncwarp();
-#pragma unroll
-                    for (int c = 0; c < 8; ++c) {
-                        const float2 x = dq_mul2(v[2 * c], s2), y = dq_mul2(v[2 * c + 1], s2);
-                        dq_sts4(piece + lane * 128 + ((c ^ (lane & 7)) << 4), __float_as_uint(x.x), __float_as_uint(x.y),
-                                __float_as_uint(y.x), __float_as_uint(y.y));
-                    }
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0 && v0 < p.n_vec) tma_store_2d(&out_map, wg * 32, (int)v0, piece);
+                for (int c = 0; c < 8; ++c) {
+                    const float2 x = dq_mul2(v[2 * c], s2), y = dq_mul2(v[2 * c + 1], s2);
+                    dq_sts4(piece + lane * 128 + ((c ^ (lane & 7)) << 4), __float_as_uint(x.x), __float_as_uint(x.y),
+                            __float_as_uint(y.x), __float_as_uint(y.y));
                 }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0 && v0 < p.n_vec) tma_store_2d(&out_map, wg * 32, (int)v0, piece);
             }
         };
         float before = 0.f;                                        // scale of the tile in the epilogue
@@ -471,10 +384,10 @@ int dequant_error_flags(unsigned int* flags) {
     return PQ_OK;
 }
 
-template <int D, int BITS, bool EXPAND>
+template <int D, int BITS>
 static int launch_dequant(const DequantParams& p, cudaStream_t st) {
     using C = DequantCfg<D>;
-    auto kern = pq_dequant_kernel<D, BITS, EXPAND>;
+    auto kern = pq_dequant_kernel<D, BITS>;
     static std::atomic<uint64_t> allowed{0};
     if (allow_shared(kern, C::smem_bytes(), allowed) != cudaSuccess) return PQ_ERR_CUDA;
     int dev = 0, sms = 0;
@@ -483,52 +396,13 @@ static int launch_dequant(const DequantParams& p, cudaStream_t st) {
         return PQ_ERR_CUDA;
     const int grid = (int)(p.n_items < sms ? p.n_items : sms);      // persistent: one CTA per SM (tensor memory)
     CUtensorMap map;
-    memset(&map, 0, sizeof(map));
-    if (!EXPAND) {
-        const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)p.n_vec}, strides[1] = {(cuuint64_t)D * (p.out_is_fp16 ? 2 : 4)};
-        const cuuint32_t box[2] = {p.out_is_fp16 ? 64u : 32u, 32u};
-        if (!encode_tensor_map_2d(&map, p.out_is_fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.out,
-                                  dims, strides, box))
-            return PQ_ERR_CUDA;
-    }
+    const cuuint64_t dims[2] = {(cuuint64_t)D, (cuuint64_t)p.n_vec}, strides[1] = {(cuuint64_t)D * (p.out_is_fp16 ? 2 : 4)};
+    const cuuint32_t box[2] = {p.out_is_fp16 ? 64u : 32u, 32u};
+    if (!encode_tensor_map_2d(&map, p.out_is_fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, p.out,
+                              dims, strides, box))
+        return PQ_ERR_CUDA;
     kern<<<grid, C::kThreads, C::smem_bytes(), st>>>(p, map);
     return cudaGetLastError() == cudaSuccess ? PQ_OK : PQ_ERR_CUDA;
-}
-
-template <int D>
-static int launch_expand(const DequantParams& p, int bits, cudaStream_t st) {
-    return bits == 4 ? launch_dequant<D, 4, true>(p, st) : launch_dequant<D, 2, true>(p, st);
-}
-
-int expand_launch(const ExpandArgs& a, int head_dim, int k_bits, int v_bits, cudaStream_t st) {
-    DequantParams p{};
-    p.blocks[0] = a.kb;
-    p.blocks[1] = a.vb;
-    p.rot = a.rot;
-    p.out = a.ws;
-    p.S = a.S;
-    p.Scap = a.Scap;
-    p.row_tiles = (int)((a.S + kDqVecs - 1) / kDqVecs);
-    p.operand_items = a.rows * p.row_tiles;
-    p.score_scale = a.score_scale;
-    const int nblk = head_dim / 32;
-    auto row_aligned = [&](const uint8_t* b, int bits) {
-        return ((reinterpret_cast<uintptr_t>(b) | (uintptr_t)(a.Scap * nblk * block_bytes(bits))) & 15) == 0;
-    };
-    const bool ka = row_aligned(a.kb, k_bits), va = row_aligned(a.vb, v_bits);
-    // one launch when the operands share a table
-    bool same = k_bits == v_bits;
-    for (int i = 0; same && i < (1 << k_bits); ++i) same = a.codebook_k[i] == a.codebook_v[i];
-    for (int op = 0; op < (same ? 1 : 2); ++op) {
-        const int bits = op ? v_bits : k_bits;
-        p.operand0 = op;
-        p.n_items = (int64_t)p.operand_items * (same ? 2 : 1);
-        p.aligned = same ? ka && va : op ? va : ka;
-        for (int i = 0; i < 16; ++i) p.cb[i] = i < (1 << bits) ? (op ? a.codebook_v : a.codebook_k)[i] : 0.f;
-        const int s = head_dim == 64 ? launch_expand<64>(p, bits, st) : launch_expand<128>(p, bits, st);
-        if (s != PQ_OK) return s;
-    }
-    return PQ_OK;
 }
 
 }  // namespace pq
@@ -547,15 +421,14 @@ extern "C" int pq_dequant(const void* blocks, int64_t n_vec, int head_dim, int n
         (reinterpret_cast<uintptr_t>(out) & 31))
         return PQ_ERR_MISALIGNED;
     DequantParams p{};
-    p.blocks[0] = static_cast<const uint8_t*>(blocks);
+    p.blocks = static_cast<const uint8_t*>(blocks);
     p.n_items = (n_vec + kDqVecs - 1) / kDqVecs;
-    p.aligned = 1;
     p.rot = rot;
     p.out = out;
     p.n_vec = n_vec;
     p.out_is_fp16 = out_is_fp16;
     for (int i = 0; i < 16; ++i) p.cb[i] = i < (1 << n_bits) ? codebook[i] : 0.f;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (head_dim == 64) return n_bits == 4 ? launch_dequant<64, 4, false>(p, st) : launch_dequant<64, 2, false>(p, st);
-    return n_bits == 4 ? launch_dequant<128, 4, false>(p, st) : launch_dequant<128, 2, false>(p, st);
+    if (head_dim == 64) return n_bits == 4 ? launch_dequant<64, 4>(p, st) : launch_dequant<64, 2>(p, st);
+    return n_bits == 4 ? launch_dequant<128, 4>(p, st) : launch_dequant<128, 2>(p, st);
 }

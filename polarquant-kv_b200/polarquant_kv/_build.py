@@ -22,7 +22,7 @@ HOST_SOURCE = os.path.join(CSRC, "pq_host.cpp")
 
 SOURCES = ["pq_compress.cu", "pq_dequant.cu", "pq_decode_attn.cu", "pq_prefill_attn.cu", "pq_lse_merge.cu", "pq_qjl.cu",
            "pq_llama_abi.cu", "pq_bridge_attn.cu", "pq_bridge_compress.cu"]
-HEADERS = ["pq_common.cuh", "pq_tcgen05.cuh", "pq_bridge.cuh", "pq_expand.cuh", os.path.join(INCLUDE, "polarquant_b200.h"),
+HEADERS = ["pq_common.cuh", "pq_tcgen05.cuh", "pq_bridge.cuh", os.path.join(INCLUDE, "polarquant_b200.h"),
            os.path.join(INCLUDE, "polarquant_llama_abi.h")]
 
 
