@@ -8,6 +8,7 @@
 // its complete checks; so every error is raised in one place only.
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
@@ -92,7 +93,7 @@ bool matrix_id(PyObject* o, MatrixId* id) {
     if (o == Py_None) return true;
     id->object = o;
     if (const at::Tensor* t = tensor(o)) {
-        if (t->layout() != at::kStrided) return false;
+        if (t->layout() != at::kStrided || t->is_inference()) return false;      // (no version counter)
         id->data = t->data_ptr();
         id->size = t->numel();
         id->a = t->_version();
@@ -205,6 +206,17 @@ PyObject* raise_status(int status, const char* where) {
     return nullptr;
 }
 
+// A launch waits when the stream's queue is full, so other Python threads go on meanwhile.  What the call uses is held by
+// local references or by the caller's arguments.
+template <class F>
+int launch(F f) {
+    struct Released {
+        PyThreadState* state = PyEval_SaveThread();
+        ~Released() { PyEval_RestoreThread(state); }         // also when an exception passes
+    } released;
+    return f();
+}
+
 void* stream_of(int device) { return (void*)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
 
 bool half_contiguous(const at::Tensor& t) {
@@ -266,10 +278,12 @@ int launch_compress(const at::Tensor& x, int64_t rows, int64_t tokens, int64_t c
     const void* js = sketch ? plan.jl_split : nullptr;
     const int m = sketch ? plan.jl_dim : 0;
     void *sp = sketch ? signs.data_ptr() : nullptr, *np = sketch ? norms.data_ptr() : nullptr, *st = stream_of(plan.device);
-    return pos.dev ? pq_compress_rows_dynamic(x.data_ptr(), rows, tokens, cap, pos.dev, plan.head_dim, n_bits, plan.rot_split,
-                                              t.thresholds, t.codebook, blocks.data_ptr(), js, m, sp, np, st)
-                   : pq_compress_rows(x.data_ptr(), rows, tokens, cap, pos.host, plan.head_dim, n_bits, plan.rot_split,
-                                      t.thresholds, t.codebook, blocks.data_ptr(), js, m, sp, np, st);
+    return launch([&] {
+        return pos.dev ? pq_compress_rows_dynamic(x.data_ptr(), rows, tokens, cap, pos.dev, plan.head_dim, n_bits, plan.rot_split,
+                                                  t.thresholds, t.codebook, blocks.data_ptr(), js, m, sp, np, st)
+                       : pq_compress_rows(x.data_ptr(), rows, tokens, cap, pos.host, plan.head_dim, n_bits, plan.rot_split,
+                                          t.thresholds, t.codebook, blocks.data_ptr(), js, m, sp, np, st);
+    });
 }
 
 const Plan* plan_for(PyObject* R, PyObject* P, int device) {
@@ -375,8 +389,11 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (!plan || plan->head_dim != c.dim || dev != c10::cuda::current_device()) Py_RETURN_NONE;
     const bool half = args[2] == Py_True;
     at::Tensor out = empty({c.rows_b, c.rows_h, c.seq, c.dim}, half ? at::kHalf : at::kFloat, dev);
-    const int st = pq_dequant(c.blocks.data_ptr(), c.rows_b * c.rows_h * c.seq, (int)c.dim, (int)c.n_bits,
-                              g_tables[c.n_bits].codebook, plan->rot, out.data_ptr(), half, stream_of(dev));
+    void* stream = stream_of(dev);
+    const int st = launch([&] {
+        return pq_dequant(c.blocks.data_ptr(), c.rows_b * c.rows_h * c.seq, (int)c.dim, (int)c.n_bits,
+                          g_tables[c.n_bits].codebook, plan->rot, out.data_ptr(), half, stream);
+    });
     if (st) return raise_status(st, "pq_dequant");
     return THPVariable_Wrap(out);
 }
@@ -396,11 +413,12 @@ struct Scratch {
 std::deque<Scratch> g_scratch;               // bounded: the least recently made entry goes
 constexpr size_t kScratchLimit = 32;
 
-void* decode_scratch(int device, void* stream, size_t* bytes_io, size_t counters) {
+// Undefined on a CUDA error.
+at::Tensor decode_scratch(int device, void* stream, size_t* bytes_io, size_t counters) {
     const size_t kept = pq_decode_attn_counter_bytes(), need = *bytes_io += kept;
     cudaStreamCaptureStatus status;
     unsigned long long id = 0;
-    if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) return nullptr;
+    if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) return {};
     if (status != cudaStreamCaptureStatusActive) id = 0;
     Scratch* s = nullptr;
     for (Scratch& e : g_scratch)
@@ -418,10 +436,10 @@ void* decode_scratch(int device, void* stream, size_t* bytes_io, size_t counters
     const size_t clear = id ? counters : kept;              // a graph replays its clear: no more of it than needed
     if (counters > kept || s->cleared < clear) {
         const size_t bytes = counters > clear ? counters : clear;
-        if (cudaMemsetAsync(s->buf.data_ptr(), 0, bytes, (cudaStream_t)stream) != cudaSuccess) return nullptr;
+        if (cudaMemsetAsync(s->buf.data_ptr(), 0, bytes, (cudaStream_t)stream) != cudaSuccess) return {};
         if (counters <= kept) s->cleared = bytes;
     }
-    return s->buf.data_ptr();
+    return s->buf;
 }
 
 // ------------------------------------------------------------------ attention
@@ -477,21 +495,23 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     void* st = stream_of(a.device);
     size_t need = pq_decode_attn_scratch_bytes((int)a.B, (int)a.Hq, (int)a.Hkv, S, (int)a.D, 0);
-    void* scratch = decode_scratch(a.device, st, &need, ((size_t)a.B * a.Hq * 4 + 255) / 256 * 256);
-    if (!scratch) return raise_status(PQ_ERR_CUDA, "pq_decode_attn");
+    const at::Tensor kept = decode_scratch(a.device, st, &need, ((size_t)a.B * a.Hq * 4 + 255) / 256 * 256);
+    if (!kept.defined()) return raise_status(PQ_ERR_CUDA, "pq_decode_attn");
+    void* scratch = kept.data_ptr();
     at::Tensor out = empty(a.q->sizes(), half ? at::kHalf : at::kFloat, a.device);
     const float *cbk = g_tables[a.ck.n_bits].codebook, *cbv = g_tables[a.cv.n_bits].codebook;
     const float* jl = qjl ? a.plan->jl : nullptr;
     const void *bits = qjl ? a.ck.signs.data_ptr() : nullptr, *norms = qjl ? a.ck.norms.data_ptr() : nullptr;
     const int m = qjl ? a.plan->jl_dim : 0;
-    const int status =
-        len.dev ? pq_decode_attn_dynamic(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
+    const int status = launch([&] {
+        return len.dev ? pq_decode_attn_dynamic(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
                                          (int)a.Hkv, S, len.dev, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits, cbk,
                                          cbv, a.plan->rot, a.scale, jl, m, bits, norms, out.data_ptr(), half, nullptr, 0,
                                          scratch, need, st)
-                : pq_decode_attn(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
+                       : pq_decode_attn(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
                                  (int)a.Hkv, S, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits, cbk, cbv, a.plan->rot,
                                  a.scale, jl, m, bits, norms, out.data_ptr(), half, nullptr, 0, scratch, need, st);
+    });
     if (status) return raise_status(status, "pq_decode_attn");
     return THPVariable_Wrap(out);
 }
@@ -506,11 +526,14 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     at::Tensor out = empty(a.q->sizes(), half ? at::kHalf : at::kFloat, a.device), ws;
     const size_t need = pq_prefill_attn_workspace_bytes((int)a.B, (int)a.Hkv, a.ck.seq, (int)a.D);
     if (a.Sq * (a.Hq / a.Hkv) > 128 && need > 0 && need <= (size_t)limit) ws = empty({(int64_t)need}, at::kByte, a.device);
-    const int status = pq_prefill_attn(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
+    void* stream = stream_of(a.device);
+    const int status = launch([&] {
+        return pq_prefill_attn(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
                                        (int)a.Hkv, (int)a.Sq, a.ck.seq, a.ck.cap, (int)a.D, (int)a.ck.n_bits,
                                        (int)a.cv.n_bits, g_tables[a.ck.n_bits].codebook, g_tables[a.cv.n_bits].codebook,
                                        a.plan->rot, a.scale, args[6] == Py_True, out.data_ptr(), half,
-                                       ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? need : 0, stream_of(a.device));
+                                       ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? need : 0, stream);
+    });
     if (status) return raise_status(status, "pq_prefill_attn");
     return THPVariable_Wrap(out);
 }
@@ -559,13 +582,15 @@ PyObject* run_prepared(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     const Prepared* p = (const Prepared*)PyCapsule_GetPointer(args[0], kPreparedCapsule);
     if (!p) return nullptr;
-    const int st = p->len ? pq_decode_attn_dynamic(p->q, p->kb, p->vb, p->B, p->Hq, p->Hkv, p->cap, p->len, p->cap, p->D, p->kbits,
+    const int st = launch([&] {
+        return p->len ? pq_decode_attn_dynamic(p->q, p->kb, p->vb, p->B, p->Hq, p->Hkv, p->cap, p->len, p->cap, p->D, p->kbits,
                                                    p->vbits, p->cbk, p->cbv, p->rot, p->scale, p->jl, p->jl_dim, p->bits, p->norms,
                                                    p->out, p->half, p->partial, p->splits, p->scratch, p->scratch_bytes,
                                                    (void*)stream)
                           : pq_decode_attn(p->q, p->kb, p->vb, p->B, p->Hq, p->Hkv, S, p->cap, p->D, p->kbits, p->vbits, p->cbk,
                                            p->cbv, p->rot, p->scale, p->jl, p->jl_dim, p->bits, p->norms, p->out, p->half,
                                            p->partial, p->splits, p->scratch, p->scratch_bytes, (void*)stream);
+    });
     return PyLong_FromLong(st);
 }
 
@@ -583,8 +608,12 @@ PyObject* bridge_compress(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_RETURN_NONE;
     const int dev = x->get_device();
     at::Tensor radius = empty({N}, at::kFloat, dev), packed = empty({N, D / 2}, at::kByte, dev);
-    polarquant_compress_cuda_c((const float*)x->data_ptr(), (const float*)R->data_ptr(), (const float*)cb->data_ptr(),
-                               (float*)radius.data_ptr(), (uint8_t*)packed.data_ptr(), (int)N, (int)D, (int)cb->numel(), stream_of(dev));
+    void* stream = stream_of(dev);
+    launch([&] {
+        polarquant_compress_cuda_c((const float*)x->data_ptr(), (const float*)R->data_ptr(), (const float*)cb->data_ptr(),
+                                   (float*)radius.data_ptr(), (uint8_t*)packed.data_ptr(), (int)N, (int)D, (int)cb->numel(), stream);
+        return 0;
+    });
     PyObject *a = THPVariable_Wrap(radius), *b = THPVariable_Wrap(packed);
     PyObject* r = a && b ? PyTuple_Pack(2, a, b) : nullptr;
     Py_XDECREF(a);
@@ -598,7 +627,11 @@ PyObject* bridge_rotate(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int dev = x->get_device();
     at::Tensor out = empty(x->sizes(), at::kFloat, dev);
     const auto fn = args[2] == Py_True ? polarquant_inverse_rotate_cuda_c : polarquant_rotate_query_cuda_c;
-    fn((const float*)x->data_ptr(), (const float*)R->data_ptr(), (float*)out.data_ptr(), (int)x->size(0), (int)x->size(1), stream_of(dev));
+    void* stream = stream_of(dev);
+    launch([&] {
+        fn((const float*)x->data_ptr(), (const float*)R->data_ptr(), (float*)out.data_ptr(), (int)x->size(0), (int)x->size(1), stream);
+        return 0;
+    });
     return THPVariable_Wrap(out);
 }
 // bridge_attention(q, packed_k, k_radius, packed_v, v_radius, codebook, scale) -> tensor or None
@@ -617,17 +650,29 @@ PyObject* bridge_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
     const int dev = q->get_device();
     at::Tensor out = empty(q->sizes(), at::kFloat, dev);
-    polarquant_fused_attention_cuda_c((const float*)q->data_ptr(), (const uint8_t*)pk->data_ptr(), (const float*)kr->data_ptr(),
-                                      (const uint8_t*)pv->data_ptr(), (const float*)vr->data_ptr(), (const float*)cb->data_ptr(),
-                                      (float*)out.data_ptr(), (int)hq, (int)hkv, (int)S, (int)D, (int)cb->numel(), (float)scale,
-                                      stream_of(dev));
+    void* stream = stream_of(dev);
+    launch([&] {
+        polarquant_fused_attention_cuda_c((const float*)q->data_ptr(), (const uint8_t*)pk->data_ptr(), (const float*)kr->data_ptr(),
+                                          (const uint8_t*)pv->data_ptr(), (const float*)vr->data_ptr(), (const float*)cb->data_ptr(),
+                                          (float*)out.data_ptr(), (int)hq, (int)hkv, (int)S, (int)D, (int)cb->numel(), (float)scale,
+                                          stream);
+        return 0;
+    });
     return THPVariable_Wrap(out);
 }
 // bridge_error() -> code of the calling thread's last failed bridge call, cleared
 PyObject* bridge_error(PyObject*, PyObject*) { return PyLong_FromLong(polarquant_last_error_c()); }
 
 // ------------------------------------------------------------------ module
-#define PQ_FAST(name, doc) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, doc}
+using Fast = PyObject*(PyObject*, PyObject* const*, Py_ssize_t);
+// C++ exceptions (no memory, a tensor without storage) become the Python errors that torch makes of them.
+template <Fast* F>
+PyObject* guarded(PyObject* self, PyObject* const* args, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    return F(self, args, n);
+    END_HANDLE_TH_ERRORS
+}
+#define PQ_FAST(name, doc) {#name, (PyCFunction)(void (*)(void))guarded<name>, METH_FASTCALL, doc}
 PyMethodDef methods[] = {
     {"register", (PyCFunction)(void (*)(void))register_types, METH_FASTCALL, "register(CompressedKV, DevicePlan, check)"},
     PQ_FAST(plan_get, "cached plan of the matrix objects"),

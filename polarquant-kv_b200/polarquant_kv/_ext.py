@@ -106,6 +106,7 @@ def host():
     global _host
     if _host is None:
         lib()                                        # its own, clearer error comes first
+        import torch  # noqa: F401                   # before the module: its C++ types have to be torch's own
         try:
             from . import _host as module
         except ImportError as exc:

@@ -85,12 +85,24 @@ class DevicePlan:
             self.jl_dim = P.shape[0]
             self.jl = torch.from_numpy(P.astype(np.float32)).contiguous().to(self.device)
             self.jl_split = torch.from_numpy(split_fp16(P @ R.T, JL_SCALE)).contiguous().to(self.device)
+        self._attach()
+
+    def _attach(self):
+        """The native handle (raw addresses of this object's tensors)."""
         self._native = None
         if self.device.type == "cuda":
             self.device = self.rot.device                    # with its index
             ptr = lambda t: t.data_ptr() if t is not None else 0                # noqa: E731
             self._native = _ext.host().plan_handle(self.head_dim, self.device.index, ptr(self.rot), ptr(self.rot_split),
                                                    ptr(self.jl), ptr(self.jl_split), self.jl_dim)
+
+    # a copied or unpickled plan has tensors, and so a handle, of its own
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "_native"}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self._attach()
 
 
 _PLANS: dict = {}

@@ -408,3 +408,24 @@ def test_decode_split_mode_partition_arithmetic():
     for batch, hq, hkv, s in ((1, 64, 8, 131072), (32, 32, 8, 8192), (1, 8, 8, 16), (4, 14, 2, 5000)):
         d = lib.pq_decode_attn_default_splits(batch, hq, hkv, s, 128)
         assert 1 <= d <= max(1, min(64, -(-s // 16) // 32))
+
+
+def test_host_module_loads_before_torch():
+    import subprocess
+    import sys
+    pkg = os.path.join(ROOT, "polarquant-kv_b200")
+    code = f"import sys; sys.path.insert(0, {pkg!r}); from polarquant_kv import _ext; assert 'torch' not in sys.modules; _ext.host()"
+    assert subprocess.run([sys.executable, "-c", code], timeout=300).returncode == 0
+
+
+def test_host_module_turns_cpp_exceptions_into_python_errors():
+    """A tensor without storage (inside vmap) raises instead of ending the process; an inference tensor, which has no
+    version counter, is not recognised by identity."""
+    import torch
+
+    from polarquant_kv import _ext
+    host = _ext.host()
+    with pytest.raises(RuntimeError):
+        torch.vmap(lambda m: host.plan_get(m, 0, None) or m)(torch.zeros(2, 4, 4))
+    with torch.inference_mode():
+        assert host.plan_get(torch.zeros(4, 4), 0, None) is None
