@@ -64,6 +64,11 @@ struct PrefillParams {
     float scale_log2;
     float cbk[16], cbv[16];
     const uint8_t* ws;     // expanded tiles (see PrefillCfg::kRec) or null
+    // Split over the tokens (blockIdx.z): tiles per split, and the records [split][output row][m, l, o in rotated space]
+    // that pq_lse_merge combines.  Null: one split, results straight to `out`.
+    float* parts;
+    int split_tiles;
+    int64_t out_rows;
 };
 
 // Barriers that two roles wait on come in pairs, one per tile parity: a barrier's next phase can then
@@ -454,11 +459,16 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
         if (kv_end > p.S) kv_end = p.S;
         if (kv_end < 0) kv_end = 0;
     }
-    const int n_tiles = (int)((kv_end + kPfTok - 1) / kPfTok);
-    const uint8_t* k_row = p.kb + (size_t)kvrow * p.Scap * TBK;
-    const uint8_t* v_row = p.vb + (size_t)kvrow * p.Scap * TBV;
+    // ... of which this split takes up to split_tiles tiles; token numbers below count from its first one
+    const int64_t first = p.parts ? (int64_t)blockIdx.z * p.split_tiles * kPfTok : 0;
+    int n_tiles = kv_end > first ? (int)((kv_end - first + kPfTok - 1) / kPfTok) : 0;
+    if (p.parts) n_tiles = min(n_tiles, p.split_tiles);
+    const int64_t S = p.S - first;
+    const uint8_t* k_row = p.kb + ((size_t)kvrow * p.Scap + first) * TBK;
+    const uint8_t* v_row = p.vb + ((size_t)kvrow * p.Scap + first) * TBV;
     bool ok = true;
     float inv_l = 0.f;                                                    // row owners: 1 / (1024 * row sum)
+    float row_m = 0.f, row_l = 0.f;                                       // ... maximum in use and sum
 
     if (warp < kPfSoftWarps) {
         // =================================================== softmax: NSPLIT threads per query row
@@ -466,8 +476,8 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
         const int r = q * 32 + lane;
         const uint32_t tlane = tmem_base + ((uint32_t)(q * 32) << 16);
         const int row = row0 + r;
-        int limit = p.causal ? (int)(p.S - p.Sq + (row % p.Sq) + 1) : (int)p.S;        // tokens [0, limit)
-        if (limit > p.S) limit = (int)p.S;
+        int limit = p.causal ? (int)(S - p.Sq + (row % p.Sq) + 1) : (int)S;            // tokens [0, limit)
+        if (limit > S) limit = (int)S;
         if (row >= n_rows || limit < 0) limit = 0;
         float m_run = -INFINITY, m_used = -INFINITY, l_run = 0.f;
         const uint32_t prow = (uint32_t)((r >> 3) * 1024 + (r & 7) * 128);
@@ -617,6 +627,8 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
 #pragma unroll
         for (int k = 0; k < NSPLIT; ++k) l_run += xchg[k * kPfRows + r];
         inv_l = l_run > 0.f ? (1.0f / kPfValScale) / l_run : 0.f;
+        row_m = m_used;
+        row_l = l_run;
     } else if (PRE && warp < kMmaWarp) {
         // =================================================== copy warp: expanded tiles from the workspace
         if (warp == kPfSoftWarps) {
@@ -661,8 +673,8 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
         RawItems<D, KBITS> rk;
         RawItems<D, VBITS> rv;
         if (n_tiles > 0) {
-            rk.load(k_row, (int)min((int64_t)kPfTok, p.S), it_tok, it_blk, it_qw);
-            rv.load(v_row, (int)min((int64_t)kPfTok, p.S), it_tok, it_blk, it_qw);
+            rk.load(k_row, (int)min((int64_t)kPfTok, S), it_tok, it_blk, it_qw);
+            rv.load(v_row, (int)min((int64_t)kPfTok, S), it_tok, it_blk, it_qw);
         }
         for (int i = 0; i < n_tiles && ok; ++i) {
             const int bb = i & 1;
@@ -674,7 +686,7 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
             typename RawItems<D, VBITS>::Pending pv;
             const bool more = i + 1 < n_tiles;
             const int64_t tok1 = more ? (int64_t)(i + 1) * kPfTok : 0;            // (the last tile re-reads tile 0)
-            const int ntok1 = (int)min((int64_t)kPfTok, p.S - tok1);
+            const int ntok1 = (int)min((int64_t)kPfTok, S - tok1);
             RawItems<D, KBITS>::issue(pk, k_row + tok1 * TBK, ntok1, it_tok, it_blk, it_qw);
             RawItems<D, VBITS>::issue(pv, v_row + tok1 * TBV, ntok1, it_tok, it_blk, it_qw);
             // K buffer bb: free once S(i-2) is complete; its dmaxK slot once the softmax of tile i-2 has read it
@@ -779,6 +791,39 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
     tc_fence_before();
     __syncthreads();          // every tile buffer is dead
     tc_fence_after();
+
+    if (!PRE && p.parts) {
+        // ---- a split's record: the merge normalises and rotates back
+        if (warp < kPfRowWarps) {
+            const uint32_t tlane = tmem_base + ((uint32_t)(warp * 32) << 16);
+            const int row = row0 + tid;
+            const int head = hkv * p.G + (row < n_rows ? row / p.Sq : 0), sq = row < n_rows ? row % p.Sq : 0;
+            float* rec = p.parts + ((size_t)blockIdx.z * p.out_rows + ((size_t)b * p.Hq + head) * p.Sq + sq) * (D + 2);
+            const bool bad = row_l != row_l;                              // the merge leaves out parts without a positive sum:
+            if (row < n_rows) *reinterpret_cast<float2*>(rec) = bad ? make_float2(0.f, 1.f) : make_float2(row_m, row_l);   // a NaN stays one
+#pragma unroll 1
+            for (int c = 0; c < D / 32; ++c) {
+                float o[32];
+                if (n_tiles > 0) {
+                    tmem_ld32(o, tlane + C::kOCol + c * 32);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < 32; ++k) o[k] = 0.f;
+                }
+                if (row < n_rows) {
+#pragma unroll
+                    for (int k = 0; k < 32; k += 2)
+                        *reinterpret_cast<float2*>(rec + 2 + c * 32 + k) =
+                            bad ? make_float2(row_l, row_l)
+                                : make_float2(o[k] * (1.0f / kPfValScale), o[k + 1] * (1.0f / kPfValScale));
+                }
+            }
+        }
+        tc_fence_before();
+        __syncthreads();
+        if (warp == 0) tmem_dealloc(tmem_base, C::kTmemCols);
+        return;
+    }
 
     // ---- normalise and rotate back on the tensor core: out = o_rot @ R as o_hi*Rt_hi + o_hi*Rt_lo +
     // o_lo*Rt_hi with Rt = 4096 * R^T.  A = o as two float16 terms in the query buffers, B = [Rt_hi ; Rt_lo]
@@ -900,20 +945,20 @@ template <int D, int KBITS, int VBITS>
 static int launch_prefill(const PrefillParams& p, int rows, uint8_t* ws, cudaStream_t st) {
     const size_t smem = PrefillCfg<D>::smem_bytes();
     const int n_rows = p.G * p.Sq;
-    dim3 grid((n_rows + kPfRows - 1) / kPfRows, rows, 1);
+    const int tiles = (int)((p.S + kPfTok - 1) / kPfTok);
+    dim3 grid((n_rows + kPfRows - 1) / kPfRows, rows, p.parts ? (tiles + p.split_tiles - 1) / p.split_tiles : 1);
     if (ws) {
         // expand every tile once, then run the attention kernel on the expanded tiles
-        const int n_tiles = (int)((p.S + kPfTok - 1) / kPfTok);
-        pq_prefill_expand_kernel<D, KBITS, VBITS><<<dim3(n_tiles, rows, 1), kPfDeqThreads, 0, st>>>(p, ws, n_tiles);
+        pq_prefill_expand_kernel<D, KBITS, VBITS><<<dim3(tiles, rows, 1), kPfDeqThreads, 0, st>>>(p, ws, tiles);
         if (cudaGetLastError() != cudaSuccess) return PQ_ERR_CUDA;
         auto kern = pq_prefill_attn_kernel<D, 4, 4, true>;
         static std::atomic<uint64_t> allowed{0};
-    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
+        if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
         kern<<<grid, pf_threads(true), smem, st>>>(p);
     } else {
         auto kern = pq_prefill_attn_kernel<D, KBITS, VBITS, false>;
         static std::atomic<uint64_t> allowed{0};
-    if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
+        if (allow_shared(kern, smem, allowed) != cudaSuccess) return PQ_ERR_CUDA;
         kern<<<grid, pf_threads(false), smem, st>>>(p);
     }
     return cudaGetLastError() == cudaSuccess ? PQ_OK : PQ_ERR_CUDA;
@@ -936,12 +981,36 @@ extern "C" size_t pq_prefill_attn_workspace_bytes(int batch, int kv_heads, int64
     return (size_t)batch * kv_heads * (size_t)((seq_len + pq::kPfTok - 1) / pq::kPfTok) * rec;
 }
 
-extern "C" int pq_prefill_attn(const void* q, const void* k_blocks, const void* v_blocks,
-                               int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len,
-                               int64_t seq_capacity, int head_dim, int k_bits, int v_bits,
-                               const float* codebook_k, const float* codebook_v, const float* rot,
-                               float scale, int causal, void* out, int out_is_fp16, void* workspace,
-                               size_t workspace_bytes, void* stream) {
+// How many CTAs share a query tile's tokens.  A CTA has an SM to itself and walks its tiles one after the other (about
+// 2.8 us each), so a grid of fewer CTAs than SMs leaves the rest idle.  The cost of s splits, in tiles: waves of CTAs x
+// (set-up and epilogue, about 5, + tiles per split), and 3 for the merge kernel's launch and round trips.  One query tile per
+// KV head only: with more of them the expanded workspace is the faster way.  8 sequences x 8 KV heads, 5 positions x 4 heads
+// against 3001 tokens: one CTA per KV row 147 us, two 88 us.
+static int prefill_splits(int rows, int64_t n_rows, int64_t seq_len) {
+    const int64_t tiles = (seq_len + pq::kPfTok - 1) / pq::kPfTok;
+    if (n_rows > pq::kPfRows || rows <= 0 || tiles < 2) return 1;
+    int64_t best = 1, best_cost = 0;
+    for (int64_t s = 1; s <= 64 && s <= tiles; ++s) {
+        const int64_t cost = (rows * s + 147) / 148 * (5 + (tiles + s - 1) / s) + (s > 1 ? 3 : 0);
+        if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
+    }
+    return (int)best;
+}
+
+extern "C" size_t pq_prefill_attn_partial_bytes(int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len, int head_dim) {
+    if (batch <= 0 || kv_heads <= 0 || q_heads <= 0 || seq_q <= 0 || seq_len <= 0 || q_heads % kv_heads ||
+        (head_dim != 64 && head_dim != 128))
+        return 0;
+    const int s = prefill_splits(batch * kv_heads, (int64_t)(q_heads / kv_heads) * seq_q, seq_len);
+    return s > 1 ? (size_t)s * batch * q_heads * seq_q * (head_dim + 2) * sizeof(float) : 0;
+}
+
+static int prefill_call(const void* q, const void* k_blocks, const void* v_blocks,
+                        int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len,
+                        int64_t seq_capacity, int head_dim, int k_bits, int v_bits,
+                        const float* codebook_k, const float* codebook_v, const float* rot,
+                        float scale, int causal, void* out, int out_is_fp16, void* workspace,
+                        size_t workspace_bytes, void* partials, size_t partial_bytes, void* stream) {
     using namespace pq;
     if (batch < 0 || q_heads <= 0 || kv_heads <= 0 || q_heads % kv_heads || seq_q < 0 || seq_len < 0 ||
         seq_capacity < seq_len)
@@ -983,15 +1052,52 @@ extern "C" int pq_prefill_attn(const void* q, const void* k_blocks, const void* 
     p.out_is_fp16 = out_is_fp16;
     p.scale_log2 = scale * 1.4426950408889634f;
     p.ws = static_cast<const uint8_t*>(workspace);
+    int splits = 1;
+    if (partials) {
+        if (reinterpret_cast<uintptr_t>(partials) & 15) return PQ_ERR_MISALIGNED;
+        if (partial_bytes < pq_prefill_attn_partial_bytes(batch, q_heads, kv_heads, seq_q, seq_len, head_dim))
+            return PQ_ERR_SCRATCH_TOO_SMALL;
+        splits = prefill_splits(rows, (int64_t)p.G * seq_q, seq_len);
+        if (splits > 1) {
+            const int64_t tiles = (seq_len + kPfTok - 1) / kPfTok;
+            p.split_tiles = (int)((tiles + splits - 1) / splits);
+            splits = (int)((tiles + p.split_tiles - 1) / p.split_tiles);
+            p.parts = static_cast<float*>(partials);
+            p.out_rows = (int64_t)batch * q_heads * seq_q;
+        }
+    }
     for (int i = 0; i < 16; ++i) {
         p.cbk[i] = i < (1 << k_bits) ? codebook_k[i] : 0.f;
         p.cbv[i] = i < (1 << v_bits) ? codebook_v[i] : 0.f;
     }
+    int status = PQ_ERR_BAD_HEAD_DIM;
 #define PQ_PF(DD, KB, VB) \
     if (head_dim == DD && k_bits == KB && v_bits == VB) \
-        return launch_prefill<DD, KB, VB>(p, rows, static_cast<uint8_t*>(workspace), st);
+        status = launch_prefill<DD, KB, VB>(p, rows, static_cast<uint8_t*>(workspace), st);
     PQ_PF(64, 4, 4) PQ_PF(64, 4, 2) PQ_PF(64, 2, 4) PQ_PF(64, 2, 2)
     PQ_PF(128, 4, 4) PQ_PF(128, 4, 2) PQ_PF(128, 2, 4) PQ_PF(128, 2, 2)
 #undef PQ_PF
-    return PQ_ERR_BAD_HEAD_DIM;
+    if (status != PQ_OK || !p.parts) return status;
+    return pq_lse_merge(p.parts, splits, p.out_rows, head_dim, rot, out, out_is_fp16, stream);
+}
+
+extern "C" int pq_prefill_attn(const void* q, const void* k_blocks, const void* v_blocks,
+                               int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len,
+                               int64_t seq_capacity, int head_dim, int k_bits, int v_bits,
+                               const float* codebook_k, const float* codebook_v, const float* rot,
+                               float scale, int causal, void* out, int out_is_fp16, void* workspace,
+                               size_t workspace_bytes, void* stream) {
+    return prefill_call(q, k_blocks, v_blocks, batch, q_heads, kv_heads, seq_q, seq_len, seq_capacity, head_dim, k_bits, v_bits,
+                        codebook_k, codebook_v, rot, scale, causal, out, out_is_fp16, workspace, workspace_bytes, nullptr, 0,
+                        stream);
+}
+
+extern "C" int pq_prefill_attn_split(const void* q, const void* k_blocks, const void* v_blocks,
+                                     int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len,
+                                     int64_t seq_capacity, int head_dim, int k_bits, int v_bits,
+                                     const float* codebook_k, const float* codebook_v, const float* rot,
+                                     float scale, int causal, void* out, int out_is_fp16, void* partials,
+                                     size_t partial_bytes, void* stream) {
+    return prefill_call(q, k_blocks, v_blocks, batch, q_heads, kv_heads, seq_q, seq_len, seq_capacity, head_dim, k_bits, v_bits,
+                        codebook_k, codebook_v, rot, scale, causal, out, out_is_fp16, nullptr, 0, partials, partial_bytes, stream);
 }
