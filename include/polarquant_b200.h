@@ -340,15 +340,15 @@ int pq_prefill_attn(const void* q, const void* k_blocks, const void* v_blocks,
                     float scale, int causal, void* out, int out_is_fp16,
                     void* workspace, size_t workspace_bytes, void* stream);
 
-/* pq_prefill_attn_split — pq_prefill_attn without a workspace, for few query rows per KV head (seq_q *
- * q_heads/kv_heads <= 128): when batch * kv_heads leaves SMs idle the tokens are split over several CTAs and
- * merged by a second kernel.  partials: 16-byte aligned device buffer of at least
+/* pq_prefill_attn_split — pq_prefill_attn for grids that leave SMs idle (few KV rows and query tiles): the tokens
+ * are split over several CTAs and merged by a second kernel.  partials: 16-byte aligned device buffer of at least
  * pq_prefill_attn_partial_bytes(...) bytes; where that is 0, or partials is NULL, nothing is split. */
 int pq_prefill_attn_split(const void* q, const void* k_blocks, const void* v_blocks,
                           int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len,
                           int64_t seq_capacity, int head_dim, int k_bits, int v_bits,
                           const float* codebook_k, const float* codebook_v, const float* rot,
                           float scale, int causal, void* out, int out_is_fp16,
+                          void* workspace, size_t workspace_bytes,
                           void* partials, size_t partial_bytes, void* stream);
 size_t pq_prefill_attn_partial_bytes(int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len, int head_dim);
 

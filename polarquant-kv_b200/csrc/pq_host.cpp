@@ -526,16 +526,15 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     at::Tensor out = empty(a.q->sizes(), half ? at::kHalf : at::kFloat, a.device), ws;
     const size_t need = pq_prefill_attn_workspace_bytes((int)a.B, (int)a.Hkv, a.ck.seq, (int)a.D);
     if (a.Sq * (a.Hq / a.Hkv) > 128 && need > 0 && need <= (size_t)limit) ws = empty({(int64_t)need}, at::kByte, a.device);
-    const size_t parts_need = ws.defined() ? 0 : pq_prefill_attn_partial_bytes((int)a.B, (int)a.Hq, (int)a.Hkv, (int)a.Sq, a.ck.seq, (int)a.D);
+    const size_t parts_need = pq_prefill_attn_partial_bytes((int)a.B, (int)a.Hq, (int)a.Hkv, (int)a.Sq, a.ck.seq, (int)a.D);
     at::Tensor parts;
     if (parts_need) parts = empty({(int64_t)parts_need}, at::kByte, a.device);
     void *stream = stream_of(a.device), *wsp = ws.defined() ? ws.data_ptr() : nullptr, *pp = parts_need ? parts.data_ptr() : nullptr;
-    const auto fn = parts_need ? pq_prefill_attn_split : pq_prefill_attn;
     const int status = launch([&] {
-        return fn(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq, (int)a.Hkv, (int)a.Sq,
-                  a.ck.seq, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits, g_tables[a.ck.n_bits].codebook,
-                  g_tables[a.cv.n_bits].codebook, a.plan->rot, a.scale, args[6] == Py_True, out.data_ptr(), half,
-                  parts_need ? pp : wsp, parts_need ? parts_need : wsp ? need : 0, stream);
+        return pq_prefill_attn_split(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
+                                     (int)a.Hkv, (int)a.Sq, a.ck.seq, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits,
+                                     g_tables[a.ck.n_bits].codebook, g_tables[a.cv.n_bits].codebook, a.plan->rot, a.scale,
+                                     args[6] == Py_True, out.data_ptr(), half, wsp, wsp ? need : 0, pp, parts_need, stream);
     });
     if (status) return raise_status(status, "pq_prefill_attn");
     return THPVariable_Wrap(out);

@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
     } else if (PRE && warp < kMmaWarp) {
         // =================================================== copy warp: expanded tiles from the workspace
         if (warp == kPfSoftWarps) {
-            const uint8_t* rec0 = p.ws + (size_t)kvrow * ((p.S + kPfTok - 1) / kPfTok) * C::kRec;
+            const uint8_t* rec0 = p.ws + ((size_t)kvrow * ((p.S + kPfTok - 1) / kPfTok) + first / kPfTok) * C::kRec;
             for (int i = 0; i < n_tiles && ok; ++i) {
                 const int bb = i & 1;
                 const uint32_t par2 = (uint32_t)(((i >> 1) - 1) & 1);
@@ -792,7 +792,7 @@ __global__ void __launch_bounds__(pf_threads(PRE), 1) pq_prefill_attn_kernel(con
     __syncthreads();          // every tile buffer is dead
     tc_fence_after();
 
-    if (!PRE && p.parts) {
+    if (p.parts) {
         // ---- a split's record: the merge normalises and rotates back
         if (warp < kPfRowWarps) {
             const uint32_t tlane = tmem_base + ((uint32_t)(warp * 32) << 16);
@@ -981,17 +981,18 @@ extern "C" size_t pq_prefill_attn_workspace_bytes(int batch, int kv_heads, int64
     return (size_t)batch * kv_heads * (size_t)((seq_len + pq::kPfTok - 1) / pq::kPfTok) * rec;
 }
 
-// How many CTAs share a query tile's tokens.  A CTA has an SM to itself and walks its tiles one after the other (about
-// 2.8 us each), so a grid of fewer CTAs than SMs leaves the rest idle.  The cost of s splits, in tiles: waves of CTAs x
-// (set-up and epilogue, about 5, + tiles per split), and 3 for the merge kernel's launch and round trips.  One query tile per
-// KV head only: with more of them the expanded workspace is the faster way.  8 sequences x 8 KV heads, 5 positions x 4 heads
-// against 3001 tokens: one CTA per KV row 147 us, two 88 us.
+// How many CTAs share a query tile's tokens.  A CTA has an SM to itself and walks its tiles one after the other (2.8 us each
+// when it dequantises them, 1.6 from the workspace), so a grid of fewer CTAs than SMs leaves the rest idle.  The cost of s
+// splits, in tiles: waves of CTAs x (set-up and epilogue, about 6, + tiles per split), and for the merge kernel 3, plus its
+// waves of rows and its records' bytes.  8 sequences x 8 KV heads, 5 positions x 4 heads against 3001 tokens: one CTA per KV
+// row 147 us, two 88 us.
 static int prefill_splits(int rows, int64_t n_rows, int64_t seq_len) {
-    const int64_t tiles = (seq_len + pq::kPfTok - 1) / pq::kPfTok;
-    if (n_rows > pq::kPfRows || rows <= 0 || tiles < 2) return 1;
+    const int64_t tiles = (seq_len + pq::kPfTok - 1) / pq::kPfTok, out_rows = rows * n_rows;
+    const int64_t ctas = rows * ((n_rows + pq::kPfRows - 1) / pq::kPfRows);
+    if (ctas <= 0 || ctas >= 148) return 1;
     int64_t best = 1, best_cost = 0;
     for (int64_t s = 1; s <= 64 && s <= tiles; ++s) {
-        const int64_t cost = (rows * s + 147) / 148 * (5 + (tiles + s - 1) / s) + (s > 1 ? 3 : 0);
+        const int64_t cost = (ctas * s + 147) / 148 * (6 + (tiles + s - 1) / s) + (s > 1 ? 3 + out_rows / 700 + s * out_rows / 8000 : 0);
         if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
     }
     return (int)best;
@@ -1096,8 +1097,9 @@ extern "C" int pq_prefill_attn_split(const void* q, const void* k_blocks, const 
                                      int batch, int q_heads, int kv_heads, int seq_q, int64_t seq_len,
                                      int64_t seq_capacity, int head_dim, int k_bits, int v_bits,
                                      const float* codebook_k, const float* codebook_v, const float* rot,
-                                     float scale, int causal, void* out, int out_is_fp16, void* partials,
-                                     size_t partial_bytes, void* stream) {
+                                     float scale, int causal, void* out, int out_is_fp16, void* workspace,
+                                     size_t workspace_bytes, void* partials, size_t partial_bytes, void* stream) {
     return prefill_call(q, k_blocks, v_blocks, batch, q_heads, kv_heads, seq_q, seq_len, seq_capacity, head_dim, k_bits, v_bits,
-                        codebook_k, codebook_v, rot, scale, causal, out, out_is_fp16, nullptr, 0, partials, partial_bytes, stream);
+                        codebook_k, codebook_v, rot, scale, causal, out, out_is_fp16, workspace, workspace_bytes, partials,
+                        partial_bytes, stream);
 }

@@ -56,7 +56,7 @@ SIGNATURES = {
                                 c_void_p, c_int, c_void_p, c_size_t, c_void_p]),
     "pq_prefill_attn_split": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int64, c_int64,
                                 c_int, c_int, c_int, c_float_p, c_float_p, c_void_p, c_float, c_int,
-                                c_void_p, c_int, c_void_p, c_size_t, c_void_p]),
+                                c_void_p, c_int, c_void_p, c_size_t, c_void_p, c_size_t, c_void_p]),
     "pq_prefill_attn_partial_bytes": (c_size_t, [c_int, c_int, c_int, c_int, c_int64, c_int]),
     "pq_prefill_attn_workspace_bytes": (c_size_t, [c_int, c_int, c_int64, c_int]),
     # include/polarquant_llama_abi.h: the llama.cpp bridge's entry points
