@@ -72,7 +72,8 @@ __device__ __forceinline__ float fast_exp2(float x) {
 }
 
 // Raises a kernel's dynamic shared-memory limit, once per device (the driver call costs a few hundred nanoseconds, a
-// fifth of a launch).  `done` belongs to the kernel: a bit per device; racing first calls repeat the same setting.
+// fifth of a launch).  `bytes` is therefore the most that any call of this kernel asks for, the same on every call.
+// `done` belongs to the kernel: a bit per device; racing first calls repeat the same setting.
 template <typename Kernel>
 inline cudaError_t allow_shared(Kernel kern, size_t bytes, std::atomic<uint64_t>& done) {
     int dev = 0;
