@@ -17,7 +17,7 @@
 #include <cmath>
 #include <cstring>
 #include <deque>
-#include <vector>
+#include <string>
 
 #include "polarquant_b200.h"
 #include "polarquant_llama_abi.h"
@@ -77,59 +77,95 @@ const Plan* plan_of(PyObject* o) {
     return p;
 }
 
-// ------------------------------------------------------------------ plans by the matrix objects of a call
-// The identity of a matrix without reading it: the object, where its data lives, and for arrays three probe values,
-// for tensors the version counter.
-struct MatrixId {
-    PyObject* object = nullptr;
-    const void* data = nullptr;
-    int64_t size = 0, a = 0, b = 0, c = 0;
-    bool operator==(const MatrixId& o) const {
-        return object == o.object && data == o.data && size == o.size && a == o.a && b == o.b && c == o.c;
-    }
+// ------------------------------------------------------------------ plans by the matrices of a call
+// A matrix as a call gives it.  On the host (a C-contiguous float array or CPU tensor) it is its type, shape and bytes, all
+// of them: an edit in place anywhere is noticed, and an equal matrix in another object is recognised (two of 128 x 128 float64
+// take 5 us).  On a device it is the tensor object, its type and layout, and its version counter, which
+// every in-place operation of torch moves; reading the contents back would stop the stream.
+struct Matrix {
+    enum Kind { kNone, kHost, kDevice } kind = kNone;
+    int type = 0;                            // format character of an array, or 256 + scalar type of a tensor
+    int64_t size[2] = {0, 0}, stride[2] = {0, 0}, version = 0;
+    const void* data = nullptr;              // host: valid while the call's view is open
+    size_t bytes = 0;                        // host
+    PyObject* object = nullptr;              // device
 };
-bool matrix_id(PyObject* o, MatrixId* id) {
-    *id = MatrixId();
-    if (o == Py_None) return true;
-    id->object = o;
-    if (const at::Tensor* t = tensor(o)) {
-        if (t->layout() != at::kStrided || t->is_inference()) return false;      // (no version counter)
-        id->data = t->data_ptr();
-        id->size = t->numel();
-        id->a = t->_version();
+constexpr size_t kMatrixLimit = 1 << 20;     // larger ones are left to the caller's digest
+
+class MatrixView {
+  public:
+    Matrix m;
+    bool good;
+    explicit MatrixView(PyObject* o) : good(read(o)) {}
+    ~MatrixView() { if (open_) PyBuffer_Release(&buf_); }
+    MatrixView(const MatrixView&) = delete;
+    MatrixView& operator=(const MatrixView&) = delete;
+
+  private:
+    Py_buffer buf_;
+    bool open_ = false;
+    bool read(PyObject* o) {
+        if (o == Py_None) return true;
+        if (const at::Tensor* t = tensor(o)) {
+            if (t->layout() != at::kStrided || t->dim() != 2 || t->is_conj() || t->is_neg()) return false;
+            m.type = 256 + (int)t->scalar_type();
+            for (int i = 0; i < 2; ++i) { m.size[i] = t->size(i); m.stride[i] = t->stride(i); }
+            m.data = t->data_ptr();
+            if (t->is_cpu()) {
+                m.kind = Matrix::kHost;
+                m.bytes = t->nbytes();
+                return t->is_contiguous() && m.bytes <= kMatrixLimit;
+            }
+            if (t->is_inference()) return false;                 // (no version counter)
+            m.kind = Matrix::kDevice;
+            m.version = t->_version();
+            m.object = o;
+            return true;
+        }
+        if (PyObject_GetBuffer(o, &buf_, PyBUF_C_CONTIGUOUS | PyBUF_FORMAT) != 0) {
+            PyErr_Clear();
+            return false;
+        }
+        open_ = true;
+        const char* f = buf_.format;
+        if (buf_.ndim != 2 || !f || f[1] || (*f != 'd' && *f != 'f' && *f != 'e') || (size_t)buf_.len > kMatrixLimit) return false;
+        m.kind = Matrix::kHost;
+        m.type = *f;
+        for (int i = 0; i < 2; ++i) m.size[i] = buf_.shape[i];
+        m.data = buf_.buf;
+        m.bytes = (size_t)buf_.len;
         return true;
     }
-    Py_buffer buf;
-    if (PyObject_GetBuffer(o, &buf, PyBUF_SIMPLE) != 0) {        // contiguous arrays only
-        PyErr_Clear();
-        return false;
+};
+// A matrix kept from an earlier call: host bytes copied, a device tensor held (its identity cannot be reused meanwhile).
+struct KeptMatrix {
+    Matrix m;
+    std::string bytes;
+    explicit KeptMatrix(const Matrix& v) : m(v) {
+        if (m.kind == Matrix::kHost) bytes.assign((const char*)m.data, m.bytes);
+        Py_XINCREF(m.object);
     }
-    const bool ok = buf.len >= 8;
-    if (ok) {
-        const char* p = (const char*)buf.buf;
-        id->data = p;
-        id->size = buf.len;
-        memcpy(&id->a, p, 8);
-        memcpy(&id->b, p + (buf.len / 16) * 8, 8);
-        memcpy(&id->c, p + buf.len - 8, 8);
+    bool operator==(const Matrix& o) const {
+        if (m.kind != o.kind || m.type != o.type || m.size[0] != o.size[0] || m.size[1] != o.size[1]) return false;
+        if (m.kind == Matrix::kHost) return m.bytes == o.bytes && memcmp(bytes.data(), o.data, m.bytes) == 0;
+        return m.object == o.object && m.data == o.data && m.version == o.version && m.stride[0] == o.stride[0] &&
+               m.stride[1] == o.stride[1];
     }
-    PyBuffer_Release(&buf);
-    return ok;
-}
+};
 struct Known {
-    MatrixId r, p;
+    KeptMatrix r, p;
     int device;
     PyObject* plan;
 };
-std::deque<Known> g_known;          // strong references: the identities cannot be reused while an entry lives
+std::deque<Known> g_known;
 constexpr size_t kKnownLimit = 64;
 
 // Borrowed reference or nullptr.
 PyObject* known_plan(PyObject* R, PyObject* P, int device) {
-    MatrixId r, p;
-    if (!matrix_id(R, &r) || !matrix_id(P, &p)) return nullptr;
+    const MatrixView r(R), p(P);
+    if (!r.good || !p.good) return nullptr;
     for (auto it = g_known.rbegin(); it != g_known.rend(); ++it)
-        if (it->device == device && it->r == r && it->p == p) return it->plan;
+        if (it->device == device && it->r == r.m && it->p == p.m) return it->plan;
     return nullptr;
 }
 
@@ -145,22 +181,18 @@ PyObject* plan_get(PyObject*, PyObject* const* args, Py_ssize_t n) {
 // plan_put(R, device_index, P, plan)
 PyObject* plan_put(PyObject*, PyObject* const* args, Py_ssize_t n) {
     int64_t dev;
-    Known k;
-    if (n != 4 || !as_int(args[1], &dev) || !matrix_id(args[0], &k.r) || !matrix_id(args[2], &k.p)) Py_RETURN_NONE;
-    k.device = (int)dev;
-    k.plan = args[3];
-    Py_XINCREF(k.r.object);
-    Py_XINCREF(k.p.object);
-    Py_INCREF(k.plan);
-    Known old{};
-    if (g_known.size() >= kKnownLimit) {
-        old = g_known.front();
+    if (n != 4 || !as_int(args[1], &dev)) Py_RETURN_NONE;
+    const MatrixView r(args[0]), p(args[2]);
+    if (!r.good || !p.good || r.m.kind == Matrix::kNone) Py_RETURN_NONE;
+    g_known.push_back(Known{KeptMatrix(r.m), KeptMatrix(p.m), (int)dev, args[3]});
+    Py_INCREF(args[3]);
+    if (g_known.size() > kKnownLimit) {
+        const Known old = std::move(g_known.front());
         g_known.pop_front();
+        Py_XDECREF(old.r.m.object);
+        Py_XDECREF(old.p.m.object);
+        Py_DECREF(old.plan);
     }
-    g_known.push_back(k);
-    Py_XDECREF(old.r.object);
-    Py_XDECREF(old.p.object);
-    Py_XDECREF(old.plan);
     Py_RETURN_NONE;
 }
 

@@ -116,10 +116,11 @@ def _digest(m) -> str:
 
 
 def device_plan(rotation_matrix, device, jl_matrix=None) -> DevicePlan:
-    """Cached DevicePlan for (R, P, device).  The same matrix OBJECTS are recognised without being read
-    (the usual case: a caller passes its R and P on every call) by where their data lives and three probe values
-    (tensors: the version counter), enough to notice the in-place edits that the digest would notice; otherwise the
-    plan is looked up by a digest of the contents.  Callers on a hot loop can also hold the plan and pass it instead of R."""
+    """Cached DevicePlan for (R, P, device), looked up by what the matrices hold: C-contiguous float arrays and CPU tensors
+    are compared byte by byte with those of earlier plans, other host forms go through a digest.  CUDA tensors are
+    recognised by the object and its version counter instead, which every in-place operation moves; a write that goes
+    past it (through ``.data``, from another library's kernel) needs a new tensor or a plan of its own.  Callers on a hot
+    loop can also hold the plan and pass it instead of R."""
     if isinstance(rotation_matrix, DevicePlan):
         return rotation_matrix
     dev = torch.device(device)

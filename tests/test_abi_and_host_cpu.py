@@ -429,3 +429,35 @@ def test_host_module_turns_cpp_exceptions_into_python_errors():
         torch.vmap(lambda m: host.plan_get(m, 0, None) or m)(torch.zeros(2, 4, 4))
     with torch.inference_mode():
         assert host.plan_get(torch.zeros(4, 4), 0, None) is None
+
+
+def test_kept_plans_are_found_by_what_the_matrices_hold():
+    """Host matrices are compared whole: an edit of any element (none of the first, middle and last among them), another
+    shape or another type is another matrix; an equal matrix in another object is the same.  The plans here are stand-ins."""
+    import torch
+
+    from polarquant_kv import _ext
+    host = _ext.host()
+    rng = np.random.default_rng(3)
+    for wrap in (lambda a: a, lambda a: torch.from_numpy(a)):
+        base, proj = rng.standard_normal((64, 64)), rng.standard_normal((32, 64))
+        R, P, plan, plain = wrap(base), wrap(proj), object(), object()
+        host.plan_put(R, 0, P, plan)
+        host.plan_put(R, 0, None, plain)
+        assert host.plan_get(R, 0, P) is plan and host.plan_get(R, 0, None) is plain
+        assert host.plan_get(R, 1, P) is None and host.plan_get(P, 0, R) is None
+        assert host.plan_get(wrap(base.copy()), 0, wrap(proj.copy())) is plan
+        for i, j in ((5, 17), (0, 1), (63, 62), (31, 63), (32, 0)):
+            kept, base[i, j] = base[i, j], base[i, j] + 1e-3
+            assert host.plan_get(R, 0, P) is None and host.plan_get(R, 0, None) is None
+            base[i, j] = kept
+            assert host.plan_get(R, 0, P) is plan
+        base[:] = np.asarray(rng.permutation(base))
+        assert host.plan_get(R, 0, P) is None
+    square = rng.standard_normal((64, 64))
+    host.plan_put(square, 0, None, plan)
+    for other in (square.reshape(32, 128), square.ravel(), square.T, square.astype(np.float32), square.view(np.int64),
+                  square[:, :32]):
+        assert host.plan_get(other, 0, None) is None
+    square.shape = (128, 32)
+    assert host.plan_get(square, 0, None) is None
