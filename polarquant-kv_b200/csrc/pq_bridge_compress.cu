@@ -1,30 +1,35 @@
 // Compress of the llama.cpp bridge's codec for head dims 64 and 128 and more than a few hundred vectors: rotate,
 // Euclidean norm, divide, nearest level of a device-side codebook, pack two indices per byte.
 //
-// The rotation is a [N x D] . [D x D] product of float32 operands.  On CUDA cores it is the bound (17 TFLOP at 2^20
+// The rotation is a [N x D] . [D x D] product of float32 operands.  On CUDA cores it is the bound (34 GFLOP at 2^20
 // vectors of 128: 0.5 ms at the FP32 peak); here it runs on the 5th-generation tensor cores with both operands as the
-// sum of three bfloat16 terms, which is exact for float32 (3 x 8 significant bits) and needs no range scaling.  Six of
-// the nine product terms are issued; the three left out are below 2^-24 of the product.  The correction terms go into
-// the accumulator before the leading one, so they are added while the accumulator is still small.
+// sum of three bfloat16 terms.  The tensor core cuts off what falls below its accumulator's last bit at every step, always
+// towards zero, which took 1.4e-7 off every radius while all products shared one accumulator and the leading terms were the
+// operands rounded to bfloat16.  Therefore
+//   * the leading term of a row (of x, of R) is the row in whole units of 2^-8 of its largest element's power of two:
+//     integers up to 256, whose products add up to at most 2^23 units at D = 128, exactly;
+//   * their sum has an accumulator to itself.  The five correction products (the three left out are below 2^-25 of the
+//     largest one) go into a second one, whose cuts are 2^-8 as large, and the two are added in float32.
+// The error of a coordinate is then a third of an FP32 chain's, that of the radius four fifths (3.3e-8 against 4.2e-8 rms).
 //
 // A persistent CTA owns 128 vectors at a time:
 //   copy warp    boxes of 128 vectors x 32 floats by TMA (128-byte swizzle), a ring of them in flight;
 //   worker warps (4 per 32 dims) one thread = one vector x 32 dims: reads its row of the box, writes the three terms
-//                into tensor memory as the A operand (two buffers); one tile behind, reads its 32 accumulator columns
-//                and runs the float32 epilogue;
+//                into tensor memory as the A operand; one tile behind, reads its 32 columns of both accumulators
+//                and runs the float32 epilogue, under which the MMAs of the next tile go on;
 //   MMA warp     6 x D/16 MMAs per tile (A from tensor memory, B = the three terms of R in shared memory), 3.1 K
-//                cycles at D = 128, which is what the tile's 74 KB take at the HBM's rate (3.2 K): the kernel is
-//                balanced between the two.
+//                cycles at D = 128.
 // Index search: the reference scans the levels and keeps the first of the closest.  For a codebook in ascending order
 // that is "how many decision points lie below", with the decision points found once per CTA by bisection over the
 // float32 numbers; a coordinate's bucket (1/128 wide) holds at most one of them.  Any other codebook (unsorted, levels
 // closer than 1e-5, two decision points in a bucket) is scanned level by level as the reference does.
-// Measured (D = 128, 16 levels): 131 072 vectors 45 us with the second pass described below, 32 without it (the FP32 kernel
-// before it, R^T in shared memory: 226 us).
+// Measured (16 levels, second pass included): 131 072 vectors of 128 48 us, 2^20 of them 242 (R^T in shared memory on CUDA
+// cores: 238 and 1834); of 64: 29 and 125 us (80 and 595).  One accumulator and plain bfloat16 terms: 45.5, 230, 27, 117.
 // The rotation's last bits depend on the order of its additions, and a coordinate within them of a decision point gets one
 // index or the other.  So that stored bytes do not depend on which kernel wrote them, a block with a coordinate closer
 // than kBcNear to a decision point (one in 500 at 16 levels) is put on a list and done again at the end in the order of
-// an FP32 chain, k ascending per output.  R's fp32 words are the exact sums of their three terms in shared memory.
+// an FP32 chain, k ascending per output, with R copied over the boxes, which are free by then.  The same goes for whole vectors whose radius is not a number,
+// infinite, or so small that its squares are subnormal: there too the stored values are the chain's.
 // All waits are bounded (bit 10 of pq_poll_device_errors).
 #include <cstring>
 
@@ -58,11 +63,11 @@ struct BridgeCompressCfg {
     static constexpr uint32_t kBoxAddr = (kBAddr + 3 * kBTerm + 1023) & ~1023u;
     static constexpr uint32_t kSmallAddr = kBoxAddr + kBoxes * kBox;
     static constexpr uint32_t kATerm = D / 2;                      // tensor-memory columns of one term
-    static constexpr uint32_t kABuf = 3 * kATerm;
-    static constexpr uint32_t kAcc = 2 * kABuf;
-    static constexpr uint32_t kTmemCols = D == 128 ? 512 : 256;
-    // norms [2][128][WG], codebook 16, decision points 16, barriers, tensor-memory slot, abort flag, fast flag
-    static constexpr uint32_t kSmall = 2 * kBcVecs * WG * 4 + 2 * 16 * 4 + (2 * kBoxes + 6) * 8 + 32 + kBcList * 4;
+    static constexpr uint32_t kAcc = 2 * D;                        // leading products; the corrections D columns further
+    static constexpr uint32_t kTmemCols = 4 * D;
+    // norms and largest elements [2][128][WG] each, codebook 16, decision points 16, barriers, tensor-memory slot, abort
+    // flag, fast flag, list
+    static constexpr uint32_t kSmall = 4 * kBcVecs * WG * 4 + 2 * 16 * 4 + (2 * kBoxes + 6) * 8 + 32 + kBcList * 4;
     static constexpr size_t smem_bytes() { return kSmallAddr + kSmall; }
 };
 
@@ -84,16 +89,32 @@ __device__ __forceinline__ float2 bc_fma2(float2 a, float2 b, float2 c) {
           "l"(*reinterpret_cast<unsigned long long*>(&c)));
     return d;
 }
+__device__ __forceinline__ float2 bc_add2(float2 a, float2 b) {
+    float2 d;
+    asm("add.rn.f32x2 %0, %1, %2;\n"
+        : "=l"(*reinterpret_cast<unsigned long long*>(&d))
+        : "l"(*reinterpret_cast<unsigned long long*>(&a)), "l"(*reinterpret_cast<unsigned long long*>(&b)));
+    return d;
+}
+// 1.5 x 2^23 units, for a row whose largest element is `most` and whose unit is 2^-8 of the power of two above it: adding
+// and taking it off again rounds to whole units.  From 2^112 on it is not a number, and then the whole row becomes none.
+__device__ __forceinline__ float bc_unit_magic(float most) {
+    return __uint_as_float((min((__float_as_uint(most) >> 23) + 16u, 255u) << 23) | 0x400000u);
+}
+// leading term of two elements, packed bfloat16 (exact), and what it leaves (exact)
+__device__ __forceinline__ uint32_t bc_lead(float2& x, float magic) {
+    const float2 h = bc_add2(bc_add2(x, make_float2(magic, magic)), make_float2(-magic, -magic));
+    uint32_t w;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(w) : "f"(h.y), "f"(h.x));
+    x = bc_fma2(h, make_float2(-1.f, -1.f), x);
+    return w;
+}
 // two floats -> packed bfloat16 (first in the low half), and what the rounding left
 __device__ __forceinline__ uint32_t bc_term(float2& x) {
     uint32_t w;
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(w) : "f"(x.y), "f"(x.x));
     const float2 neg = make_float2(__uint_as_float((w << 16) ^ 0x80000000u), __uint_as_float((w & 0xFFFF0000u) ^ 0x80000000u));
-    float2 r;
-    asm("add.rn.f32x2 %0, %1, %2;\n"
-        : "=l"(*reinterpret_cast<unsigned long long*>(&r))
-        : "l"(*reinterpret_cast<unsigned long long*>(&x)), "l"(*reinterpret_cast<const unsigned long long*>(&neg)));
-    x = r;                                                          // exact
+    x = bc_add2(x, neg);                                            // exact
     return w;
 }
 __device__ __forceinline__ void bc_tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
@@ -124,15 +145,21 @@ struct BridgeCompressParams {
     int N, n_levels;
 };
 
-// One block of one vector once more, by a whole warp (lane l: elements l + 32 i): k ascending per output as on CUDA cores,
-// squares as a tree over i and the lanes, then level by level.  Its 16 bytes were stored before.  (Out of line and with
-// real loops: it runs for a few blocks per CTA, and straight-line code would spend its time on instruction fetches.)
+// Byte offset of R[n][k] in the second pass's copy: consecutive n at one k, and consecutive k at one n, are in different banks.
 template <int D>
-__device__ __noinline__ void bc_again(const float* input, uint8_t* packed_out, const float* cb, int n_levels, int vec, int block) {
+__device__ __forceinline__ uint32_t bc_staged(int n, int k) { return (uint32_t)(k * D + (n ^ (k & 31))) * 4; }
+
+// One block of one vector once more, by a whole warp (lane l: elements l + 32 i): k ascending per output as on CUDA cores,
+// squares as a tree over i and the lanes, then level by level; block 0 brings the radius along.  What it overwrites was
+// stored by this warp, or before a barrier.  (Out of line and with real loops: it runs for a few blocks per CTA, and
+// straight-line code would spend its time on instruction fetches.)  SHARED: R is where the second pass put it, else in L2,
+// whose lines every lane of a load would hit one of (ten times the time).
+template <int D, bool SHARED>
+__device__ __noinline__ void bc_again(const BridgeCompressParams& p, const float* cb, int vec, int block) {
     using C = BridgeCompressCfg<D>;
     constexpr int WG = C::WG;
     const int lane = threadIdx.x & 31;
-    const float* x = input + (size_t)vec * D;
+    const float* x = p.x + (size_t)vec * D;
     float acc[WG], xl[WG];
 #pragma unroll
     for (int m = 0; m < WG; ++m) { xl[m] = __ldg(x + lane + 32 * m); acc[m] = 0.f; }
@@ -147,20 +174,13 @@ __device__ __noinline__ void bc_again(const float* input, uint8_t* packed_out, c
         }
 #pragma unroll
         for (int i = 0; i < WG; ++i) {
-            // R[n][8 kc .. 8 kc + 7]: the sum of the three terms, exact in any order
-            const int n = lane + 32 * i;
-            const uint32_t a = C::kBAddr + (uint32_t)(kc * (D / 8) * 128 + (n >> 3) * 128 + (n & 7) * 16);
-            float r[8];
+            float r[8];                                        // R[lane + 32 i][8 kc .. 8 kc + 7]
 #pragma unroll
-            for (int t = 2; t >= 0; --t) {
-                uint32_t w[4];
-                asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "r"(a + t * C::kBTerm));
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float lo = __uint_as_float(w[k] << 16), hi = __uint_as_float(w[k] & 0xFFFF0000u);
-                    r[2 * k] = t == 2 ? lo : r[2 * k] + lo;
-                    r[2 * k + 1] = t == 2 ? hi : r[2 * k + 1] + hi;
-                }
+            for (int k = 0; k < 8; ++k) {
+                if constexpr (SHARED)
+                    asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(r[k]) : "r"(C::kBoxAddr + bc_staged<D>(lane + 32 * i, 8 * kc + k)));
+                else
+                    r[k] = __ldg(p.R + (size_t)(lane + 32 * i) * D + 8 * kc + k);
             }
 #pragma unroll
             for (int k = 0; k < 8; ++k) acc[i] = fmaf(xv[k], r[k], acc[i]);
@@ -185,18 +205,19 @@ __device__ __noinline__ void bc_again(const float* input, uint8_t* packed_out, c
     uint32_t best = 0;
     float dist = 1e30f;
 #pragma unroll 1
-    for (int l = 0; l < n_levels; ++l) {
+    for (int l = 0; l < p.n_levels; ++l) {
         const float d = fabsf(dir - cb[l]);
         if (d < dist) { dist = d; best = l; }
     }
     const uint32_t up = __shfl_down_sync(0xffffffffu, best, 1);
     __syncwarp();
-    if (!(lane & 1)) packed_out[(size_t)vec * (D / 2) + block * 16 + (lane >> 1)] = (uint8_t)(best | (up << 4));
+    if (!(lane & 1)) p.packed_out[(size_t)vec * (D / 2) + block * 16 + (lane >> 1)] = (uint8_t)(best | (up << 4));
+    if (block == 0 && lane == 0) p.radius_out[vec] = radius;
 }
 
 template <int D>
 __global__ void __launch_bounds__(BridgeCompressCfg<D>::THREADS, 1)
-bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUtensorMap x_map) {
+bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __grid_constant__ CUtensorMap x_map) {
     using C = BridgeCompressCfg<D>;
     constexpr int WG = C::WG, WORKERS = C::WORKERS, NB = C::kBoxes;
     extern __shared__ __align__(128) uint8_t smem[];
@@ -208,11 +229,12 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
     uint8_t* zero = smem - base;                               // generic address of shared address 0
     uint8_t* Bt = zero + C::kBAddr;
     float* norm_s = reinterpret_cast<float*>(zero + C::kSmallAddr);          // [tile parity][vector][WG]
-    float* cb = norm_s + 2 * kBcVecs * WG;
+    float* most_s = norm_s + 2 * kBcVecs * WG;                               // the same
+    float* cb = most_s + 2 * kBcVecs * WG;
     float* thr = cb + 16;
     uint64_t* mbar = reinterpret_cast<uint64_t*>(thr + 16);
-    // [0, NB) box landed; [NB, 2 NB) box read; then A buffer 0 / 1 written; tile's MMAs done (per parity: frees the A
-    // buffer, completes the accumulator); accumulator read out (per parity)
+    // [0, NB) box landed; [NB, 2 NB) box read; then, per parity of the tile: A written; its MMAs done (A free, the
+    // accumulators complete); accumulators read out
     uint64_t* box_full = mbar;
     uint64_t* box_free = mbar + NB;
     uint64_t* a_full = mbar + 2 * NB;
@@ -242,19 +264,44 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
         *n_list = 0;
     }
     if (tid < 16) cb[tid] = __ldg(p.codebook + min(tid, p.n_levels - 1));
-    // B: three bfloat16 terms of R, K-major core matrices (8 rows x 16 bytes), K chunks D / 8 * 128 bytes apart
-    for (int e = tid; e < D * (D / 8); e += C::THREADS) {
-        const int n = (e & 7) + 8 * (e / (8 * (D / 8))), kc = (e >> 3) % (D / 8);
-        float2 x[4];
+    // B: three bfloat16 terms of R, K-major core matrices (8 rows x 16 bytes), K chunks D / 8 * 128 bytes apart.  A thread's
+    // pieces (8 elements of a row) are all in flight at once; the largest element of a row comes from its pieces' threads.
+    {
+        constexpr int PIECES = D * (D / 8), MINE = (PIECES + C::THREADS - 1) / C::THREADS;
+        auto row = [](int e) { return (e & 7) + 8 * (e / D); };
+        auto chunk = [](int e) { return (e >> 3) % (D / 8); };
+        float2 x[MINE][4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = __ldg(reinterpret_cast<const float2*>(p.R + (size_t)n * D + kc * 8) + i);
-        const uint32_t off = (uint32_t)(kc * (D / 8) * 128 + (n >> 3) * 128 + (n & 7) * 16);
+        for (int j = 0; j < MINE; ++j) {
+            const int e = min(tid + j * C::THREADS, PIECES - 1);
 #pragma unroll
-        for (int t = 0; t < 3; ++t) {
-            uint32_t w[4];
+            for (int i = 0; i < 4; ++i) x[j][i] = __ldg(reinterpret_cast<const float2*>(p.R + (size_t)row(e) * D + chunk(e) * 8) + i);
+        }
+        if (tid < D) most_s[tid] = 0.f;
+        __syncthreads();
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = bc_term(x[i]);
-            *reinterpret_cast<uint4*>(Bt + t * C::kBTerm + off) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int j = 0; j < MINE; ++j) {
+            float most = 0.f;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) most = fmaxf(most, fmaxf(fabsf(x[j][i].x), fabsf(x[j][i].y)));
+            // (the bits of floats that are not negative are in their order)
+            atomicMax(reinterpret_cast<int*>(most_s) + row(min(tid + j * C::THREADS, PIECES - 1)), __float_as_int(most));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < MINE; ++j) {
+            const int e = tid + j * C::THREADS;
+            if (e >= PIECES) break;
+            const int n = row(e);
+            const uint32_t off = (uint32_t)(chunk(e) * (D / 8) * 128 + (n >> 3) * 128 + (n & 7) * 16);
+            const float unit = bc_unit_magic(most_s[n]);
+#pragma unroll
+            for (int t = 0; t < 3; ++t) {
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) w[i] = t == 0 ? bc_lead(x[j][i], unit) : bc_term(x[j][i]);
+                *reinterpret_cast<uint4*>(Bt + t * C::kBTerm + off) = make_uint4(w[0], w[1], w[2], w[3]);
+            }
         }
     }
     if (warp == 0) tmem_alloc(sm_addr(tmem_slot), C::kTmemCols);
@@ -331,16 +378,15 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
             if (i >= 1) ok = mbar_wait(sm_addr(acc_free + (b ^ 1)), (uint32_t)((i - 1) >> 1) & 1u, abort_s, 32) && ok;
             if (!ok) break;
             tc_fence_after();
-            const uint32_t a = tmem_base + b * C::kABuf;
-            // (term of x, term of R): the smallest products first
-            constexpr int ta[6] = {2, 0, 1, 1, 0, 0}, tb[6] = {0, 2, 1, 0, 1, 0};
+            // (term of x, term of R): the leading products, then the corrections, smallest first
+            constexpr int ta[6] = {0, 2, 0, 1, 1, 0}, tb[6] = {0, 0, 2, 1, 0, 1};
 #pragma unroll
             for (int t = 0; t < 6; ++t)
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
-                    umma_f16_ts_pred(acc, a + ta[t] * C::kATerm + ks * 8,
+                    umma_f16_ts_pred(acc + (t ? D : 0), tmem_base + ta[t] * C::kATerm + ks * 8,
                                      b0 + (uint32_t)((tb[t] * C::kBTerm + 2 * ks * kLbo) >> 4), b_hi, idesc,
-                                     (t || ks) ? 1u : 0u, issue);
+                                     (t > 1 || ks) ? 1u : 0u, issue);
             umma_commit_pred(sm_addr(mma_done + b), issue);
             __syncwarp();
         }
@@ -379,30 +425,45 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
                 x[2 * c + 1] = make_float2(v.z, v.w);
             }
             mbar_arrive(sm_addr(box_free + slot));
-            const uint32_t b = i & 1;
-            if (i >= 2) {                                      // the A buffer's MMAs (tile i - 2) are done
-                ok = mbar_wait(sm_addr(mma_done + b), (uint32_t)((i >> 1) - 1) & 1u, abort_s) && ok;
+            // the vector's largest element, from its WG threads (infinities and NaN turn up in the radius)
+            float most = fmaxf(fabsf(x[0].x), fabsf(x[0].y));
+#pragma unroll
+            for (int k = 1; k < 16; ++k) most = fmaxf(most, fmaxf(fabsf(x[k].x), fabsf(x[k].y)));
+            float* ms = most_s + (i & 1) * kBcVecs * WG + row * WG;
+            ms[wg] = most;
+            asm volatile("bar.sync %0, %1;\n" ::"r"(1 + q), "r"(32 * WG) : "memory");
+#pragma unroll
+            for (int k = 0; k < WG; ++k) most = fmaxf(most, ms[k]);
+            const float unit = bc_unit_magic(most);
+            if (i >= 1) {                                      // the MMAs of the tile before are done with A
+                ok = mbar_wait(sm_addr(mma_done + ((i - 1) & 1)), (uint32_t)((i - 1) >> 1) & 1u, abort_s) && ok;
                 tc_fence_after();
             }
 #pragma unroll
             for (int t = 0; t < 3; ++t) {
                 uint32_t w[16];
 #pragma unroll
-                for (int k = 0; k < 16; ++k) w[k] = bc_term(x[k]);
-                bc_tmem_st16(tmem_lane + b * C::kABuf + t * C::kATerm + wg * 16, w);
+                for (int k = 0; k < 16; ++k) w[k] = t == 0 ? bc_lead(x[k], unit) : bc_term(x[k]);
+                bc_tmem_st16(tmem_lane + t * C::kATerm + wg * 16, w);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
             tc_fence_before();
-            mbar_arrive(sm_addr(a_full + b));
+            mbar_arrive(sm_addr(a_full + (i & 1)));
         };
         auto epilogue = [&](int i) -> bool {
             const uint32_t b = i & 1;
             ok = mbar_wait(sm_addr(mma_done + b), (uint32_t)(i >> 1) & 1u, abort_s) && ok;
             tc_fence_after();
             float2 v2[16];
-            tmem_ld32(v2, tmem_lane + C::kAcc + wg * 32);
-            tc_fence_before();
-            mbar_arrive(sm_addr(acc_free + b));
+            {
+                float2 low[16];
+                tmem_ld32(v2, tmem_lane + C::kAcc + wg * 32);
+                tmem_ld32(low, tmem_lane + C::kAcc + D + wg * 32);
+                tc_fence_before();
+                mbar_arrive(sm_addr(acc_free + b));
+#pragma unroll
+                for (int k = 0; k < 16; ++k) v2[k] = bc_add2(v2[k], low[k]);
+            }
             // squares: this thread's 32 as a tree, then the vector's WG parts
             float2 s2[16];
 #pragma unroll
@@ -429,6 +490,15 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
             }
             const float radius = __fsqrt_rn(ss);
             const int vec = ((int)blockIdx.x + i * (int)gridDim.x) * kBcVecs + row;
+            // radii that the FP32 chain has to give: its infinities and NaN are others, and subnormal squares lose bits
+            bool odd = !(radius >= 1e-17f && radius <= 1.8e19f);
+            if (odd) {
+                const float* ms = most_s + (i & 1) * kBcVecs * WG + row * WG;
+                float most = ms[0];
+#pragma unroll
+                for (int k = 1; k < WG; ++k) most = fmaxf(most, ms[k]);
+                odd = !(radius == 0.f && most == 0.f);              // (rows of zeros are common)
+            }
             const bool live = radius > 1e-30f && radius < 3.4e38f;      // otherwise every direction is 0
             const float dsafe = live ? radius : 1.f;
             // IEEE-rounded quotient from the correctly rounded reciprocal and one residual step (Markstein 1990)
@@ -486,7 +556,7 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
                 *reinterpret_cast<uint4*>(p.packed_out + (size_t)vec * (D / 2) + wg * 16) =
                     make_uint4(packed[0], packed[1], packed[2], packed[3]);
             }
-            uint32_t todo = __ballot_sync(0xffffffffu, near < kBcNear && live && vec < p.N);
+            uint32_t todo = __ballot_sync(0xffffffffu, ((near < kBcNear && live) || odd) && vec < p.N);
             if (todo) {
                 int at = 0;
                 if (lane == 0) at = atomicAdd(n_list, __popc(todo));
@@ -497,7 +567,7 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
                 while (todo) {                                 // the list is full: at once
                     const int v = __ffs(todo) - 1;
                     todo &= todo - 1;
-                    bc_again<D>(p.x, p.packed_out, cb, p.n_levels, vec - lane + v, wg);
+                    bc_again<D, false>(p, cb, vec - lane + v, wg);
                 }
             }
             return true;
@@ -508,9 +578,17 @@ bridge_compress_kernel(const BridgeCompressParams p, const __grid_constant__ CUt
             if (i >= 1) going = epilogue(i - 1);
         }
         if (going && n_my >= 1) epilogue(n_my - 1);
-        asm volatile("bar.sync 9, %0;\n" ::"r"(WORKERS) : "memory");       // the list is complete, its blocks are stored
+        // the second pass: the list is complete, its blocks are stored, and every box has been read
+        static_assert((uint32_t)D * D * 4 <= NB * C::kBox, "R fits the boxes");
+        const bool stop = group_barrier_any(9u, WORKERS, !ok || *abort_s != 0u);
         const int n = min(*n_list, kBcList);
-        for (int e = warp; e < n; e += WORKERS / 32) bc_again<D>(p.x, p.packed_out, cb, p.n_levels, list[e] / WG, list[e] % WG);
+        if (n > 0 && !stop) {
+#pragma unroll 8
+            for (int e = tid; e < D * D; e += WORKERS)
+                *reinterpret_cast<float*>(zero + C::kBoxAddr + bc_staged<D>(e / D, e % D)) = __ldg(p.R + e);
+            asm volatile("bar.sync 9, %0;\n" ::"r"(WORKERS) : "memory");
+            for (int e = warp; e < n; e += WORKERS / 32) bc_again<D, true>(p, cb, list[e] / WG, list[e] % WG);
+        }
     }
     if (!ok && lane == 0) { *abort_s = 1u; atomicOr(&g_bridge_compress_error, 1u); }
     if (*abort_s && tid == 0) {                                // give box copies still in flight time to land

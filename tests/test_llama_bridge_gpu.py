@@ -230,3 +230,107 @@ def test_fused_attention_group_widths_vs_oracle(hq, hkv, s, d):
     # float32 throughout: scores of a few tens carry about 1e-5, which the weights inherit
     assert np.abs(out - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
     assert _ext.poll_device_errors() == 0
+
+
+def fp32_chain(x, R, cb):
+    """The bridge's compress in float32 as a chain: k ascending per coordinate, one rounding per multiply-add; squares as a
+    tree (element t with t + D/2, then + D/4, ...); quotient; the first of the closest levels.  (A float64 sum rounded to
+    float32 is the fused operation's result but for ties of the double rounding, one in 2^29.)"""
+    n, d = x.shape
+    xd, Rd = torch.from_numpy(x).cuda().double(), torch.from_numpy(R).cuda().double()
+    acc = torch.zeros(n, d, device="cuda")
+    for k in range(d):
+        acc = (acc.double() + xd[:, k:k + 1] * Rd[:, k][None]).float()
+    v = acc.cpu().numpy()
+    with np.errstate(all="ignore"):
+        t = v * v
+        while t.shape[1] > 1:
+            t = t[:, :t.shape[1] // 2] + t[:, t.shape[1] // 2:]
+        radius = np.sqrt(t[:, 0])
+        direction = np.where(radius[:, None] > np.float32(1e-30), v / radius[:, None], np.float32(0))
+        best, dist = np.zeros((n, d), np.uint8), np.full((n, d), 1e30, np.float32)
+        for level in range(len(cb)):
+            far = np.abs(direction - cb[level])
+            closer = far < dist
+            best[closer], dist[closer] = level, far[closer]
+    return radius, (best[:, 0::2] | (best[:, 1::2] << 4)).astype(np.uint8)
+
+
+def kv_like(n, d, rng):
+    scale = np.exp(rng.standard_normal(d))
+    scale[rng.choice(d, 2, replace=False)] *= 10.0
+    return (rng.standard_normal((n, d)) * scale).astype(np.float32)
+
+
+@pytest.mark.parametrize("d,n", [(128, 20_003), (64, 30_001), (128, 4096)])
+@pytest.mark.parametrize("kind", ["kv", "normal", "positive"])
+def test_radius_is_as_close_to_64_bits_as_an_fp32_chain(d, n, kind):
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(n + d)
+    x = kv_like(n, d, rng) if kind == "kv" else rng.standard_normal((n, d)).astype(np.float32)
+    if kind == "positive":
+        x = np.abs(x) + np.float32(1)
+    R, cb = orthogonal(d, rng), codebook_for(16, rng)
+    radius, _ = LB.compress(torch.from_numpy(x).cuda(), torch.from_numpy(R).cuda(), torch.from_numpy(cb).cuda())
+    chain, _ = fp32_chain(x, R, cb)
+    want = np.linalg.norm(x.astype(np.float64) @ R.astype(np.float64).T, axis=1)
+    off = lambda r: (r.astype(np.float64) - want) / want
+    ours, theirs = off(radius.cpu().numpy()), off(chain)
+    print(f"radius D{d} {kind}: rms {np.sqrt((ours**2).mean()):.2e} mean {ours.mean():.1e} (chain {np.sqrt((theirs**2).mean()):.2e})")
+    assert np.sqrt((ours**2).mean()) <= np.sqrt((theirs**2).mean())
+    assert np.abs(ours.mean()) <= 2.0**-25                     # no drift of more than half a rounding
+
+
+@pytest.mark.parametrize("d,n", [(128, 4097), (64, 4097), (128, 3)])
+def test_compress_of_infinities_nan_and_extreme_vectors(d, n):
+    """What the FP32 chain gives, from 4096 vectors on too: an infinity in an input is an infinite radius, not NaN."""
+    from polarquant_kv import _ext
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(d)
+    x = rng.standard_normal((n, d)).astype(np.float32)
+    special = {0: lambda v: v * np.float32(1e25), 1: lambda v: v * np.float32(0), 2: lambda v: np.where(np.arange(d) == 5, np.inf, v)}
+    if n > 3:
+        special.update({77: lambda v: np.where(np.arange(d) == d - 1, -np.inf, v), 78: lambda v: np.where(np.arange(d) == 40, np.nan, v),
+                        79: lambda v: v * np.float32(1e-20), 80: lambda v: v * np.float32(1e-23), 81: lambda v: v * np.float32(1e-39),
+                        200: lambda v: np.full(d, 3.4e38), 4096: lambda v: np.full(d, np.inf), 4095: lambda v: v * np.float32(3e18),
+                        300: lambda v: v * np.float32(1e-17)})
+    for row, f in special.items():
+        x[row] = f(x[row]).astype(np.float32)
+    R, cb = orthogonal(d, rng), codebook_for(16, rng)
+    radius, packed = LB.compress(torch.from_numpy(x).cuda(), torch.from_numpy(R).cuda(), torch.from_numpy(cb).cuda())
+    radius, packed = radius.cpu().numpy(), packed.cpu().numpy()
+    want_radius, want_packed = fp32_chain(x, R, cb)
+    rows = sorted(special)
+    assert np.array_equal(np.isnan(radius), np.isnan(want_radius)) and np.array_equal(np.isinf(radius), np.isinf(want_radius))
+    finite = np.isfinite(want_radius)
+    # subnormal squares: below 4096 vectors in another order, where a unit in the last place of the sum is up to 2^-10 of it
+    np.testing.assert_allclose(radius[finite], want_radius[finite], rtol=2e-6 if n > 3 else 1e-3)
+    assert np.array_equal(packed[rows], want_packed[rows])
+    assert _ext.poll_device_errors() == 0
+
+
+@pytest.mark.parametrize("d,n", [(128, 20_003), (64, 40_001), (128, 4096)])
+def test_near_ties_are_settled_as_an_fp32_chain_does(d, n):
+    """Half of the coordinates within 1e-6 of a decision point, so that nearly every block goes through the second pass and
+    the list of a CTA overflows (512 blocks a tile at D = 128, 256 at D = 64; it holds 480): every stored byte is the
+    chain's."""
+    from polarquant_kv import _ext
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(d + n)
+    R, cb = orthogonal(d, rng), codebook_for(16, rng)
+    points = (cb[1:].astype(np.float64) + cb[:-1]) / 2
+    points = points[np.abs(points) < 0.11]
+    direction = rng.standard_normal((n, d))
+    at = rng.permuted(np.tile(np.arange(d) % 2 == 0, (n, 1)), axis=1)
+    tied = rng.choice(points, (n, d)) + rng.uniform(-1e-6, 1e-6, (n, d))
+    rest = np.where(at, 0.0, direction)
+    room = 1.0 - (np.where(at, tied, 0.0) ** 2).sum(1, keepdims=True)
+    assert (room > 0).all()
+    unit = np.where(at, tied, rest * np.sqrt(room) / np.linalg.norm(rest, axis=1, keepdims=True))
+    x = (unit @ R.astype(np.float64) * np.exp(rng.uniform(-5, 5, (n, 1)))).astype(np.float32)
+    radius, packed = LB.compress(torch.from_numpy(x).cuda(), torch.from_numpy(R).cuda(), torch.from_numpy(cb).cuda())
+    want_radius, want_packed = fp32_chain(x, R, cb)
+    differ = int((packed.cpu().numpy() != want_packed).sum())
+    assert differ == 0, f"{differ} of {want_packed.size} bytes"
+    np.testing.assert_allclose(radius.cpu().numpy(), want_radius, rtol=5e-7)     # two roundings of the radius and its sums
+    assert _ext.poll_device_errors() == 0
