@@ -31,9 +31,8 @@ cudaError_t bridge_attention_launch(const BridgeAttnParams& p, int total_kv_head
 // bit 0: a bounded wait for a tile copy gave up; bit 1: the shared-memory window started too high
 int bridge_error_flags(unsigned int* flags);
 
-// pq_bridge_compress.cu: head dims 64 and 128, aligned buffers, at least kBridgeCompressMin vectors.
-constexpr int kBridgeCompressMin = 4096;
-bool bridge_compress_fits(int N, int D, const float* input, const float* rotation, const uint8_t* packed);
+// pq_bridge_compress.cu: head dims 64 and 128, aligned buffers.
+bool bridge_compress_fits(int D, const float* input, const float* rotation, const uint8_t* packed);
 cudaError_t bridge_compress_launch(const float* input, const float* rotation, const float* codebook, float* radius_out,
                                    uint8_t* packed_out, int N, int D, int n_levels, int sms, cudaStream_t st);
 // the same bits as bridge_error_flags

@@ -1,4 +1,4 @@
-// Compress of the llama.cpp bridge's codec for head dims 64 and 128 and more than a few hundred vectors: rotate,
+// Compress of the llama.cpp bridge's codec for head dims 64 and 128 and many vectors: rotate,
 // Euclidean norm, divide, nearest level of a device-side codebook, pack two indices per byte.
 //
 // The rotation is a [N x D] . [D x D] product of float32 operands.  On CUDA cores it is the bound (34 GFLOP at 2^20
@@ -601,10 +601,9 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
 }
 
 // ------------------------------------------------------------------ host side
-bool bridge_compress_fits(int N, int D, const float* input, const float* rotation, const uint8_t* packed) {
-    // Below kBridgeCompressMin the kernel with a few vectors per CTA, which reads R from L2, is about as fast (the set-up
-    // and the second pass here are a fixed cost of 17 us at D = 128), and its summation order settles near ties there.
-    return (D == 64 || D == 128) && N >= kBridgeCompressMin && (reinterpret_cast<uintptr_t>(input) & 15) == 0 &&
+bool bridge_compress_fits(int D, const float* input, const float* rotation, const uint8_t* packed) {
+    // a tensor map's base and 16-byte stores; the rotation is read in pairs
+    return (D == 64 || D == 128) && (reinterpret_cast<uintptr_t>(input) & 15) == 0 &&
            (reinterpret_cast<uintptr_t>(rotation) & 7) == 0 && (reinterpret_cast<uintptr_t>(packed) & 15) == 0;
 }
 

@@ -2,8 +2,9 @@
 // decoded lines 695-763) for sm_100a: the per-vector-radius codec with nibble-packed
 // indices, as kernels laid out for a 148-SM part instead of one CTA per vector / per head.
 //
-//   compress   head dims 64 and 128 and more than a few hundred vectors: pq_bridge_compress.cu (tensor cores); everything
-//              else one CTA per vector, which streams R from L2.
+//   compress   below 4096 vectors, and for other head dims than 64 and 128, a CTA takes one vector (four from 512 vectors
+//              on) and streams R from L2; above that an FP32 kernel with R^T in shared memory, and for buffers on 16-byte
+//              boundaries and more than a wave of its CTAs pq_bridge_compress.cu (tensor cores).
 //   attention  head dims 64 and 128: pq_bridge_attn.cu.  Other head dims: CTAs own (kv head, query group, slice of S); a
 //              warp takes 32 tokens at a time, each lane holds D/32 (rounded up) dims, the 32 partial dot products are
 //              transposed and summed with 31 shuffles so that lane t ends with token t's score; online softmax; the
@@ -19,6 +20,7 @@
 
 #include "polarquant_llama_abi.h"
 #include "pq_bridge.cuh"
+#include "pq_common.cuh"
 
 namespace {
 
@@ -139,6 +141,107 @@ __device__ __forceinline__ int nearest_level(float v, const float* cb, int n_lev
         if (d < dist) { dist = d; best = i; }
     }
     return best;
+}
+
+constexpr int kCmpWarps = 8;
+constexpr int kCmpVecs = 4;      // vectors a warp carries through the rotation together
+constexpr int kCmpMin = 4096;
+
+// Head dims 64 and 128, whatever the alignment.  R^T sits in shared memory once per CTA, a warp carries four vectors, lane l
+// owns rotated elements l + 32 i; the sum of squares is combined in the order of the reference's shared-memory tree.  The
+// tensor-core kernel stores the same bytes and is the faster one once there is more than a wave of this one's CTAs (Lloyd-Max
+// table, this kernel / that one: 9472 vectors of 128 22.6 / 22.8 us, 18 944 39 / 23; 18 944 vectors of 64 15.3 / 16.5 us,
+// 40 000 29 / 21).
+template <int D>
+__global__ void __launch_bounds__(kCmpWarps * 32) compress_kernel(const float* __restrict__ input,
+                                                                   const float* __restrict__ R,
+                                                                   const float* __restrict__ codebook,
+                                                                   float* __restrict__ radius_out,
+                                                                   uint8_t* __restrict__ packed_out,
+                                                                   int N, int n_levels) {
+    constexpr int DPL = D / 32;
+    constexpr int kPitch = D + 1;                       // transposed fill and row reads both conflict-free
+    extern __shared__ __align__(16) float smem[];
+    float* Rt = smem;                                   // Rt[k][j] = R[j][k]
+    float* xs = smem + D * kPitch;                      // [warp][k][kCmpVecs]
+    __shared__ float cb[16];
+    if (threadIdx.x < n_levels) cb[threadIdx.x] = codebook[threadIdx.x];
+    for (int e = threadIdx.x; e < D * D; e += blockDim.x) {
+        const int j = e / D, k = e - j * D;
+        Rt[k * kPitch + j] = R[e];
+    }
+    __syncthreads();
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float4* xw = reinterpret_cast<float4*>(xs + warp * D * kCmpVecs);
+    const int n_groups = (N + kCmpVecs - 1) / kCmpVecs;
+    for (int grp = blockIdx.x * kCmpWarps + warp; grp < n_groups; grp += gridDim.x * kCmpWarps) {
+        const int v0 = grp * kCmpVecs;
+        // stage the four inputs interleaved: xw[k] = {x0[k], x1[k], x2[k], x3[k]}
+        for (int k = lane; k < D; k += 32) {
+            float4 x;
+            x.x = input[(size_t)v0 * D + k];
+            x.y = v0 + 1 < N ? input[(size_t)(v0 + 1) * D + k] : 0.0f;
+            x.z = v0 + 2 < N ? input[(size_t)(v0 + 2) * D + k] : 0.0f;
+            x.w = v0 + 3 < N ? input[(size_t)(v0 + 3) * D + k] : 0.0f;
+            xw[k] = x;
+        }
+        __syncwarp();
+        float acc[kCmpVecs][DPL];
+#pragma unroll
+        for (int v = 0; v < kCmpVecs; ++v)
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) acc[v][i] = 0.0f;
+#pragma unroll 4
+        for (int k = 0; k < D; ++k) {
+            const float4 x = xw[k];
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) {
+                const float r = Rt[k * kPitch + lane + 32 * i];
+                acc[0][i] = fmaf(x.x, r, acc[0][i]);
+                acc[1][i] = fmaf(x.y, r, acc[1][i]);
+                acc[2][i] = fmaf(x.z, r, acc[2][i]);
+                acc[3][i] = fmaf(x.w, r, acc[3][i]);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int v = 0; v < kCmpVecs; ++v) {
+            // sum of squares: element t pairs with t + D/2, then + D/4, ... down to + 1
+            float sq[DPL];
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) sq[i] = __fmul_rn(acc[v][i], acc[v][i]);   // no contraction into the adds
+#pragma unroll
+            for (int h = DPL / 2; h; h >>= 1)
+#pragma unroll
+                for (int i = 0; i < h; ++i) sq[i] = __fadd_rn(sq[i], sq[i + h]);
+            float s = sq[0];
+#pragma unroll
+            for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+            const float radius = sqrtf(s);
+            const bool live = v0 + v < N;
+            if (live && lane == 0) radius_out[v0 + v] = radius;
+#pragma unroll
+            for (int i = 0; i < DPL; ++i) {
+                const float dir = radius > 1e-30f ? acc[v][i] / radius : 0.0f;
+                const int idx = nearest_level(dir, cb, n_levels);
+                const int up = __shfl_down_sync(kFull, idx, 1);
+                if (live && !(lane & 1))
+                    packed_out[(size_t)(v0 + v) * (D / 2) + (lane >> 1) + 16 * i] = (uint8_t)(idx | (up << 4));
+            }
+        }
+    }
+}
+
+template <int D>
+cudaError_t launch_compress(int ctas, const float* input, const float* R, const float* codebook, float* radius_out,
+                            uint8_t* packed_out, int N, int n_levels, cudaStream_t stream) {
+    constexpr size_t smem = ((size_t)D * (D + 1) + (size_t)kCmpWarps * D * kCmpVecs) * sizeof(float);
+    static std::atomic<uint64_t> allowed{0};
+    const cudaError_t e = pq::allow_shared(compress_kernel<D>, smem, allowed);
+    if (e != cudaSuccess) return e;
+    compress_kernel<D><<<ctas, kCmpWarps * 32, smem, stream>>>(input, R, codebook, radius_out, packed_out, N, n_levels);
+    return cudaGetLastError();
 }
 
 // Any even head dim up to 1024: V vectors per CTA.  One, so that a token's few vectors spread over the SMs; four once there
@@ -600,11 +703,21 @@ void polarquant_compress_cuda_c(const float* input, const float* rotation, const
     if (!dim_ok(D)) { fail(kErrDim, "compress: head dim must be even and at most 1024"); return; }
     if (n_levels < 1 || n_levels > 16) { fail(kErrLevels, "compress: n_levels outside [1, 16]"); return; }
     cudaStream_t st = (cudaStream_t)stream;
-    if (pq::bridge_compress_fits(N, D, input, rotation, packed_out)) {
+    // The shared-memory transpose of R costs 13 us per launch (7 at D = 64); below a few thousand vectors the kernel that
+    // streams R from L2 finishes first.
+    if ((D == 64 || D == 128) && N >= kCmpMin) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        const cudaError_t e = pq::bridge_compress_launch(input, rotation, codebook, radius_out, packed_out, N, D, n_levels, sms, st);
+        const int wave = (D == 64 ? 4 : 2) * sms;
+        cudaError_t e;
+        if (N > wave * kCmpWarps * kCmpVecs && pq::bridge_compress_fits(D, input, rotation, packed_out)) {
+            e = pq::bridge_compress_launch(input, rotation, codebook, radius_out, packed_out, N, D, n_levels, sms, st);
+        } else {
+            const int ctas = std::min(((N + kCmpVecs - 1) / kCmpVecs + kCmpWarps - 1) / kCmpWarps, wave);
+            e = D == 64 ? launch_compress<64>(ctas, input, rotation, codebook, radius_out, packed_out, N, n_levels, st)
+                        : launch_compress<128>(ctas, input, rotation, codebook, radius_out, packed_out, N, n_levels, st);
+        }
         if (e != cudaSuccess) fail(kErrCuda, cudaGetErrorString(e));
         return;
     }

@@ -39,8 +39,8 @@ def explained(direction, cb, got, want):
     return len(bad), unexplained, worst
 
 
-# n >= 4096 at head dim 64 / 128 takes the warp-per-four-vectors kernel (R transposed in shared memory), everything
-# else the CTA-per-vector kernel
+# n >= 4096 at head dim 64 / 128 takes the kernel with R transposed in shared memory, or, above a wave of its CTAs, the
+# tensor-core kernel; everything else the kernel with one vector (from 512 on four) per CTA
 @pytest.mark.parametrize("d,n_levels,n", [(128, 16, 1000), (128, 4, 37), (64, 16, 513), (64, 8, 3),
                                           (96, 16, 200), (256, 16, 65), (130, 8, 9), (128, 16, 1),
                                           (128, 16, 20_003), (64, 4, 4096), (64, 16, 70_001), (128, 8, 4097)])
@@ -281,7 +281,7 @@ def test_radius_is_as_close_to_64_bits_as_an_fp32_chain(d, n, kind):
     assert np.abs(ours.mean()) <= 2.0**-25                     # no drift of more than half a rounding
 
 
-@pytest.mark.parametrize("d,n", [(128, 4097), (64, 4097), (128, 3)])
+@pytest.mark.parametrize("d,n", [(128, 20_001), (64, 40_001), (128, 4097), (64, 4097), (128, 3)])
 def test_compress_of_infinities_nan_and_extreme_vectors(d, n):
     """What the FP32 chain gives, from 4096 vectors on too: an infinity in an input is an infinite radius, not NaN."""
     from polarquant_kv import _ext
@@ -334,3 +334,22 @@ def test_near_ties_are_settled_as_an_fp32_chain_does(d, n):
     assert differ == 0, f"{differ} of {want_packed.size} bytes"
     np.testing.assert_allclose(radius.cpu().numpy(), want_radius, rtol=5e-7)     # two roundings of the radius and its sums
     assert _ext.poll_device_errors() == 0
+
+
+# the edges of a wave of the kernel with R in shared memory, and buffers off the 16-byte grid, which stay with it
+@pytest.mark.parametrize("d,n,offset", [(128, 9472, 0), (128, 9473, 0), (64, 18_944, 0), (64, 18_945, 0), (128, 30_003, 1),
+                                        (64, 50_001, 3), (128, 4096, 2)])
+def test_compress_kernels_store_the_same_bytes(d, n, offset):
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(n + offset)
+    x, R, cb = kv_like(n, d, rng), orthogonal(d, rng), codebook_for(16, rng)
+
+    def at(a):
+        return torch.cat([torch.zeros(offset), torch.from_numpy(a).flatten()]).cuda()[offset:].view(a.shape)
+
+    radius, packed = LB.compress(at(x), at(R), at(cb))
+    want_radius, want_packed = fp32_chain(x, R, cb)
+    assert np.array_equal(packed.cpu().numpy(), want_packed)
+    np.testing.assert_allclose(radius.cpu().numpy(), want_radius, rtol=5e-7)
+    first, _ = LB.compress(at(x[:5000]), at(R), at(cb))
+    np.testing.assert_allclose(radius[:5000].cpu().numpy(), first.cpu().numpy(), rtol=5e-7)
