@@ -19,12 +19,14 @@
 //                and runs the float32 epilogue, under which the MMAs of the next tile go on;
 //   MMA warp     6 x D/16 MMAs per tile (A from tensor memory, B = the three terms of R in shared memory), 3.1 K
 //                cycles at D = 128.
-// Index search: the reference scans the levels and keeps the first of the closest.  For a codebook in ascending order
-// that is "how many decision points lie below", with the decision points found once per CTA by bisection over the
-// float32 numbers; a coordinate's bucket (1/128 wide) holds at most one of them.  Any other codebook (unsorted, levels
-// closer than 1e-5, two decision points in a bucket) is scanned level by level as the reference does.
-// Measured (16 levels, second pass included): 131 072 vectors of 128 48 us, 2^20 of them 242 (R^T in shared memory on CUDA
-// cores: 238 and 1834); of 64: 29 and 125 us (80 and 595).  One accumulator and plain bfloat16 terms: 45.5, 230, 27, 117.
+// Index search: the reference scans the levels and keeps the first of the closest.  For levels in ascending order that is
+// "how many decision points lie below", with the decision points found once per CTA by bisection over the float32 numbers;
+// a coordinate's bucket (1/128 wide) holds at most one of them.  Where two fall into one bucket, or the levels come in
+// another order or repeat themselves, a search tree of the sorted decision points takes four lookups instead of one; levels
+// closer than 1e-5, or outside (-1, 1), are scanned as the reference does.
+// Measured (16 levels, second pass included): 131 072 vectors of 128 49 us, 2^20 of them 244 (R^T in shared memory on CUDA
+// cores: 238 and 1835); of 64: 30 and 125 us (80 and 595).  One accumulator and plain bfloat16 terms: 45.5, 230, 27, 117.
+// By the search tree 2^20 vectors of 128 take 340 us and of 64 184 (level by level: 805 and 625).
 // The rotation's last bits depend on the order of its additions, and a coordinate within them of a decision point gets one
 // index or the other.  So that stored bytes do not depend on which kernel wrote them, a block with a coordinate closer
 // than kBcNear to a decision point (one in 500 at 16 levels) is put on a list and done again at the end in the order of
@@ -42,6 +44,7 @@ static __device__ unsigned int g_bridge_compress_error = 0;
 
 constexpr int kBcVecs = 128;
 constexpr float kBcNear = 6e-7f;               // ten times the typical difference between two summation orders
+constexpr uint32_t kBcScan = 0, kBcTree = 1, kBcBuckets = 2;    // how indices are found
 constexpr int kBcList = 480;                   // (vector, block) entries a CTA keeps for the second pass
 
 template <int D>
@@ -65,9 +68,9 @@ struct BridgeCompressCfg {
     static constexpr uint32_t kATerm = D / 2;                      // tensor-memory columns of one term
     static constexpr uint32_t kAcc = 2 * D;                        // leading products; the corrections D columns further
     static constexpr uint32_t kTmemCols = 4 * D;
-    // norms and largest elements [2][128][WG] each, codebook 16, decision points 16, barriers, tensor-memory slot, abort
-    // flag, fast flag, list
-    static constexpr uint32_t kSmall = 4 * kBcVecs * WG * 4 + 2 * 16 * 4 + (2 * kBoxes + 6) * 8 + 32 + kBcList * 4;
+    // norms and largest elements [2][128][WG] each, four arrays of 16 around the codebook, barriers, tensor-memory slot,
+    // flags, list
+    static constexpr uint32_t kSmall = 4 * kBcVecs * WG * 4 + 4 * 16 * 4 + (2 * kBoxes + 6) * 8 + 32 + kBcList * 4;
     static constexpr size_t smem_bytes() { return kSmallAddr + kSmall; }
 };
 
@@ -232,7 +235,9 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
     float* most_s = norm_s + 2 * kBcVecs * WG;                               // the same
     float* cb = most_s + 2 * kBcVecs * WG;
     float* thr = cb + 16;
-    uint64_t* mbar = reinterpret_cast<uint64_t*>(thr + 16);
+    float* sorted = thr + 16;
+    int* which = reinterpret_cast<int*>(sorted + 16);
+    uint64_t* mbar = reinterpret_cast<uint64_t*>(which + 16);
     // [0, NB) box landed; [NB, 2 NB) box read; then, per parity of the tile: A written; its MMAs done (A free, the
     // accumulators complete); accumulators read out
     uint64_t* box_full = mbar;
@@ -242,7 +247,7 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
     uint64_t* acc_free = a_full + 4;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(a_full + 6);
     volatile uint32_t* abort_s = tmem_slot + 1;
-    uint32_t* fast_s = tmem_slot + 2;
+    uint32_t* kind_s = tmem_slot + 2;
     float* magic_s = reinterpret_cast<float*>(tmem_slot + 3);
     int* n_list = reinterpret_cast<int*>(tmem_slot + 4);
     int* list = reinterpret_cast<int*>(tmem_slot + 8);          // vector * WG + block
@@ -260,7 +265,6 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
             mbar_init(sm_addr(acc_free + i), WORKERS);
         }
         *abort_s = 0u;
-        *fast_s = 1u;
         *n_list = 0;
     }
     if (tid < 16) cb[tid] = __ldg(p.codebook + min(tid, p.n_levels - 1));
@@ -306,61 +310,92 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
     }
     if (warp == 0) tmem_alloc(sm_addr(tmem_slot), C::kTmemCols);
     __syncthreads();
-    // decision points: the largest v for which level i is at least as close as level i + 1 (both distances rounded to
-    // float32, as the scan rounds them)
-    if (tid < p.n_levels - 1) {
-        const float a = cb[tid], b = cb[tid + 1];
-        bool good = a > -1.f && b < 1.f && b - a > 1e-5f;
-        if (good) {
-            int lo = bc_key(a), hi = bc_key(b);                // holds at a, not at b
+    if (warp == 0) {
+        // The different levels in ascending order (of equal ones the first counts), and between neighbours the decision
+        // point: the largest v for which the lower one is taken, both distances rounded to float32 as a scan rounds them;
+        // equally close, the scan keeps the one it meets first.
+        const int n_levels = p.n_levels;
+        const float v = cb[lane & 15];
+        float other[16];                                           // (entries past the last level repeat it)
+#pragma unroll
+        for (int j = 0; j < 16; ++j) other[j] = cb[j];
+        bool first = lane < n_levels;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) first = first && !(j < lane && other[j] == v);
+        const uint32_t firsts = __ballot_sync(0xffffffffu, first);
+        const int n = __popc(firsts);
+        int rank = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) rank += (firsts >> j & 1u) && other[j] < v ? 1 : 0;
+        if (first) { sorted[rank] = v; which[rank] = lane; }
+        __syncwarp();
+        bool good = lane >= n_levels || (v > -1.f && v < 1.f);     // (a NaN is not)
+        if (lane < n - 1) good = good && sorted[lane + 1] - sorted[lane] > 1e-5f;
+        const bool all_good = __all_sync(0xffffffffu, good), straight = __all_sync(0xffffffffu, !first || rank == lane) && n == n_levels;
+        float t = 3.0e38f;                                         // no coordinate reaches it
+        if (all_good && lane < n - 1) {
+            const float a = sorted[lane], b = sorted[lane + 1];
+            const bool lower_first = which[lane] < which[lane + 1];
+            int lo = bc_key(a), hi = bc_key(b);                    // the lower level is taken at a, not at b
             while (hi - lo > 1) {
                 const int mid = lo + (hi - lo) / 2;
-                const float v = bc_unkey(mid);
-                if (v - a <= b - v) lo = mid; else hi = mid;
+                const float x = bc_unkey(mid), da = x - a, db = b - x;
+                if (da < db || (lower_first && da == db)) lo = mid; else hi = mid;
             }
-            thr[tid] = bc_unkey(lo);
+            t = bc_unkey(lo);
         }
-        if (!good) *fast_s = 0u;
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // the first shift for which every decision point lies alone in its bucket and off its edges
-        const bool mine = lane < p.n_levels - 1;
-        const float t = mine ? thr[lane] : 0.f;
-        bool found = false;
-        for (int k = 0; k < 16 && !found; ++k) {
-            const float magic = 98432.f + (float)k * 0.0625f;
-            const uint32_t b = bc_bucket_bits(t, magic);
-            const uint32_t next = __shfl_down_sync(0xffffffffu, b, 1);
-            const bool bad = mine && (bc_bucket_bits(t - 4e-6f, magic) != b || bc_bucket_bits(t + 4e-6f, magic) != b ||
-                                      (lane + 1 < p.n_levels - 1 && next == b));
-            found = !__any_sync(0xffffffffu, bad);
-            if (found && lane == 0) *magic_s = magic;
+        if (lane < 16) thr[lane] = t;
+        uint32_t kind = all_good ? kBcTree : kBcScan;
+        float magic = 98432.f;
+        if (all_good && straight) {
+            // the first shift for which every decision point lies alone in its bucket and off its edges
+            const bool mine = lane < n - 1;
+            bool found = false;
+            for (int k = 0; k < 16 && !found; ++k) {
+                magic = 98432.f + (float)k * 0.0625f;
+                const float at = mine ? t : 0.f;
+                const uint32_t b = bc_bucket_bits(at, magic);
+                const uint32_t next = __shfl_down_sync(0xffffffffu, b, 1);
+                const bool bad = mine && (bc_bucket_bits(at - 4e-6f, magic) != b || bc_bucket_bits(at + 4e-6f, magic) != b ||
+                                          (lane + 1 < n - 1 && next == b));
+                found = !__any_sync(0xffffffffu, bad);
+            }
+            if (found) kind = kBcBuckets;
         }
-        if (!found && lane == 0) { *fast_s = 0u; *magic_s = 98432.f; }
+        if (lane == 0) { *kind_s = kind; *magic_s = magic; }
     }
     __syncthreads();
     const float magic1 = *magic_s;
-    // a bucket's entry: its decision point (or a number no coordinate reaches) and the count of lower ones,
-    // replicated into every index field of a word
-    for (int e = tid; e < (int)C::kTabRows * 16; e += C::THREADS) {
-        const uint32_t bits = (uint32_t)(e >> 4) << 7;
-        float t = 3.0e38f;
-        uint32_t cnt = 0;
-        for (int i = 0; i < p.n_levels - 1; ++i) {
-            const uint32_t tb = bc_bucket_bits(thr[i], magic1);
-            if (tb == bits) t = thr[i];
-            cnt += tb < bits ? 1u : 0u;
+    const uint32_t kind = *kind_s;
+    if (kind == kBcBuckets) {
+        // a bucket's entry: its decision point (or a number no coordinate reaches) and the count of lower ones,
+        // replicated into every index field of a word
+        for (int e = tid; e < (int)C::kTabRows * 16; e += C::THREADS) {
+            const uint32_t bits = (uint32_t)(e >> 4) << 7;
+            float t = 3.0e38f;
+            uint32_t cnt = 0;
+            for (int i = 0; i < p.n_levels - 1; ++i) {
+                const uint32_t tb = bc_bucket_bits(thr[i], magic1);
+                if (tb == bits) t = thr[i];
+                cnt += tb < bits ? 1u : 0u;
+            }
+            *reinterpret_cast<uint2*>(zero + C::kTabAddr + (e >> 4) * 128 + (e & 15) * 8) =
+                make_uint2(__float_as_uint(t), cnt * 0x11111111u);
         }
-        *reinterpret_cast<uint2*>(zero + C::kTabAddr + (e >> 4) * 128 + (e & 15) * 8) =
-            make_uint2(__float_as_uint(t), cnt * 0x11111111u);
+    } else if (kind == kBcTree) {
+        // row i of 32 copies: 1 to 15 the search tree (children of i: 2 i and 2 i + 1), 16 to 31 the levels' indices
+        for (int e = tid; e < 32 * 32; e += C::THREADS) {
+            const int i = e >> 5, depth = 31 - __clz(i | 1);
+            const uint32_t entry = i >= 16 ? (uint32_t)which[i - 16]
+                                           : __float_as_uint(thr[i ? ((2 * (i - (1 << depth)) + 1) << (3 - depth)) - 1 : 0]);
+            *reinterpret_cast<uint32_t*>(zero + C::kTabAddr + i * 128 + (e & 31) * 4) = entry;
+        }
     }
     fence_async_smem();                                        // B is read by the tensor core through the async proxy
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const bool fast = *fast_s != 0u;
     const int n_tiles = (p.N + kBcVecs - 1) / kBcVecs;
     const int n_my = (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     bool ok = true;
@@ -510,7 +545,7 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
 #pragma unroll
                 for (int k = 0; k < 16; ++k) v2[k] = make_float2(0.f, 0.f);
             }
-            if (fast) {
+            if (kind == kBcBuckets) {
                 const float2 c128 = make_float2(128.f, 128.f), magic = make_float2(magic1, magic1);
 #pragma unroll
                 for (int k = 0; k < 16; ++k) {
@@ -532,6 +567,27 @@ bridge_compress_kernel(const __grid_constant__ BridgeCompressParams p, const __g
                             "@p add.u32 %0, %0, %2;\n\t}\n"
                             : "+r"(pw)
                             : "f"(off), "r"(1u << sh));
+                    }
+                }
+            } else if (kind == kBcTree) {
+                const uint32_t lane4 = (uint32_t)lane * 4;
+#pragma unroll
+                for (int k = 0; k < 16; ++k) {
+                    const float2 y = bc_mul2(v2[k], rinv2);
+                    const float2 dir = bc_fma2(bc_fma2(y, negd2, v2[k]), rinv2, y);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        uint32_t row = 128u, best;
+#pragma unroll
+                        for (int step = 0; step < 4; ++step) {
+                            float t;
+                            asm volatile("ld.shared.f32 %0, [%1 + %2];\n" : "=f"(t) : "r"(row | lane4), "n"(C::kTabAddr));
+                            const float off = (e ? dir.y : dir.x) - t;                        // its sign is exact
+                            near = fminf(near, fabsf(off));
+                            row = 2u * row + (off > 0.f ? 128u : 0u);
+                        }
+                        asm volatile("ld.shared.u32 %0, [%1 + %2];\n" : "=r"(best) : "r"(row | lane4), "n"(C::kTabAddr));
+                        packed[k >> 2] |= best << (((2 * k + e) * 4) & 31);
                     }
                 }
             } else {

@@ -309,17 +309,36 @@ def test_compress_of_infinities_nan_and_extreme_vectors(d, n):
     assert _ext.poll_device_errors() == 0
 
 
-@pytest.mark.parametrize("d,n", [(128, 20_003), (64, 40_001), (128, 4096)])
-def test_near_ties_are_settled_as_an_fp32_chain_does(d, n):
+@pytest.mark.parametrize("d,n,book", [(128, 20_003, "lloyd"), (64, 40_001, "lloyd"), (128, 4096, "lloyd"), (128, 20_003, "descending"),
+                                      (64, 40_001, "descending"), (128, 20_003, "crowded"), (64, 40_001, "pairs"), (128, 20_003, "shuffled"),
+                                      (64, 40_001, "eleven"), (64, 40_001, "close"), (128, 20_003, "one")])
+def test_near_ties_are_settled_as_an_fp32_chain_does(d, n, book):
     """Half of the coordinates within 1e-6 of a decision point, so that nearly every block goes through the second pass and
     the list of a CTA overflows (512 blocks a tile at D = 128, 256 at D = 64; it holds 480): every stored byte is the
     chain's."""
     from polarquant_kv import _ext
     from polarquant_kv import llama_bridge as LB
     rng = np.random.default_rng(d + n)
-    R, cb = orthogonal(d, rng), codebook_for(16, rng)
+    from polarquant_kv.codebook import build_lloyd_max_codebook
+    R, cb = orthogonal(d, rng), build_lloyd_max_codebook(d, 4)[0].astype(np.float32)
     points = (cb[1:].astype(np.float64) + cb[:-1]) / 2
     points = points[np.abs(points) < 0.11]
+    # tables for the search tree: descending, two decision points in a bucket, levels that occur twice, any order, eleven
+    # levels; for the scan: levels closer than 1e-5; one level
+    if book == "descending":
+        cb = cb[::-1].copy()
+    elif book == "crowded":
+        cb[8] = cb[7] + np.float32(1e-3)
+    elif book == "pairs":
+        cb[1::2] = cb[0::2]
+    elif book == "shuffled":
+        cb = rng.permutation(cb)
+    elif book == "eleven":
+        cb = rng.permutation(cb[3:14])
+    elif book == "close":
+        cb[8] = cb[7] + np.float32(2e-6)
+    elif book == "one":
+        cb = cb[5:6].copy()
     direction = rng.standard_normal((n, d))
     at = rng.permuted(np.tile(np.arange(d) % 2 == 0, (n, 1)), axis=1)
     tied = rng.choice(points, (n, d)) + rng.uniform(-1e-6, 1e-6, (n, d))
