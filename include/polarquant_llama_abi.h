@@ -28,6 +28,7 @@
 #define POLARQUANT_LLAMA_ABI_H
 
 #include <stdbool.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
@@ -89,6 +90,20 @@ void polarquant_fused_attention_cuda_c(const float* q_rotated, const uint8_t* pa
                                        const float* v_radius, const float* codebook, float* output,
                                        int total_q_heads, int total_kv_heads,
                                        int S, int D, int n_levels, float scale, void* stream);
+
+/* No counterpart in the reference: the same attention with a workspace of the caller's, so that calls on several
+ * streams of a device need no order among them (a workspace serves one stream).  ws: 16-byte aligned device buffer
+ * whose first POLARQUANT_ATTENTION_COUNTER_BYTES read zero before the first call that uses it; every call leaves them
+ * zero, whatever its shape.  With fewer bytes than polarquant_fused_attention_ws_bytes_c(...) gives (on the current
+ * device; 0: none needed) the sequence is sliced less.  ws == NULL: the library's own. */
+#define POLARQUANT_ATTENTION_COUNTER_BYTES 65536
+void polarquant_fused_attention_ws_cuda_c(const float* q_rotated, const uint8_t* packed_k,
+                                          const float* k_radius, const uint8_t* packed_v,
+                                          const float* v_radius, const float* codebook, float* output,
+                                          int total_q_heads, int total_kv_heads,
+                                          int S, int D, int n_levels, float scale,
+                                          void* ws, size_t ws_bytes, void* stream);
+size_t polarquant_fused_attention_ws_bytes_c(int total_q_heads, int total_kv_heads, int S, int D);
 
 /* Replaces polarquant_inverse_rotate_cuda_c (patch 756-762 → kernel 418-435). */
 void polarquant_inverse_rotate_cuda_c(const float* input, const float* rotation, float* output,

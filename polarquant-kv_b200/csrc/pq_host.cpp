@@ -430,11 +430,13 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t n) {
     return THPVariable_Wrap(out);
 }
 
-// ------------------------------------------------------------------ scratch of pq_decode_attn
+// ------------------------------------------------------------------ scratch of the attention calls
 // One buffer per (device, stream) and, while the stream is being captured, one per capture (allocated from the graph's
 // own pool, so it lives as long as the graph does).  The counters at its start must read zero when a launch starts; a
 // launch leaves its own at zero, and with pq_decode_attn_counter_bytes() more than a call needs no record lies below
-// that, so one clear when the buffer is new serves all later calls whose counters fit there.
+// that, so one clear when the buffer is new serves all later calls whose counters fit there.  The bridge's attention lays
+// its workspace out the same way and shares the buffer.
+static_assert(POLARQUANT_ATTENTION_COUNTER_BYTES == 65536, "the counter region of both kinds of attention");
 struct Scratch {
     int device;
     void* stream;
@@ -446,7 +448,7 @@ std::deque<Scratch> g_scratch;               // bounded: the least recently made
 constexpr size_t kScratchLimit = 32;
 
 // Undefined on a CUDA error.
-at::Tensor decode_scratch(int device, void* stream, size_t* bytes_io, size_t counters) {
+at::Tensor attention_scratch(int device, void* stream, size_t* bytes_io, size_t counters) {
     const size_t kept = pq_decode_attn_counter_bytes(), need = *bytes_io += kept;
     cudaStreamCaptureStatus status;
     unsigned long long id = 0;
@@ -527,7 +529,7 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     }
     void* st = stream_of(a.device);
     size_t need = pq_decode_attn_scratch_bytes((int)a.B, (int)a.Hq, (int)a.Hkv, S, (int)a.D, 0);
-    const at::Tensor kept = decode_scratch(a.device, st, &need, ((size_t)a.B * a.Hq * 4 + 255) / 256 * 256);
+    const at::Tensor kept = attention_scratch(a.device, st, &need, ((size_t)a.B * a.Hq * 4 + 255) / 256 * 256);
     if (!kept.defined()) return raise_status(PQ_ERR_CUDA, "pq_decode_attn");
     void* scratch = kept.data_ptr();
     at::Tensor out = empty(a.q->sizes(), half ? at::kHalf : at::kFloat, a.device);
@@ -668,9 +670,9 @@ PyObject* bridge_rotate(PyObject*, PyObject* const* args, Py_ssize_t n) {
     });
     return THPVariable_Wrap(out);
 }
-// bridge_attention(q, packed_k, k_radius, packed_v, v_radius, codebook, scale) -> tensor or None
+// bridge_attention(q, packed_k, k_radius, packed_v, v_radius, codebook, scale, out) -> out, a new tensor for None, or None
 PyObject* bridge_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 7) Py_RETURN_NONE;
+    if (n != 8) Py_RETURN_NONE;
     const at::Tensor *q = f32(args[0]), *kr = f32(args[2]), *vr = f32(args[4]), *cb = f32(args[5]), *pk = tensor(args[1]), *pv = tensor(args[3]);
     if (!q || !kr || !vr || !cb || !pk || !pv || q->dim() != 2 || pk->dim() != 3) Py_RETURN_NONE;
     for (const at::Tensor* t : {pk, pv})
@@ -683,15 +685,30 @@ PyObject* bridge_attention(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const double scale = PyFloat_AsDouble(args[6]);
     if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
     const int dev = q->get_device();
-    at::Tensor out = empty(q->sizes(), at::kFloat, dev);
+    const at::Tensor* given = f32(args[7]);
+    if (args[7] != Py_None && (!given || given->sizes() != q->sizes())) Py_RETURN_NONE;
+    const at::Tensor out = given ? *given : empty(q->sizes(), at::kFloat, dev);
     void* stream = stream_of(dev);
+    const size_t need = polarquant_fused_attention_ws_bytes_c((int)hq, (int)hkv, (int)S, (int)D);
+    at::Tensor ws;
+    size_t bytes = 0;
+    if (need) {
+        bytes = need - POLARQUANT_ATTENTION_COUNTER_BYTES;
+        ws = attention_scratch(dev, stream, &bytes, ((size_t)hq * 4 + 255) / 256 * 256);
+        if (!ws.defined()) return raise_status(PQ_ERR_CUDA, "polarquant_fused_attention_ws_cuda_c");
+    }
+    void* wsp = need ? ws.data_ptr() : nullptr;
     launch([&] {
-        polarquant_fused_attention_cuda_c((const float*)q->data_ptr(), (const uint8_t*)pk->data_ptr(), (const float*)kr->data_ptr(),
-                                          (const uint8_t*)pv->data_ptr(), (const float*)vr->data_ptr(), (const float*)cb->data_ptr(),
-                                          (float*)out.data_ptr(), (int)hq, (int)hkv, (int)S, (int)D, (int)cb->numel(), (float)scale,
-                                          stream);
+        polarquant_fused_attention_ws_cuda_c((const float*)q->data_ptr(), (const uint8_t*)pk->data_ptr(), (const float*)kr->data_ptr(),
+                                             (const uint8_t*)pv->data_ptr(), (const float*)vr->data_ptr(), (const float*)cb->data_ptr(),
+                                             (float*)out.data_ptr(), (int)hq, (int)hkv, (int)S, (int)D, (int)cb->numel(), (float)scale,
+                                             wsp, bytes, stream);
         return 0;
     });
+    if (given) {
+        Py_INCREF(args[7]);
+        return args[7];
+    }
     return THPVariable_Wrap(out);
 }
 // bridge_error() -> code of the calling thread's last failed bridge call, cleared

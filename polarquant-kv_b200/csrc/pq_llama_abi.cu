@@ -435,11 +435,15 @@ struct TileScores {
 };
 
 // Workspace of the sliced launches: records of the slices and one arrival counter per (kv head,
-// query group).  Part of the module, so nothing is allocated per call; the last slice to arrive
-// puts its counter back to zero.  Launches on one device therefore have to be ordered with
-// respect to each other, which the bridge's single compute stream gives.
+// query group); the last slice to arrive puts its counter back to zero.  The one below is part of
+// the module, so that the bridge's own entry point allocates nothing: launches that use it have to be
+// ordered with respect to each other, which the bridge's single compute stream gives.  Callers with
+// several streams bring their own (polarquant_fused_attention_ws_cuda_c): counters in its first
+// kWsCounterBytes, records behind them.
 constexpr size_t kWsFloats = size_t(1) << 20;
 constexpr int kWsTickets = 4096;
+constexpr size_t kWsCounterBytes = POLARQUANT_ATTENTION_COUNTER_BYTES;
+static_assert(kWsTickets * sizeof(unsigned) <= kWsCounterBytes, "the counters fit their region");
 __device__ float g_partials[kWsFloats];
 __device__ unsigned g_tickets[kWsTickets];
 
@@ -616,8 +620,58 @@ __global__ void __launch_bounds__(kAttWarps * 32, 3) attention_kernel(const Attn
     }
 }
 
-// Device addresses of the workspace on the current device.
-bool workspace(AttnParams& p) {
+// How a call is cut: which kernel, and over how many slices (p.n_split, p.tiles_per_split).
+struct AttnPlan {
+    bool tuned;               // pq_bridge_attn.cu
+    int DPL, G, groups;       // of the general kernel (DPL, G); groups of either
+};
+AttnPlan plan_attention(AttnParams& p, bool tuned, int total_q_heads, int total_kv_heads, int sms, size_t ws_floats) {
+    AttnPlan a{};
+    a.tuned = tuned;
+    if (tuned) {
+        a.groups = pq::bridge_attention_plan(p, total_kv_heads, sms, ws_floats, kWsTickets, total_q_heads);
+        return a;
+    }
+    a.DPL = 2;
+    while (32 * a.DPL < p.D) a.DPL *= 2;
+    a.G = 8;
+    while (a.G > 1 && (p.gqa % a.G || a.G * a.DPL > 32)) a.G >>= 1;
+    a.groups = p.gqa / a.G;
+    const int n_tiles = (p.S + kTile - 1) / kTile;
+    const int base = total_kv_heads * a.groups;
+    // two CTAs per SM with at least two tiles per warp (three CTAs per SM measured slower)
+    int n_split = std::max(1, std::min((2 * sms + base - 1) / base, n_tiles / (2 * kAttWarps)));
+    int tiles_per_split = (n_tiles + n_split - 1) / n_split;
+    n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
+    if (n_split > 1) {
+        const size_t per_split = (size_t)total_q_heads * (32 * a.DPL + 2);
+        if (base > kWsTickets || per_split * 2 > ws_floats) {
+            n_split = 1;
+        } else {
+            n_split = (int)std::min<size_t>(n_split, ws_floats / per_split);
+        }
+        tiles_per_split = (n_tiles + n_split - 1) / n_split;
+        n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
+    }
+    p.n_split = n_split;
+    p.tiles_per_split = tiles_per_split;
+    return a;
+}
+
+int device_sms() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
+// The records and counters of a sliced call: the caller's workspace, or the module's own on the current device.
+bool workspace(AttnParams& p, void* given) {
+    if (given) {
+        p.tickets = static_cast<unsigned*>(given);
+        p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(given) + kWsCounterBytes);
+        return true;
+    }
     if (cudaGetSymbolAddress((void**)&p.partials, g_partials) == cudaSuccess &&
         cudaGetSymbolAddress((void**)&p.tickets, g_tickets) == cudaSuccess)
         return true;
@@ -706,9 +760,7 @@ void polarquant_compress_cuda_c(const float* input, const float* rotation, const
     // The shared-memory transpose of R costs 13 us per launch (7 at D = 64); below a few thousand vectors the kernel that
     // streams R from L2 finishes first.
     if ((D == 64 || D == 128) && N >= kCmpMin) {
-        int dev = 0, sms = 148;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        const int sms = device_sms();
         const int wave = (D == 64 ? 4 : 2) * sms;
         cudaError_t e;
         if (N > wave * kCmpWarps * kCmpVecs && pq::bridge_compress_fits(D, input, rotation, packed_out)) {
@@ -728,11 +780,25 @@ void polarquant_compress_cuda_c(const float* input, const float* rotation, const
     launched();
 }
 
-void polarquant_fused_attention_cuda_c(const float* q_rotated, const uint8_t* packed_k,
-                                       const float* k_radius, const uint8_t* packed_v,
-                                       const float* v_radius, const float* codebook, float* output,
-                                       int total_q_heads, int total_kv_heads,
-                                       int S, int D, int n_levels, float scale, void* stream) {
+size_t polarquant_fused_attention_ws_bytes_c(int total_q_heads, int total_kv_heads, int S, int D) {
+    if (total_q_heads <= 0 || total_kv_heads <= 0 || total_q_heads % total_kv_heads || S <= 0 || !dim_ok(D)) return 0;
+    size_t floats = 0;
+    for (const bool tuned : {false, true}) {                   // which of the two depends on the buffers' alignment
+        if (tuned && !pq::bridge_attention_fits(D, nullptr, nullptr)) continue;
+        AttnParams p{};
+        p.gqa = total_q_heads / total_kv_heads; p.S = S; p.D = D;
+        const AttnPlan a = plan_attention(p, tuned, total_q_heads, total_kv_heads, device_sms(), kWsFloats);
+        if (p.n_split > 1) floats = std::max(floats, (size_t)p.n_split * total_q_heads * ((tuned ? D : 32 * a.DPL) + 2));
+    }
+    return floats ? kWsCounterBytes + floats * sizeof(float) : 0;
+}
+
+void polarquant_fused_attention_ws_cuda_c(const float* q_rotated, const uint8_t* packed_k,
+                                          const float* k_radius, const uint8_t* packed_v,
+                                          const float* v_radius, const float* codebook, float* output,
+                                          int total_q_heads, int total_kv_heads,
+                                          int S, int D, int n_levels, float scale,
+                                          void* ws, size_t ws_bytes, void* stream) {
     if (total_q_heads <= 0 || S <= 0 || D <= 0) return;
     if (!q_rotated || !packed_k || !k_radius || !packed_v || !v_radius || !codebook || !output) {
         fail(kErrNull, "attention: NULL pointer");
@@ -745,62 +811,43 @@ void polarquant_fused_attention_cuda_c(const float* q_rotated, const uint8_t* pa
         return;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const int gqa = total_q_heads / total_kv_heads;
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-
     AttnParams p{};
     p.q = q_rotated; p.pk = packed_k; p.kr = k_radius; p.pv = packed_v; p.vr = v_radius;
     p.codebook = codebook; p.out = output;
-    p.gqa = gqa; p.S = S; p.D = D; p.n_levels = n_levels; p.scale = scale;
+    p.gqa = total_q_heads / total_kv_heads; p.S = S; p.D = D; p.n_levels = n_levels; p.scale = scale;
 
     // Head dims 64 and 128 on 16-byte boundaries (the bridge's own buffers are) have a kernel of their own.  It masks
     // indices with n_levels - 1 like the general one, so other table sizes than powers of two behave alike.
-    if (pq::bridge_attention_fits(D, packed_k, packed_v) && (reinterpret_cast<uintptr_t>(q_rotated) & 7) == 0) {
-        const int groups = pq::bridge_attention_plan(p, total_kv_heads, sms, kWsFloats, kWsTickets, total_q_heads);
-        if (p.n_split > 1 && !workspace(p)) return;
-        const cudaError_t e = pq::bridge_attention_launch(p, total_kv_heads, groups, st);
+    const bool tuned = pq::bridge_attention_fits(D, packed_k, packed_v) && (reinterpret_cast<uintptr_t>(q_rotated) & 7) == 0;
+    size_t floats = kWsFloats;
+    if (ws) floats = ws_bytes <= kWsCounterBytes ? 0 : std::min(kWsFloats, (ws_bytes - kWsCounterBytes) / sizeof(float));
+    const AttnPlan a = plan_attention(p, tuned, total_q_heads, total_kv_heads, device_sms(), floats);
+    if (p.n_split > 1 && !workspace(p, ws)) return;
+    if (tuned) {
+        const cudaError_t e = pq::bridge_attention_launch(p, total_kv_heads, a.groups, st);
         if (e != cudaSuccess) fail(kErrCuda, cudaGetErrorString(e));
         return;
     }
-
-    int DPL = 2;
-    while (32 * DPL < D) DPL *= 2;
-    int G = 8;
-    while (G > 1 && (gqa % G || G * DPL > 32)) G >>= 1;
-    const int groups = gqa / G;
-    const int n_tiles = (S + kTile - 1) / kTile;
-    const int base = total_kv_heads * groups;
-    // two CTAs per SM with at least two tiles per warp (three CTAs per SM measured slower)
-    int n_split = std::max(1, std::min((2 * sms + base - 1) / base, n_tiles / (2 * kAttWarps)));
-    int tiles_per_split = (n_tiles + n_split - 1) / n_split;
-    n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
-    const int bpl = DPL / 2;
+    const int bpl = a.DPL / 2;
     p.vector_loads = ((D / 2) % bpl == 0) && (reinterpret_cast<uintptr_t>(packed_k) % bpl == 0) &&
                      (reinterpret_cast<uintptr_t>(packed_v) % bpl == 0);
+    const dim3 grid(p.n_split, a.groups, total_kv_heads);
+    switch (a.DPL) {
+        case 2:  dispatch_group<2>(a.G, p, grid, st); break;
+        case 4:  dispatch_group<4>(a.G, p, grid, st); break;
+        case 8:  dispatch_group<8>(a.G, p, grid, st); break;
+        case 16: dispatch_group<16>(a.G, p, grid, st); break;
+        default: dispatch_group<32>(a.G, p, grid, st); break;
+    }
+}
 
-    if (n_split > 1) {
-        const size_t per_split = (size_t)total_q_heads * (32 * DPL + 2);
-        if (base > kWsTickets || per_split * 2 > kWsFloats) {
-            n_split = 1;
-        } else {
-            n_split = (int)std::min<size_t>(n_split, kWsFloats / per_split);
-        }
-        tiles_per_split = (n_tiles + n_split - 1) / n_split;
-        n_split = (n_tiles + tiles_per_split - 1) / tiles_per_split;
-        if (n_split > 1 && !workspace(p)) return;
-    }
-    p.n_split = n_split;
-    p.tiles_per_split = tiles_per_split;
-    const dim3 grid(n_split, groups, total_kv_heads);
-    switch (DPL) {
-        case 2:  dispatch_group<2>(G, p, grid, st); break;
-        case 4:  dispatch_group<4>(G, p, grid, st); break;
-        case 8:  dispatch_group<8>(G, p, grid, st); break;
-        case 16: dispatch_group<16>(G, p, grid, st); break;
-        default: dispatch_group<32>(G, p, grid, st); break;
-    }
+void polarquant_fused_attention_cuda_c(const float* q_rotated, const uint8_t* packed_k,
+                                       const float* k_radius, const uint8_t* packed_v,
+                                       const float* v_radius, const float* codebook, float* output,
+                                       int total_q_heads, int total_kv_heads,
+                                       int S, int D, int n_levels, float scale, void* stream) {
+    polarquant_fused_attention_ws_cuda_c(q_rotated, packed_k, k_radius, packed_v, v_radius, codebook, output, total_q_heads,
+                                         total_kv_heads, S, D, n_levels, scale, nullptr, 0, stream);
 }
 
 struct polarquant_state* polarquant_init_c(int head_dim, int n_kv_heads, int n_q_heads,

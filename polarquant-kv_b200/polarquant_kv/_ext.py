@@ -67,6 +67,10 @@ SIGNATURES = {
     "polarquant_rotate_query_cuda_c": (None, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "polarquant_fused_attention_cuda_c": (None, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                                  c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p]),
+    "polarquant_fused_attention_ws_cuda_c": (None, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                                    c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                                    c_size_t, c_void_p]),
+    "polarquant_fused_attention_ws_bytes_c": (c_size_t, [c_int, c_int, c_int, c_int]),
     "polarquant_inverse_rotate_cuda_c": (None, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "polarquant_last_error_c": (c_int, []),
 }

@@ -88,11 +88,10 @@ def fused_attention(q_rot: torch.Tensor, packed_k: torch.Tensor, k_radius: torch
                     packed_v: torch.Tensor, v_radius: torch.Tensor, codebook: torch.Tensor,
                     scale: float, out: torch.Tensor | None = None) -> torch.Tensor:
     """q_rot [Hq, D]; packed_* uint8 [Hkv, S, D/2]; *_radius [Hkv, S] -> [Hq, D] (rotated space)."""
-    if out is None:
-        done = _ext.host().bridge_attention(q_rot, packed_k, k_radius, packed_v, v_radius, codebook, scale)
-        if done is not None:
-            _raise_on_error("polarquant_fused_attention_cuda_c")
-            return done
+    done = _ext.host().bridge_attention(q_rot, packed_k, k_radius, packed_v, v_radius, codebook, scale, out)
+    if done is not None:
+        _raise_on_error("polarquant_fused_attention_ws_cuda_c")
+        return done
     q_rot, k_radius, v_radius, codebook = (_f32(q_rot, "q_rot"), _f32(k_radius, "k_radius"),
                                            _f32(v_radius, "v_radius"), _f32(codebook, "codebook"))
     if packed_k.dtype != torch.uint8 or packed_v.dtype != torch.uint8:
@@ -106,11 +105,14 @@ def fused_attention(q_rot: torch.Tensor, packed_k: torch.Tensor, k_radius: torch
     if out is None:
         out = torch.empty_like(q_rot)
     with torch.cuda.device(q_rot.device):
-        _ext.lib().polarquant_fused_attention_cuda_c(
+        # a workspace of this call's own: the library's serves one stream
+        need = _ext.lib().polarquant_fused_attention_ws_bytes_c(hq, hkv, s, d)
+        ws = torch.zeros(need, dtype=torch.uint8, device=q_rot.device) if need else None
+        _ext.lib().polarquant_fused_attention_ws_cuda_c(
             q_rot.data_ptr(), packed_k.data_ptr(), k_radius.data_ptr(), packed_v.data_ptr(), v_radius.data_ptr(),
             codebook.data_ptr(), out.data_ptr(), hq, hkv, s, d, codebook.numel(), ctypes.c_float(scale),
-            _stream(q_rot))
-    _raise_on_error("polarquant_fused_attention_cuda_c")
+            ws.data_ptr() if ws is not None else None, need, _stream(q_rot))
+    _raise_on_error("polarquant_fused_attention_ws_cuda_c")
     return out
 
 

@@ -372,3 +372,64 @@ def test_compress_kernels_store_the_same_bytes(d, n, offset):
     np.testing.assert_allclose(radius.cpu().numpy(), want_radius, rtol=5e-7)
     first, _ = LB.compress(at(x[:5000]), at(R), at(cb))
     np.testing.assert_allclose(radius[:5000].cpu().numpy(), first.cpu().numpy(), rtol=5e-7)
+
+
+@pytest.mark.parametrize("d", [128, 96])
+def test_attention_on_several_streams_and_in_graphs(d):
+    """Sliced calls of different shapes in flight on three streams at once, two of them replayed from CUDA graphs, give what
+    they give one after another: no workspace is shared between them."""
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(d)
+    cb = torch.from_numpy(codebook_for(16, rng)).cuda()
+    calls, want = [], []
+    for hq, hkv, s in ((32, 8, 20_000), (8, 1, 9001), (16, 2, 33_333)):
+        pk, kr = (torch.from_numpy(a).cuda() for a in random_cache(hkv, s, d, 16, rng))
+        pv, vr = (torch.from_numpy(a).cuda() for a in random_cache(hkv, s, d, 16, rng))
+        q = torch.from_numpy(rng.standard_normal((hq, d)).astype(np.float32)).cuda()
+        calls.append((q, pk, kr, pv, vr, cb, 0.1))
+        want.append(LB.fused_attention(*calls[-1]).clone())
+        given = torch.empty_like(q)
+        assert LB.fused_attention(*calls[-1], out=given) is given and torch.equal(given, want[-1])
+    streams = [torch.cuda.Stream() for _ in calls]
+    graphs, outs = [], []
+    torch.cuda.synchronize()
+    for call, stream in list(zip(calls, streams))[:2]:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            outs.append([LB.fused_attention(*call) for _ in range(2)])
+        graphs.append(graph)
+    results = []
+    for _ in range(30):
+        for graph, stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        with torch.cuda.stream(streams[2]):
+            results.append(LB.fused_attention(*calls[2]))
+    torch.cuda.synchronize()
+    assert all(torch.equal(r, want[2]) for r in results)
+    for got, ref in zip(outs, want):
+        assert all(torch.equal(o, ref) for o in got)
+
+
+def test_attention_with_a_small_workspace_of_the_callers():
+    """Fewer bytes than a call could use: it is sliced less; the counters are zero again afterwards."""
+    import ctypes
+
+    from polarquant_kv import _ext
+    lib, rng, hq, hkv, s, d = _ext.lib(), np.random.default_rng(1), 8, 2, 9000, 128
+    cb = codebook_for(16, rng)
+    pk, kr = random_cache(hkv, s, d, 16, rng)
+    pv, vr = random_cache(hkv, s, d, 16, rng)
+    q = rng.standard_normal((hq, d)).astype(np.float32)
+    want = LO.fused_attention(q, pk, kr, pv, vr, cb, 16, 0.1)
+    t = [torch.from_numpy(a).cuda() for a in (q, pk, kr, pv, vr, cb)]
+    need = lib.polarquant_fused_attention_ws_bytes_c(hq, hkv, s, d)
+    assert need > 65536 and lib.polarquant_fused_attention_ws_bytes_c(hq, hkv, 20, d) == 0
+    for size in (need, 65536 + 3 * hq * (d + 2) * 4, 65536, 16):
+        ws = torch.cat([torch.zeros(65536, dtype=torch.uint8), torch.full((need,), 255, dtype=torch.uint8)]).cuda()
+        out = torch.empty(hq, d, device="cuda")
+        lib.polarquant_fused_attention_ws_cuda_c(*[x.data_ptr() for x in t], out.data_ptr(), hq, hkv, s, d, 16, ctypes.c_float(0.1),
+                                                 ws.data_ptr(), size, torch.cuda.current_stream().cuda_stream)
+        assert lib.polarquant_last_error_c() == 0
+        assert np.abs(out.cpu().numpy() - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
+        assert not ws[:65536].any() and (ws[max(size, 65536):] == 255).all()
