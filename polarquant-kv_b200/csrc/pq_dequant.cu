@@ -81,6 +81,11 @@ __device__ __forceinline__ uint32_t dq_lds_u16(uint32_t a) {
     asm volatile("{ .reg .u16 t; ld.shared.u16 t, [%1]; cvt.u32.u16 %0, t; }\n" : "=r"(v) : "r"(a));
     return v;
 }
+// float16 bits: the larger of m and |x|, NaN if either is
+__device__ __forceinline__ unsigned short dq_max_abs(unsigned short m, uint32_t x) {
+    asm("{ .reg .f16 a; abs.f16 a, %1; max.NaN.f16 %0, %0, a; }\n" : "+h"(m) : "h"((unsigned short)x));
+    return m;
+}
 __device__ __forceinline__ uint32_t dq_lds_u32(uint32_t a) {
     uint32_t v;
     asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(a));
@@ -252,7 +257,8 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
             const int slot = i % RING;
             ok = mbar_wait(sm_addr(in_full + slot), (uint32_t)(i / RING) & 1u, abort_s) && ok;
             const uint32_t vec = ring + slot * C::kSlot + row * VB, blk = vec + wg * BB;
-            uint32_t words[BITS], dbits, dmax = 0u;
+            uint32_t words[BITS], dbits;
+            unsigned short dmax = 0;
             {
                 uint32_t w[BITS + 1];
                 const uint32_t a = blk & ~3u;
@@ -269,12 +275,12 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
                 }
             }
 #pragma unroll
-            for (int j = 0; j < NBLK; ++j) dmax = max(dmax, dq_lds_u16(vec + j * BB));      // radii are not negative
+            for (int j = 0; j < NBLK; ++j) dmax = dq_max_abs(dmax, dq_lds_u16(vec + j * BB));
             mbar_arrive(sm_addr(in_free + slot));
             // largest radius -> [1, 2)
-            const uint32_t be = __float_as_uint(__half2float(__ushort_as_half((unsigned short)dmax))) >> 23;
+            const uint32_t be = __float_as_uint(__half2float(__ushort_as_half(dmax))) >> 23;
             const bool normal = be > 0 && be < 255;
-            scale = normal ? __uint_as_float(be << 23) : 1.0f;
+            scale = normal ? __uint_as_float(be << 23) : be ? __int_as_float(0x7FFFFFFF) : 1.0f;      // NaN: no finite vector
             const float ds = __half2float(__ushort_as_half((unsigned short)dbits)) * (normal ? __uint_as_float((254u - be) << 23) : 1.0f);
             const __half2 d2 = __float2half2_rn(ds);               // exact but for radii 2^-14 below the largest
             uint32_t hi[16], lo[16];
@@ -314,7 +320,7 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
             tc_fence_before();
             mbar_arrive(sm_addr(acc_free + b));
             const float s = sc * (1.0f / (kDqCbScale * 4096.f));
-            const float2 s2 = make_float2(s, s);
+            float2 s2 = make_float2(s, s);
             const int64_t v0 = first(i) + 32 * q;
             // 32 vectors: rows of 128 bytes, 16-byte chunks swizzled as the tensor map says
             if (p.out_is_fp16) {
@@ -322,6 +328,11 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
                 // rows a TMA unit stores: 98 us for 2^20 vectors)
                 const uint32_t piece = C::kOutAddr + b * (C::kOutBytes / 2) + (uint32_t)((wg >> 1) * kDqVecs + 32 * q) * 128;
                 const bool leader = !(wg & 1) && lane == 0;
+                if (s != s) {                                  // clamped like a value below the range
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) v[k] = make_float2(-65504.f, -65504.f);
+                    s2 = make_float2(1.f, 1.f);
+                }
                 const uint32_t bar = 1u + (uint32_t)(q * (D / 64) + (wg >> 1));
                 // (the pair's barrier of the tile in between orders this wait before the partner's writes too)
 #pragma unroll
