@@ -122,7 +122,7 @@ class KVCacheManager:
         B, Hq, Sq, D = query.shape
         if self.config.enable_compression and Sq == 1:
             done = _ext.host().decode(query, self._compressed_keys, self._compressed_values, self.plan, None, None,
-                                      self.config.enable_qjl, False, seq_len_tensor)
+                                      bool(self.config.enable_qjl), False, seq_len_tensor)
             if done is not None:
                 return done
         if seq_len_tensor is not None:

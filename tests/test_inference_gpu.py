@@ -357,3 +357,17 @@ def test_reference_named_layers_and_gpu_package_functions():
             cos = torch.nn.functional.cosine_similarity(a.flatten(), b.flatten(), dim=0)
             assert a.shape == (3, chunk.shape[1], 97) and float(cos) > 0.99, float(cos)
         assert cm_c[0].seq_len == 20 and cm_c[1].compression_ratio > 3.0
+
+
+def test_cache_manager_takes_any_true_value_for_its_sketch_switch():
+    """``enable_qjl=1`` is the same manager as ``enable_qjl=True``: the sketch enters the scores of a single-token step."""
+    from polarquant_kv.inference import KVCacheManager, PolarQuantConfig
+    dev = _cuda()
+    gen = torch.Generator().manual_seed(2)
+    k, v, q = (torch.randn(shape, generator=gen).half().to(dev) for shape in ((1, 2, 40, 64), (1, 2, 40, 64), (1, 8, 1, 64)))
+    out = {}
+    for switch in (True, 1, False):
+        m = KVCacheManager(PolarQuantConfig(n_bits=2, enable_qjl=switch, jl_dim=32), 64, 1, 2, 64, dev)
+        m.append(k, v)
+        out[repr(switch)] = m.attend(q)
+    assert torch.equal(out["1"], out["True"]) and not torch.equal(out["1"], out["False"])
