@@ -275,7 +275,10 @@ bool read_cache(PyObject* o, Cache* c) {
     if (!ok || (c->n_bits != 2 && c->n_bits != 4) || !g_tables[c->n_bits].set) return false;
     c->rows_b = c->blocks.size(0);
     c->rows_h = c->blocks.size(1);
+    // the stated capacity is the tensor's; anything else goes through the Python function's checks
     c->cap = c->blocks.size(2);
+    int64_t stated;
+    if (!attr_int(o, s_cap, &stated) || stated != c->cap) return false;
     c->contiguous = c->blocks.is_contiguous();
     c->sketch = false;
     PyObject *s = attr(o, s_signs), *m = attr(o, s_norms);

@@ -84,7 +84,7 @@ def decode_attention(query: torch.Tensor, ck: CompressedKV, cv: CompressedKV, pl
         raise ValueError(f"q heads {Hq} not a multiple of kv heads {Hkv}")
     dev = query.device
     kb, vb = ck.blocks, cv.blocks
-    S, cap = ck.seq_len, ck.max_seq_len
+    S = ck.seq_len
     bits_t, norms_t = ck.qjl_signs, ck.residual_norms
     if seq_range is not None:
         lo, hi = seq_range
@@ -166,7 +166,8 @@ class PreparedDecode:
         if seq_len_tensor is not None:
             if seq_len_tensor.dtype != torch.int64 or seq_len_tensor.numel() != 1 or seq_len_tensor.device != self.dev:
                 raise ValueError("seq_len_tensor must be a one-element int64 tensor on the query's device")
-        need = lib.pq_decode_attn_scratch_bytes(B, Hq, Hkv, ck.max_seq_len, D, max(0, n_splits))
+        cap = ck.blocks.shape[2]
+        need = lib.pq_decode_attn_scratch_bytes(B, Hq, Hkv, cap, D, max(0, n_splits))
         self.scratch = torch.zeros(max(need, 256), dtype=torch.uint8, device=self.dev)   # private: no sharing
         cbk, cbv = tables(ck.n_bits)[0], tables(cv.n_bits)[0]
         use_qjl = bool(enable_qjl and plan.jl is not None and ck.qjl_signs is not None)
@@ -175,7 +176,7 @@ class PreparedDecode:
         ptr = lambda t: t.data_ptr() if t is not None else 0                    # noqa: E731
         self._tables = (cbk, cbv)
         self._prepared = _ext.host().prepare(
-            query.data_ptr(), ck.blocks.data_ptr(), cv.blocks.data_ptr(), B, Hq, Hkv, ck.max_seq_len, D, ck.n_bits, cv.n_bits,
+            query.data_ptr(), ck.blocks.data_ptr(), cv.blocks.data_ptr(), B, Hq, Hkv, cap, D, ck.n_bits, cv.n_bits,
             ctypes.addressof(cbk), ctypes.addressof(cbv), plan.rot.data_ptr(), ptr(plan.jl) if use_qjl else 0,
             plan.jl_dim if use_qjl else 0, ck.qjl_signs.data_ptr() if use_qjl else 0,
             ck.residual_norms.data_ptr() if use_qjl else 0, 0 if partial else self.out.data_ptr(),
@@ -261,7 +262,7 @@ def prefill_attention(query: torch.Tensor, ck: CompressedKV, cv: CompressedKV, p
         use_workspace = Sq * (Hq // Hkv) > 128 and 0 < need <= PREFILL_WORKSPACE_LIMIT
     ws = _prefill_workspace(dev, need) if (use_workspace and need > 0) else None
     st = lib.pq_prefill_attn(
-        q.data_ptr(), kb.data_ptr(), vb.data_ptr(), B, Hq, Hkv, Sq, ck.seq_len, ck.max_seq_len, D,
+        q.data_ptr(), kb.data_ptr(), vb.data_ptr(), B, Hq, Hkv, Sq, ck.seq_len, kb.shape[2], D,
         ck.n_bits, cv.n_bits, cbk, cbv, plan.rot.data_ptr(),
         ctypes.c_float(scale if scale is not None else 1.0 / math.sqrt(D)), 1 if causal else 0,
         out.data_ptr(), 1 if out_dtype == torch.float16 else 0,
