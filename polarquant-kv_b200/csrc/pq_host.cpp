@@ -356,7 +356,7 @@ PyObject* compress(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_RETURN_NONE;
     const int dev = x->get_device();
     const Plan* plan = plan_for(args[1], args[4], dev);
-    if (!plan || plan->head_dim != x->size(3)) Py_RETURN_NONE;
+    if (!plan || plan->head_dim != x->size(3) || (plan->head_dim != 64 && plan->head_dim != 128)) Py_RETURN_NONE;
     const int64_t B = x->size(0), H = x->size(1), S = x->size(2), D = x->size(3);
     if (args[5] != Py_None) {
         Cache c;
