@@ -67,14 +67,16 @@ bool as_int(PyObject* o, int64_t* v) {
     return true;
 }
 
-const Plan* plan_of(PyObject* o) {
-    if (!g_plan_type || !PyObject_TypeCheck(o, (PyTypeObject*)g_plan_type)) return nullptr;
+// A copy of a plan object's constants: a launch runs without the GIL, and another thread may change the object meanwhile.
+bool plan_of(PyObject* o, Plan* out) {
+    if (!g_plan_type || !PyObject_TypeCheck(o, (PyTypeObject*)g_plan_type)) return false;
     PyObject* c = attr(o, s_native);
-    if (!c) return nullptr;
+    if (!c) return false;
     const Plan* p = (const Plan*)PyCapsule_GetPointer(c, kPlanCapsule);
-    Py_DECREF(c);                   // the plan object keeps it
-    if (!p) PyErr_Clear();
-    return p;
+    if (p) *out = *p;
+    else PyErr_Clear();
+    Py_DECREF(c);
+    return p != nullptr;
 }
 
 // ------------------------------------------------------------------ plans by the matrices of a call
@@ -321,13 +323,12 @@ int launch_compress(const at::Tensor& x, int64_t rows, int64_t tokens, int64_t c
     });
 }
 
-const Plan* plan_for(PyObject* R, PyObject* P, int device) {
-    const Plan* p = plan_of(R);
-    if (!p) {
+bool plan_for(PyObject* R, PyObject* P, int device, Plan* out) {
+    if (!plan_of(R, out)) {
         PyObject* known = known_plan(R, P, device);
-        p = known ? plan_of(known) : nullptr;
+        if (!known || !plan_of(known, out)) return false;
     }
-    return p && p->device == device ? p : nullptr;
+    return out->device == device;
 }
 
 // What an append into `c` needs beyond read_cache: the input's rows and width, room, and the plan's sketch.
@@ -355,27 +356,28 @@ PyObject* compress(PyObject*, PyObject* const* args, Py_ssize_t n) {
         !g_tables[bits].set || x->dim() != 4 || x->numel() == 0 || !half_contiguous(*x))
         Py_RETURN_NONE;
     const int dev = x->get_device();
-    const Plan* plan = plan_for(args[1], args[4], dev);
-    if (!plan || plan->head_dim != x->size(3) || (plan->head_dim != 64 && plan->head_dim != 128)) Py_RETURN_NONE;
+    Plan plan;
+    if (!plan_for(args[1], args[4], dev, &plan) || plan.head_dim != x->size(3) || (plan.head_dim != 64 && plan.head_dim != 128))
+        Py_RETURN_NONE;
     const int64_t B = x->size(0), H = x->size(1), S = x->size(2), D = x->size(3);
     if (args[5] != Py_None) {
         Cache c;
         Position pos;
         if (!read_cache(args[5], &c) || c.n_bits != bits || !read_position(args[6], dev, &pos) ||
-            !append_fits(*x, c, *plan, pos))
+            !append_fits(*x, c, plan, pos))
             Py_RETURN_NONE;
-        const int st = launch_compress(*x, B * H, S, c.cap, pos, *plan, (int)bits, c.blocks, c.signs, c.norms, plan->jl_dim > 0);
+        const int st = launch_compress(*x, B * H, S, c.cap, pos, plan, (int)bits, c.blocks, c.signs, c.norms, plan.jl_dim > 0);
         if (st) return raise_status(st, "pq_compress_rows");
         if (!pos.dev && pos.host + S > c.seq && !store_seq(args[5], pos.host + S)) return nullptr;
         Py_INCREF(args[5]);
         return args[5];
     }
     at::Tensor blocks = empty({B, H, S, D / 32, 2 + 4 * bits}, at::kByte, dev), signs, norms;
-    if (plan->jl_dim) {
-        signs = empty({B, H, S, plan->jl_dim / 8}, at::kByte, dev);
+    if (plan.jl_dim) {
+        signs = empty({B, H, S, plan.jl_dim / 8}, at::kByte, dev);
         norms = empty({B, H, S}, at::kHalf, dev);
     }
-    const int st = launch_compress(*x, B * H, S, S, Position(), *plan, (int)bits, blocks, signs, norms, plan->jl_dim > 0);
+    const int st = launch_compress(*x, B * H, S, S, Position(), plan, (int)bits, blocks, signs, norms, plan.jl_dim > 0);
     if (st) return raise_status(st, "pq_compress_rows");
     auto wrap = [](const at::Tensor& t) -> PyObject* {
         if (t.defined()) return THPVariable_Wrap(t);
@@ -395,16 +397,16 @@ PyObject* append(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const at::Tensor *k = n == 7 ? tensor(args[0]) : nullptr, *v = n == 7 ? tensor(args[1]) : nullptr;
     if (!k || !v || !half_contiguous(*k) || !half_contiguous(*v) || k->get_device() != v->get_device()) Py_RETURN_NONE;
     const int dev = k->get_device();
-    const Plan *pk = plan_of(args[4]), *pv = plan_of(args[5]);
+    Plan pk, pv;
     Cache ck, cv;
     Position pos;
-    if (!pk || !pv || pk->device != dev || pv->device != dev || pv->jl_dim || !read_position(args[6], dev, &pos) ||
-        !read_cache(args[2], &ck) || !read_cache(args[3], &cv) || !append_fits(*k, ck, *pk, pos) ||
-        !append_fits(*v, cv, *pv, pos) || k->size(2) != v->size(2))
+    if (!plan_of(args[4], &pk) || !plan_of(args[5], &pv) || pk.device != dev || pv.device != dev || pv.jl_dim || !read_position(args[6], dev, &pos) ||
+        !read_cache(args[2], &ck) || !read_cache(args[3], &cv) || !append_fits(*k, ck, pk, pos) ||
+        !append_fits(*v, cv, pv, pos) || k->size(2) != v->size(2))
         Py_RETURN_NONE;
     const int64_t rows = ck.rows_b * ck.rows_h, S = k->size(2);
-    int st = launch_compress(*k, rows, S, ck.cap, pos, *pk, (int)ck.n_bits, ck.blocks, ck.signs, ck.norms, pk->jl_dim > 0);
-    if (!st) st = launch_compress(*v, rows, S, cv.cap, pos, *pv, (int)cv.n_bits, cv.blocks, cv.signs, cv.norms, false);
+    int st = launch_compress(*k, rows, S, ck.cap, pos, pk, (int)ck.n_bits, ck.blocks, ck.signs, ck.norms, pk.jl_dim > 0);
+    if (!st) st = launch_compress(*v, rows, S, cv.cap, pos, pv, (int)cv.n_bits, cv.blocks, cv.signs, cv.norms, false);
     if (st) return raise_status(st, "pq_compress_rows");
     if (!pos.dev) {
         const int64_t end = pos.host + S;
@@ -420,14 +422,14 @@ PyObject* decompress(PyObject*, PyObject* const* args, Py_ssize_t n) {
     if (n != 3 || !read_cache(args[0], &c) || c.seq == 0 || c.seq != c.cap || c.blocks.numel() == 0 || !c.contiguous)
         Py_RETURN_NONE;
     const int dev = c.blocks.get_device();
-    const Plan* plan = plan_for(args[1], Py_None, dev);
-    if (!plan || plan->head_dim != c.dim || dev != c10::cuda::current_device()) Py_RETURN_NONE;
+    Plan plan;
+    if (!plan_for(args[1], Py_None, dev, &plan) || plan.head_dim != c.dim || dev != c10::cuda::current_device()) Py_RETURN_NONE;
     const bool half = args[2] == Py_True;
     at::Tensor out = empty({c.rows_b, c.rows_h, c.seq, c.dim}, half ? at::kHalf : at::kFloat, dev);
     void* stream = stream_of(dev);
     const int st = launch([&] {
         return pq_dequant(c.blocks.data_ptr(), c.rows_b * c.rows_h * c.seq, (int)c.dim, (int)c.n_bits,
-                          g_tables[c.n_bits].codebook, plan->rot, out.data_ptr(), half, stream);
+                          g_tables[c.n_bits].codebook, plan.rot, out.data_ptr(), half, stream);
     });
     if (st) return raise_status(st, "pq_dequant");
     return THPVariable_Wrap(out);
@@ -483,7 +485,7 @@ at::Tensor attention_scratch(int device, void* stream, size_t* bytes_io, size_t 
 struct Attend {                               // what decode and prefill read from their common arguments
     const at::Tensor* q;
     Cache ck, cv;
-    const Plan* plan;
+    Plan plan;
     int device;
     float scale;
     int64_t B, Hq, Hkv, Sq, D;
@@ -505,8 +507,7 @@ bool read_attend(PyObject* const* args, Attend* a) {
         k.rows_b != a->B || v.rows_b != a->B || v.rows_h != a->Hkv || k.cap != v.cap || v.seq < k.seq || k.dim != a->D ||
         v.dim != a->D || a->Hkv == 0 || a->Hq % a->Hkv)
         return false;
-    a->plan = plan_for(args[3], args[4], a->device);
-    if (!a->plan || a->plan->head_dim != a->D) return false;
+    if (!plan_for(args[3], args[4], a->device, &a->plan) || a->plan.head_dim != a->D) return false;
     if (args[5] == Py_None) {
         a->scale = (float)(1.0 / std::sqrt((double)a->D));
     } else {
@@ -521,8 +522,8 @@ bool read_attend(PyObject* const* args, Attend* a) {
 PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     Attend a;
     if (n != 9 || !read_attend(args, &a) || a.Sq != 1) Py_RETURN_NONE;
-    const bool qjl = args[6] == Py_True && a.plan->jl && a.ck.sketch, half = args[7] == Py_True;
-    if (qjl && (!a.ck.signs.is_contiguous() || !a.ck.norms.is_contiguous() || a.ck.signs.size(-1) != a.plan->jl_dim / 8))
+    const bool qjl = args[6] == Py_True && a.plan.jl && a.ck.sketch, half = args[7] == Py_True;
+    if (qjl && (!a.ck.signs.is_contiguous() || !a.ck.norms.is_contiguous() || a.ck.signs.size(-1) != a.plan.jl_dim / 8))
         Py_RETURN_NONE;
     Position len;
     int64_t S = a.ck.seq;
@@ -537,16 +538,16 @@ PyObject* decode(PyObject*, PyObject* const* args, Py_ssize_t n) {
     void* scratch = kept.data_ptr();
     at::Tensor out = empty(a.q->sizes(), half ? at::kHalf : at::kFloat, a.device);
     const float *cbk = g_tables[a.ck.n_bits].codebook, *cbv = g_tables[a.cv.n_bits].codebook;
-    const float* jl = qjl ? a.plan->jl : nullptr;
+    const float* jl = qjl ? a.plan.jl : nullptr;
     const void *bits = qjl ? a.ck.signs.data_ptr() : nullptr, *norms = qjl ? a.ck.norms.data_ptr() : nullptr;
-    const int m = qjl ? a.plan->jl_dim : 0;
+    const int m = qjl ? a.plan.jl_dim : 0;
     const int status = launch([&] {
         return len.dev ? pq_decode_attn_dynamic(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
                                          (int)a.Hkv, S, len.dev, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits, cbk,
-                                         cbv, a.plan->rot, a.scale, jl, m, bits, norms, out.data_ptr(), half, nullptr, 0,
+                                         cbv, a.plan.rot, a.scale, jl, m, bits, norms, out.data_ptr(), half, nullptr, 0,
                                          scratch, need, st)
                        : pq_decode_attn(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
-                                 (int)a.Hkv, S, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits, cbk, cbv, a.plan->rot,
+                                 (int)a.Hkv, S, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits, cbk, cbv, a.plan.rot,
                                  a.scale, jl, m, bits, norms, out.data_ptr(), half, nullptr, 0, scratch, need, st);
     });
     if (status) return raise_status(status, "pq_decode_attn");
@@ -570,7 +571,7 @@ PyObject* prefill(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const int status = launch([&] {
         return pq_prefill_attn_split(a.q->data_ptr(), a.ck.blocks.data_ptr(), a.cv.blocks.data_ptr(), (int)a.B, (int)a.Hq,
                                      (int)a.Hkv, (int)a.Sq, a.ck.seq, a.ck.cap, (int)a.D, (int)a.ck.n_bits, (int)a.cv.n_bits,
-                                     g_tables[a.ck.n_bits].codebook, g_tables[a.cv.n_bits].codebook, a.plan->rot, a.scale,
+                                     g_tables[a.ck.n_bits].codebook, g_tables[a.cv.n_bits].codebook, a.plan.rot, a.scale,
                                      args[6] == Py_True, out.data_ptr(), half, wsp, wsp ? need : 0, pp, parts_need, stream);
     });
     if (status) return raise_status(status, "pq_prefill_attn");

@@ -89,12 +89,17 @@ class DevicePlan:
 
     def _attach(self):
         """The native handle (raw addresses of this object's tensors)."""
-        self._native = None
+        self.device = self.rot.device                        # with its index
         if self.device.type == "cuda":
-            self.device = self.rot.device                    # with its index
             ptr = lambda t: t.data_ptr() if t is not None else 0                # noqa: E731
             self._native = _ext.host().plan_handle(self.head_dim, self.device.index, ptr(self.rot), ptr(self.rot_split),
                                                    ptr(self.jl), ptr(self.jl_split), self.jl_dim)
+
+    # a plan whose constants are replaced goes on without the handle, through the Python functions that read them
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name in ("head_dim", "device", "rot", "rot_split", "jl", "jl_split", "jl_dim"):
+            object.__setattr__(self, "_native", None)
 
     # a copied or unpickled plan has tensors, and so a handle, of its own
     def __getstate__(self):
