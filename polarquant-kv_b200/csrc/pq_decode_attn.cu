@@ -240,36 +240,38 @@ struct DecodeCfg {
     static constexpr int kSignTab = QJL ? 16 * 16 * 8 : 0;
     // head of a warp's ring: kStages mbarriers (32 bytes) + the tile's value radii, compacted
     static constexpr int kRingHead = 32 + kTileTok * NBLK * 2;
-    __host__ __device__ static constexpr int stage_bits(int jl_dim) { return QJL ? kTileTok * (jl_dim / 8) : 0; }
-    __host__ __device__ static constexpr int stage_bytes_total(int jl_dim) {
+    __host__ __device__ static int stage_bits(int jl_dim) { return QJL ? kTileTok * (jl_dim / 8) : 0; }
+    __host__ __device__ static int stage_bytes_total(int jl_dim) {
         return kStageK + kStageV + stage_bits(jl_dim) + kStageN;
     }
-    __host__ __device__ static constexpr int qjl_frag_bytes(int jl_dim) { return QJL ? (jl_dim / 16) * 32 * 16 : 0; }
+    __host__ __device__ static int qjl_frag_bytes(int jl_dim) { return QJL ? (jl_dim / 16) * 32 * 16 : 0; }
     // Shared-memory plan (byte addresses in the shared window):
     //   [base, 64K)        the teams' query buffers, split codebooks, the rings of the first n_low warps
     //   [64K, 128K)        centroid table (its address is baked into the lookups)
     //   [128K, ...)        sign table, JL query fragments, the rings of the remaining warps
     // A ring = head (see kRingHead) + kStages tile stages; at the end of a work item the warp parks
     // its (m, l, o) record over the stages.
-    __host__ __device__ static constexpr int ring_bytes(int jl_dim) {
+    __host__ __device__ static int ring_bytes(int jl_dim) {
         const int r = kStages * stage_bytes_total(jl_dim), rec = HPC * (D + 2) * 4;
         return kRingHead + (((r > rec ? r : rec) + 15) & ~15);
     }
-    __host__ __device__ static constexpr int low_fixed(int jl_dim) {
+    __host__ __device__ static int low_fixed(int jl_dim) {
         // per team: rotated queries [kQRows][D], final-stage buffer [HPC][D] (+ the projected query with QJL)
         return ((kTeams * ((kQRows + HPC) * D + (QJL ? HPC * jl_dim : 0)) * 4 + 2 * 16 * 4) + 15) & ~15;
     }
     // rings that fit below the table when the dynamic window starts at or below 8 KB
-    __host__ __device__ static constexpr int n_low(int jl_dim) {
+    __host__ __device__ static int n_low(int jl_dim) {
         int n = (65536 - 8192 - low_fixed(jl_dim)) / ring_bytes(jl_dim);
         return n > NWARPS ? NWARPS : n;
     }
-    __host__ __device__ static constexpr size_t smem_bytes(int jl_dim) {
+    __host__ __device__ static size_t smem_bytes(int jl_dim) {
         size_t high = kSignTab + qjl_frag_bytes(jl_dim) + (size_t)(NWARPS - n_low(jl_dim)) * ring_bytes(jl_dim);
         return 2 * 65536 + high + 16;
     }
-    // the most a call of this instance asks for, whatever the width of its sketch
-    static constexpr size_t smem_most() {
+    // the most a call of this instance asks for, whatever the width of its sketch (at most 224 528 bytes, at 128 projections).
+    // (Not constexpr, nor the functions above: that alone changed the tile loop's code, 136.6 -> 139.7 us on the 32 x 8 x
+    // 8192-token workload.)
+    static size_t smem_most() {
         size_t most = smem_bytes(0);
         for (int m = 16; QJL && m <= 128; m += 16) most = smem_bytes(m) > most ? smem_bytes(m) : most;
         return most;
@@ -1236,10 +1238,10 @@ template <int D, int KBITS, int VBITS, int NH, bool QJL>
 static int launch_decode(const DecodeParams& p, int rows, cudaStream_t st) {
     using C = DecodeCfg<D, KBITS, VBITS, NH, QJL>;
     const size_t smem = C::smem_bytes(p.jl_dim);
-    static_assert(C::smem_most() <= 227 * 1024, "every sketch width fits a CTA's shared memory");
     auto kern = pq_decode_attn_kernel<D, KBITS, VBITS, NH, QJL>;
+    static const size_t most = C::smem_most();
     static std::atomic<uint64_t> allowed{0};
-    if (allow_shared(kern, C::smem_most(), allowed) != cudaSuccess) return PQ_ERR_CUDA;
+    if (allow_shared(kern, most, allowed) != cudaSuccess) return PQ_ERR_CUDA;
     int sms = device_sms();
     if (sms <= 0) sms = 148;
     static_assert(C::kTeams <= kMaxTeams, "balanced_plan bounds the segments of a row with kMaxTeams");
