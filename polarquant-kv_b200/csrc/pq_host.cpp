@@ -1,5 +1,5 @@
-// Host path of the Python package in native code: polarquant_kv/_host.so, a CPython extension over torch's C++ API and
-// the C ABI of libpolarquant_b200.so.
+// Host path of the Python package in native code: the module polarquant_kv._host, a CPython extension over torch's C++ API
+// and the C ABI of libpolarquant_b200.so.
 //
 // A call of the package used to spend 15 to 40 us in Python and ctypes (argument checks, plan look-up, allocation, the
 // conversion of twenty-odd arguments) around kernels of 4 to 15 us.  The functions here do the same for the ordinary

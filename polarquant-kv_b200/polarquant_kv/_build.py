@@ -13,11 +13,13 @@ import shutil
 import subprocess
 import sys
 
+from polarquant_kv._ext import host_file_name
+
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(os.path.dirname(PKG_DIR), "csrc")
 INCLUDE = os.path.join(os.path.dirname(os.path.dirname(PKG_DIR)), "include")
 LIB_PATH = os.path.join(PKG_DIR, "libpolarquant_b200.so")
-HOST_PATH = os.path.join(PKG_DIR, "_host.so")         # native host path of the Python package (CPython extension)
+HOST_PATH = os.path.join(PKG_DIR, host_file_name())    # native host path of the Python package (CPython extension)
 HOST_SOURCE = os.path.join(CSRC, "pq_host.cpp")
 
 SOURCES = ["pq_compress.cu", "pq_dequant.cu", "pq_decode_attn.cu", "pq_prefill_attn.cu", "pq_lse_merge.cu", "pq_qjl.cu",
@@ -46,7 +48,7 @@ def _stale() -> bool:
 
 
 def _start_host_build(force: bool):
-    """The compiler process for _host.so, or None when it is up to date.  Plain C++ (no device code): torch's headers,
+    """The compiler process for the host module, or None when it is up to date.  Plain C++ (no device code): torch's headers,
     the C ABI's headers; libraries are found beside the module and in torch's own lib folder."""
     headers = [h for h in HEADERS if os.path.isabs(h)]
     if not force and not _older(HOST_PATH, [HOST_SOURCE] + headers):
@@ -71,7 +73,7 @@ def _finish_host_build(proc) -> None:
     if proc is not None:
         out, _ = proc.communicate()
         if proc.returncode != 0:
-            raise RuntimeError(f"building _host.so failed:\n{out}")
+            raise RuntimeError(f"building the host module failed:\n{out}")
 
 
 def build_library(force: bool = False, verbose: bool = False) -> str:

@@ -8,7 +8,10 @@ boundary is a plain C ABI loaded with ctypes, so any host language can bind it.
 from __future__ import annotations
 
 import ctypes
+import importlib.metadata
+import importlib.util
 import os
+import sysconfig
 
 _LIB_NAME = "libpolarquant_b200.so"
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), _LIB_NAME)
@@ -109,16 +112,26 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+def host_file_name() -> str:
+    """File of the native host module.  It is built against one Python and one torch, whose C++ classes it uses, so both are
+    part of the name: after an upgrade of either the module of the other one is not loaded, and counts as not built."""
+    return f"_host-torch{importlib.metadata.version('torch')}{sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
 def host():
-    """The native host path (csrc/pq_host.cpp), set up on first use; raises when it has not been built."""
+    """The native host path (csrc/pq_host.cpp), set up on first use; raises when it has not been built for this Python and
+    this torch."""
     global _host
     if _host is None:
         lib()                                        # its own, clearer error comes first
         import torch  # noqa: F401                   # before the module: its C++ types have to be torch's own
+        path = os.path.join(os.path.dirname(_LIB_PATH), host_file_name())
         try:
-            from . import _host as module
+            spec = importlib.util.spec_from_file_location(f"{__package__}._host", path)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
         except ImportError as exc:
-            raise ImportError(f"polarquant_kv._host cannot be loaded ({exc}): build it with "
+            raise ImportError(f"{os.path.basename(path)} cannot be loaded ({exc}): build it with "
                               "`python -m polarquant_kv._build`; there is no fallback path") from exc
         from .rotation import DevicePlan
         from .types import CompressedKV

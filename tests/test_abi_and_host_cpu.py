@@ -461,3 +461,22 @@ def test_kept_plans_are_found_by_what_the_matrices_hold():
         assert host.plan_get(other, 0, None) is None
     square.shape = (128, 32)
     assert host.plan_get(square, 0, None) is None
+
+
+def test_host_module_belongs_to_one_python_and_one_torch(monkeypatch):
+    """Another torch than the module was built for: not loaded, but reported as not built, and the build makes a new one."""
+    import importlib.metadata
+    import sysconfig
+
+    import torch
+
+    from polarquant_kv import _build, _ext
+    name = _ext.host_file_name()
+    assert torch.__version__ in name and name.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert os.path.basename(_ext.host().__file__) == name == os.path.basename(_build.HOST_PATH)
+    assert not _build._older(_build.HOST_PATH, [])
+    monkeypatch.setattr(importlib.metadata, "version", lambda package: "99.0")
+    monkeypatch.setattr(_ext, "_host", None)
+    with pytest.raises(ImportError, match="torch99.0.*polarquant_kv._build"):
+        _ext.host()
+    assert _build._older(os.path.join(_build.PKG_DIR, _ext.host_file_name()), [])
