@@ -987,12 +987,18 @@ extern "C" size_t pq_prefill_attn_workspace_bytes(int batch, int kv_heads, int64
 // waves of rows and its records' bytes.  8 sequences x 8 KV heads, 5 positions x 4 heads against 3001 tokens: one CTA per KV
 // row 147 us, two 88 us.
 static int prefill_splits(int rows, int64_t n_rows, int64_t seq_len) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        sms <= 0) {
+        cudaGetLastError();
+        return 1;                                                  // no device: nothing to spread over
+    }
     const int64_t tiles = (seq_len + pq::kPfTok - 1) / pq::kPfTok, out_rows = rows * n_rows;
     const int64_t ctas = rows * ((n_rows + pq::kPfRows - 1) / pq::kPfRows);
-    if (ctas <= 0 || ctas >= 148) return 1;
+    if (ctas <= 0 || ctas >= sms) return 1;
     int64_t best = 1, best_cost = 0;
     for (int64_t s = 1; s <= 64 && s <= tiles; ++s) {
-        const int64_t cost = (ctas * s + 147) / 148 * (6 + (tiles + s - 1) / s) + (s > 1 ? 3 + out_rows / 700 + s * out_rows / 8000 : 0);
+        const int64_t cost = (ctas * s + sms - 1) / sms * (6 + (tiles + s - 1) / s) + (s > 1 ? 3 + out_rows / 700 + s * out_rows / 8000 : 0);
         if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
     }
     return (int)best;
