@@ -459,6 +459,10 @@ at::Tensor attention_scratch(int device, void* stream, size_t* bytes_io, size_t 
     unsigned long long id = 0;
     if (cudaStreamGetCaptureInfo((cudaStream_t)stream, &status, &id) != cudaSuccess) return {};
     if (status != cudaStreamCaptureStatusActive) id = 0;
+    // A stream is in one capture at a time: buffers of its earlier ones go back to their graphs' pools, which keep them for
+    // as long as the graphs live and no longer.
+    for (auto it = g_scratch.begin(); it != g_scratch.end();)
+        it = it->device == device && it->stream == stream && it->capture && it->capture != id ? g_scratch.erase(it) : it + 1;
     Scratch* s = nullptr;
     for (Scratch& e : g_scratch)
         if (e.device == device && e.stream == stream && e.capture == id) s = &e;

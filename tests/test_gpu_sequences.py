@@ -118,3 +118,44 @@ def test_prefill_and_compress_calls_of_many_shapes_share_one_stream():
                 assert torch.equal(ck.blocks, fk) and torch.equal(cv.blocks, fv)
                 assert float((outs[0] - fo).abs().max()) <= 1e-5 * max(1.0, float(fo.abs().max()))
                 assert float((dec - fd).abs().max()) <= 1e-5 * max(1.0, float(fd.abs().max()))
+
+
+def test_scratch_of_captured_calls_goes_with_the_graph():
+    """Decode recorded in one graph after another: the memory of graphs that are gone is given back, graphs that are kept
+    replay correctly."""
+    import gc
+
+    from polarquant_kv import attention, quantizer
+    from polarquant_kv.rotation import device_plan, generate_rotation_matrix
+    dev = torch.device("cuda:0")
+    plan = device_plan(generate_rotation_matrix(128, seed=1), dev)
+    c = quantizer.compress(torch.randn(4, 8, 4096, 128, device=dev).half(), plan)
+    q = torch.randn(4, 32, 128, device=dev).half()
+    want = attention.decode_attention(q, c, c, plan)
+
+    def record():
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            out = attention.decode_attention(q, c, c, plan)
+        return graph, out
+
+    def reserved():
+        gc.collect()
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        return torch.cuda.memory_reserved()
+
+    kept = record()
+    first = reserved()
+    for _ in range(6):
+        graph, out = record()
+        graph.replay()
+        del graph, out
+    last = record()
+    grown = reserved() - first                    # the last graph's own pool: a segment of 20 MB and one of 2
+    del last
+    assert grown <= 48 << 20, f"{grown >> 20} MB beyond the first graph's"
+    for _ in range(2):
+        kept[1].zero_()
+        kept[0].replay()
+        assert torch.equal(kept[1], want)
