@@ -433,3 +433,25 @@ def test_attention_with_a_small_workspace_of_the_callers():
         assert lib.polarquant_last_error_c() == 0
         assert np.abs(out.cpu().numpy() - want).max() <= 1e-4 * max(1.0, np.abs(want).max())
         assert not ws[:65536].any() and (ws[max(size, 65536):] == 255).all()
+
+
+@pytest.mark.parametrize("d,s,scale", [(64, 9000, 0.125), (128, 9000, 0.088388346), (64, 700, 0.125), (128, 5000, -0.05), (64, 300, 0.0)])
+def test_fused_attention_error_of_large_scores(d, s, scale):
+    """Scores of tens: their float32 dot products and one rounding by the radius (a few 2^-24 of a score of 30 or so) are what
+    the weights inherit.  The bounds are twice the errors measured.  A negative scale and zero are scales too."""
+    from polarquant_kv import _ext
+    from polarquant_kv import llama_bridge as LB
+    from polarquant_kv.codebook import build_lloyd_max_codebook
+    hq, hkv = 32, 8
+    rng = np.random.default_rng(d + s)
+    cb = build_lloyd_max_codebook(d, 4)[0].astype(np.float32)
+    pk, pv = (random_cache(hkv, s, d, 16, rng)[0] for _ in range(2))
+    kr, vr = ((30 * (1 + 0.2 * rng.standard_normal((hkv, s)))).astype(np.float32) for _ in range(2))
+    q = rng.standard_normal((hq, d)).astype(np.float32)
+    dev = lambda a: torch.from_numpy(a).cuda()
+    out = LB.fused_attention(dev(q), dev(pk), dev(kr), dev(pv), dev(vr), dev(cb), scale).cpu().numpy()
+    want = LO.fused_attention(q, pk, kr, pv, vr, cb, 16, float(np.float32(scale)))
+    off = np.linalg.norm(out - want, axis=1) / np.linalg.norm(want, axis=1)
+    print(f"attention D{d} s={s} scale {scale}: relative error per head, geometric mean {np.exp(np.log(off).mean()):.2e}")
+    assert np.exp(np.log(off).mean()) <= 1e-6 and off.max() <= 5e-6
+    assert _ext.poll_device_errors() == 0
