@@ -14,8 +14,8 @@
 //     from shared memory;
 //   * the running maximum moves only when a score exceeds it by 16 (log2): weights stay below 2^16 in float32;
 //   * packed rows of a 32-token tile are contiguous and arrive by bulk copy, one tile ahead.
-// Measured (D = 128, 8 kv heads): 32 query heads x 32768 tokens 26.4 us (general kernel 63.5), x 65536 43.6 (110.8); 64
-// query heads x 65536 77 (158); 8 query heads x 65536 28 (82) = 2.5 TB/s of the stored bytes.
+// Measured (D = 128, 8 kv heads, input sets in turn): 32 query heads x 32768 tokens 29 us (general kernel 68), x 65536 47
+// (119); 64 query heads x 65536 80 (164); 8 query heads x 65536 31 (89) = 2.3 TB/s of the stored bytes.
 // One CTA of 16 or 12 warps per SM; a (kv head, query group) is cut into slices over CTAs, merged by the last to arrive.
 #include "pq_bridge.cuh"
 #include "pq_tcgen05.cuh"

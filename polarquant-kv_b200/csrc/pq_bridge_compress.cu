@@ -28,7 +28,8 @@
 // cores: 238 and 1835); of 64: 30 and 125 us (80 and 595).  One accumulator and plain bfloat16 terms: 45.5, 230, 27, 117.
 // By the search tree 2^20 vectors of 128 take 340 us and of 64 184 (level by level: 805 and 625).
 // The rotation's last bits depend on the order of its additions, and a coordinate within them of a decision point gets one
-// index or the other.  So that stored bytes do not depend on which kernel wrote them, a block with a coordinate closer
+// index or the other.  So that stored bytes do not depend on which of the two kernels for many vectors wrote them (the one
+// below 4096 vectors adds in another order, and may differ there), a block with a coordinate closer
 // than kBcNear to a decision point (one in 500 at 16 levels) is put on a list and done again at the end in the order of
 // an FP32 chain, k ascending per output, with R copied over the boxes, which are free by then.  The same goes for whole vectors whose radius is not a number,
 // infinite, or so small that its squares are subnormal: there too the stored values are the chain's.

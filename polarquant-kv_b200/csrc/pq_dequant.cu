@@ -20,8 +20,11 @@
 //   MMA warp      3 x D/16 MMAs per tile (1.5 K cycles at D = 128; HBM needs 1.8 K for the float16 output);
 //   the same worker warps, one tile behind, read their vector's 32 accumulator columns, scale, and send the results off
 //                 through swizzled shared memory by TMA (stores straight from the threads, one vector's 32 bytes per lane,
-//                 took two thirds of the load-store pipe: 136 us against the figure below).
+//                 took two thirds of the load-store pipe: 136 us against 118).
 // A power of two per vector keeps the largest radius in [1, 2) inside, so tiny vectors keep their precision.
+// Error against 64 bits: 4e-8 of a vector's largest component rms, 7e-7 at most over 400 000 vectors (8e-8 and 2e-6 with
+// float32 products split afterwards and the cross term in an accumulator of its own).
+// Measured: 2^20 vectors of 128 at 4 bits to float16 118 us (181 with operands staged through shared memory).
 // All waits are bounded (a lost completion sets an error flag instead of hanging).
 #include <atomic>
 
@@ -325,7 +328,7 @@ __global__ void __launch_bounds__(DequantCfg<D>::kThreads, 1) pq_dequant_kernel(
             // 32 vectors: rows of 128 bytes, 16-byte chunks swizzled as the tensor map says
             if (p.out_is_fp16) {
                 // 64 dims = rows of 128 bytes, shared by two warps (boxes of 64-byte rows are limited by the number of
-                // rows a TMA unit stores: 98 us for 2^20 vectors)
+                // rows a TMA unit stores)
                 const uint32_t piece = C::kOutAddr + b * (C::kOutBytes / 2) + (uint32_t)((wg >> 1) * kDqVecs + 32 * q) * 128;
                 const bool leader = !(wg & 1) && lane == 0;
                 if (s != s) {                                  // clamped like a value below the range
