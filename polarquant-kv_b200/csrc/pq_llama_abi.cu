@@ -53,6 +53,13 @@ bool launched() {
 // rows · Rᵀ and rows · R
 // ---------------------------------------------------------------------------------------------
 
+int device_sms() {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms;
+}
+
 // These run over a few dozen rows per call and are bound by the latency of R's loads from L2, so what counts is how many
 // of them a warp has in flight: a warp takes kRowBatch rows of R at once (a row per loop step, as a first version did,
 // is one round trip after another: 6 us instead of 2.5 for a token's eight vectors of 128).
@@ -102,30 +109,44 @@ __global__ void __launch_bounds__(512) rotate_rows_kernel(const float* in, const
     }
 }
 
-// out[n][j] = sum_k in[n][k] * R[k][j]: kInvCols columns at a time, k dealt to kInvParts threads of a column.  (One CTA
-// per row, which reads its input before it writes: `out` may be `in`.)
-constexpr int kInvCols = 128, kInvParts = 8;
-__global__ void __launch_bounds__(kInvCols * kInvParts) inverse_rotate_rows_kernel(const float* in, const float* __restrict__ R,
-                                                                                  float* out, int D) {
+// out[n][j] = sum_k in[n][k] * R[k][j] for the COLS columns from blockIdx.y * COLS, k dealt to PARTS threads of a column.
+// Latency again: a thread's loads of R are independent, and with 1024 threads a row takes one to eight round trips.
+template <int COLS, int PARTS>
+__global__ void __launch_bounds__(COLS * PARTS) inverse_rotate_split_kernel(const float* __restrict__ in, const float* __restrict__ R,
+                                                                            float* __restrict__ out, int D) {
     __shared__ float xs[kMaxDim];
-    __shared__ float part[kInvParts][kInvCols];
-    const int n = blockIdx.x, c = threadIdx.x, y = threadIdx.y;
-    for (int k = y * kInvCols + c; k < D; k += kInvCols * kInvParts) xs[k] = in[(size_t)n * D + k];
+    __shared__ float part[PARTS][COLS];
+    const int n = blockIdx.x, c = threadIdx.x, y = threadIdx.y, j = blockIdx.y * COLS + c;
+    for (int k = y * COLS + c; k < D; k += COLS * PARTS) xs[k] = in[(size_t)n * D + k];
     __syncthreads();
-    for (int j0 = 0; j0 < D; j0 += kInvCols) {
-        const int j = min(j0 + c, D - 1);
-        float s = 0.0f;
+    const float* col = R + min(j, D - 1);
+    float s = 0.0f;
 #pragma unroll 16
-        for (int k = y; k < D; k += kInvParts) s = fmaf(xs[k], __ldg(R + (size_t)k * D + j), s);
-        part[y][c] = s;
-        __syncthreads();
-        if (y == 0 && j0 + c < D) {
-            float t = 0.0f;
+    for (int k = y; k < D; k += PARTS) s = fmaf(xs[k], __ldg(col + (size_t)k * D), s);
+    part[y][c] = s;
+    __syncthreads();
+    if (y == 0 && j < D) {
+        float t = 0.0f;
 #pragma unroll
-            for (int u = 0; u < kInvParts; ++u) t += part[u][c];
-            out[(size_t)n * D + j] = t;
-        }
-        __syncthreads();
+        for (int u = 0; u < PARTS; ++u) t += part[u][c];
+        out[(size_t)n * D + j] = t;
+    }
+}
+
+// The same by one CTA per row, a thread per column, which reads its input before it writes: `output` may be `input`.  Also
+// the faster one for many rows, whose CTAs fill the card by themselves.  Split / one CTA per row: 32 rows of 128 2.9 / 4.8 us,
+// of 1024 16 / 108; 200 rows of 256 7.9 / 8.7, of 1024 80 / 111; 512 rows of 128 6.2 / 5.2, of 256 16 / 9.8, of 1024 201 / 125.
+__global__ void __launch_bounds__(256) inverse_rotate_rows_kernel(const float* __restrict__ in,
+                                                                  const float* __restrict__ R,
+                                                                  float* __restrict__ out, int D) {
+    __shared__ float xs[kMaxDim];
+    const int n = blockIdx.x;
+    for (int k = threadIdx.x; k < D; k += blockDim.x) xs[k] = in[(size_t)n * D + k];
+    __syncthreads();
+    for (int j = threadIdx.x; j < D; j += blockDim.x) {
+        float s = 0.0f;
+        for (int k = 0; k < D; ++k) s = fmaf(xs[k], R[(size_t)k * D + j], s);
+        out[(size_t)n * D + j] = s;
     }
 }
 
@@ -658,13 +679,6 @@ AttnPlan plan_attention(AttnParams& p, bool tuned, int total_q_heads, int total_
     return a;
 }
 
-int device_sms() {
-    int dev = 0, sms = 148;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return sms;
-}
-
 // The records and counters of a sliced call: the caller's workspace, or the module's own on the current device.
 bool workspace(AttnParams& p, void* given) {
     if (given) {
@@ -745,7 +759,14 @@ void polarquant_inverse_rotate_cuda_c(const float* input, const float* rotation,
     if (total_q_heads <= 0 || D <= 0) return;
     if (!input || !rotation || !output) { fail(kErrNull, "inverse_rotate: NULL pointer"); return; }
     if (D > kMaxDim) { fail(kErrDim, "inverse_rotate: head dim above 1024"); return; }
-    inverse_rotate_rows_kernel<<<total_q_heads, dim3(kInvCols, kInvParts), 0, (cudaStream_t)stream>>>(input, rotation, output, D);
+    cudaStream_t st = (cudaStream_t)stream;
+    const int blocks = (D + 127) / 128;
+    if (input == output || total_q_heads > device_sms() * 4 / 3)
+        inverse_rotate_rows_kernel<<<total_q_heads, 256, 0, st>>>(input, rotation, output, D);
+    else if (D <= 64)
+        inverse_rotate_split_kernel<64, 16><<<total_q_heads, dim3(64, 16), 0, st>>>(input, rotation, output, D);
+    else
+        inverse_rotate_split_kernel<128, 8><<<dim3(total_q_heads, blocks), dim3(128, 8), 0, st>>>(input, rotation, output, D);
     launched();
 }
 

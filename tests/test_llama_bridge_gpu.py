@@ -455,3 +455,20 @@ def test_fused_attention_error_of_large_scores(d, s, scale):
     print(f"attention D{d} s={s} scale {scale}: relative error per head, geometric mean {np.exp(np.log(off).mean()):.2e}")
     assert np.exp(np.log(off).mean()) <= 1e-6 and off.max() <= 5e-6
     assert _ext.poll_device_errors() == 0
+
+
+# both kernels of the inverse rotation: few rows (columns and k dealt out), many rows, and in place
+@pytest.mark.parametrize("d", [2, 64, 66, 128, 130, 256, 1000])
+@pytest.mark.parametrize("rows", [1, 197, 198, 400])
+def test_inverse_rotation_kernels_vs_oracle(d, rows):
+    from polarquant_kv import _ext
+    from polarquant_kv import llama_bridge as LB
+    rng = np.random.default_rng(d + rows)
+    y, R = rng.standard_normal((rows, d)).astype(np.float32), orthogonal(d, rng)
+    yt, Rt = torch.from_numpy(y).cuda(), torch.from_numpy(R).cuda()
+    want = LO.inverse_rotate(y, R)
+    # chains of up to 1000 float32 multiply-adds of terms below 4 |R|: a few 2^-24 of the row's norm
+    bound = 4e-7 * np.linalg.norm(y, axis=1).max()
+    assert np.abs(LB.inverse_rotate(yt, Rt).cpu().numpy() - want).max() <= bound
+    _ext.lib().polarquant_inverse_rotate_cuda_c(yt.data_ptr(), Rt.data_ptr(), yt.data_ptr(), rows, d, torch.cuda.current_stream().cuda_stream)
+    assert np.abs(yt.cpu().numpy() - want).max() <= bound and _ext.lib().polarquant_last_error_c() == 0
