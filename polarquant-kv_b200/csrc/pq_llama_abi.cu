@@ -2,7 +2,7 @@
 // decoded lines 695-763) for sm_100a: the per-vector-radius codec with nibble-packed
 // indices, as kernels laid out for a 148-SM part instead of one CTA per vector / per head.
 //
-//   compress   below 4096 vectors, and for other head dims than 64 and 128, a CTA takes one vector (four from 512 vectors
+//   compress   below 4096 vectors, and for other head dims than 64 and 128, a CTA takes one vector (four from 768 vectors
 //              on) and streams R from L2; above that an FP32 kernel with R^T in shared memory, and for buffers on 16-byte
 //              boundaries and more than a wave of its CTAs pq_bridge_compress.cu (tensor cores).
 //   attention  head dims 64 and 128: pq_bridge_attn.cu.  Other head dims: CTAs own (kv head, query group, slice of S); a
@@ -265,9 +265,10 @@ cudaError_t launch_compress(int ctas, const float* input, const float* R, const 
     return cudaGetLastError();
 }
 
-// Any even head dim up to 1024: V vectors per CTA.  One, so that a token's few vectors spread over the SMs; four once there
-// are more vectors than SMs can hold, because every CTA streams the whole of R from L2 (1024 vectors of 128: 12.3 us at
-// one, where L2 delivers 64 KB per vector).
+// Any even head dim up to 1024: V vectors per CTA.  One, so that a token's few vectors spread over the SMs; four once L2,
+// which every CTA streams the whole of R from, is what counts (one / four: 511 vectors of 128 7.8 / 9.3 us, of 256 15 / 22, of
+// 1024 125 / 254; 1000 of 128 14 / 11.6, of 256 30 / 25, of 1024 245 / 254).
+constexpr int kCmpFour = 768;
 constexpr int kSmallWarps = 16;
 template <int V>
 __global__ void __launch_bounds__(kSmallWarps * 32) compress_any_dim_kernel(const float* __restrict__ input,
@@ -794,7 +795,7 @@ void polarquant_compress_cuda_c(const float* input, const float* rotation, const
         if (e != cudaSuccess) fail(kErrCuda, cudaGetErrorString(e));
         return;
     }
-    if (N < 512)
+    if (N < kCmpFour)
         compress_any_dim_kernel<1><<<N, kSmallWarps * 32, 0, st>>>(input, rotation, codebook, radius_out, packed_out, N, D, n_levels);
     else
         compress_any_dim_kernel<4><<<(N + 3) / 4, kSmallWarps * 32, 0, st>>>(input, rotation, codebook, radius_out, packed_out, N, D, n_levels);

@@ -40,8 +40,8 @@ def explained(direction, cb, got, want):
 
 
 # n >= 4096 at head dim 64 / 128 takes the kernel with R transposed in shared memory, or, above a wave of its CTAs, the
-# tensor-core kernel; everything else the kernel with one vector (from 512 on four) per CTA
-@pytest.mark.parametrize("d,n_levels,n", [(128, 16, 1000), (128, 4, 37), (64, 16, 513), (64, 8, 3),
+# tensor-core kernel; everything else the kernel with one vector (from 768 on four) per CTA
+@pytest.mark.parametrize("d,n_levels,n", [(128, 16, 767), (256, 16, 768), (64, 4, 769), (128, 16, 1000), (128, 4, 37), (64, 16, 513), (64, 8, 3),
                                           (96, 16, 200), (256, 16, 65), (130, 8, 9), (128, 16, 1),
                                           (128, 16, 20_003), (64, 4, 4096), (64, 16, 70_001), (128, 8, 4097)])
 def test_compress_vs_oracle(d, n_levels, n):
