@@ -417,12 +417,17 @@ bool bridge_attention_fits(int D, const void* packed_k, const void* packed_v) {
 }
 
 // Query heads per CTA: the smallest of 1, 2, 4, 8 that holds the group (a missing head costs its multiply-adds, a
-// second CTA over the same keys would repeat the lookups too); groups above eight heads are cut into eights.
-static int bridge_heads(int gqa) { return gqa >= 5 ? 8 : gqa >= 3 ? 4 : gqa; }
+// second CTA over the same keys would repeat the lookups too); groups above eight heads are cut into eights.  Short calls,
+// where a CTA's latency counts, take fours unless eights come out even (14 query / 2 kv heads of 128, 200 tokens: eights
+// 10.6 us, fours 8.5, the general kernel 9.8).
+static int bridge_heads(int gqa, int S) {
+    if (gqa >= 5) return gqa % 8 && S <= 512 ? 4 : 8;
+    return gqa >= 3 ? 4 : gqa;
+}
 
 int bridge_attention_plan(BridgeAttnParams& p, int total_kv_heads, int sms, size_t ws_floats, int ws_tickets,
                           int total_q_heads) {
-    const int G = bridge_heads(p.gqa), groups = (p.gqa + G - 1) / G;
+    const int G = bridge_heads(p.gqa, p.S), groups = (p.gqa + G - 1) / G;
     const int n_tiles = (p.S + kBaTile - 1) / kBaTile, rows = total_kv_heads * groups;
     // one CTA per SM; a slice has at least four tiles (four warps already keep an SM's schedulers busy, and a tile takes
     // an SM 250 cycles of issue, about what merging one more slice costs)
@@ -450,7 +455,7 @@ static cudaError_t launch_bridge(const BridgeAttnParams& p, int total_kv_heads, 
 }
 
 cudaError_t bridge_attention_launch(const BridgeAttnParams& p, int total_kv_heads, int groups, cudaStream_t st) {
-    const int G = bridge_heads(p.gqa);
+    const int G = bridge_heads(p.gqa, p.S);
 #define PQ_BA(DD, GG) if (p.D == DD && G == GG) return launch_bridge<DD, GG>(p, total_kv_heads, groups, st);
     PQ_BA(128, 1) PQ_BA(128, 2) PQ_BA(128, 4) PQ_BA(128, 8)
     PQ_BA(64, 1) PQ_BA(64, 2) PQ_BA(64, 4) PQ_BA(64, 8)

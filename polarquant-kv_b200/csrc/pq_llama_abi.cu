@@ -642,6 +642,15 @@ __global__ void __launch_bounds__(kAttWarps * 32, 3) attention_kernel(const Attn
     }
 }
 
+// Whether pq_bridge_attn.cu serves the call.  Its CTA has an SM to itself, so very many heads over a tile or two of tokens
+// are left to the general kernel, more so while its three CTAs per SM hold all of them (512 kv heads of 64, 33 tokens: 10.8 us,
+// general 9.8; of 128 12.0 and 12.5; 320 of 128 9.2 and 7.2).
+bool tuned_attention(const AttnParams& p, int total_kv_heads, const void* packed_k, const void* packed_v) {
+    const int sms = device_sms();
+    const long long little = total_kv_heads <= 2 * sms ? 0 : total_kv_heads <= 3 * sms ? 8192 : 4096;
+    return pq::bridge_attention_fits(p.D, packed_k, packed_v) && (long long)p.S * p.D > little;
+}
+
 // How a call is cut: which kernel, and over how many slices (p.n_split, p.tiles_per_split).
 struct AttnPlan {
     bool tuned;               // pq_bridge_attn.cu
@@ -806,9 +815,9 @@ size_t polarquant_fused_attention_ws_bytes_c(int total_q_heads, int total_kv_hea
     if (total_q_heads <= 0 || total_kv_heads <= 0 || total_q_heads % total_kv_heads || S <= 0 || !dim_ok(D)) return 0;
     size_t floats = 0;
     for (const bool tuned : {false, true}) {                   // which of the two depends on the buffers' alignment
-        if (tuned && !pq::bridge_attention_fits(D, nullptr, nullptr)) continue;
         AttnParams p{};
         p.gqa = total_q_heads / total_kv_heads; p.S = S; p.D = D;
+        if (tuned && !tuned_attention(p, total_kv_heads, nullptr, nullptr)) continue;
         const AttnPlan a = plan_attention(p, tuned, total_q_heads, total_kv_heads, device_sms(), kWsFloats);
         if (p.n_split > 1) floats = std::max(floats, (size_t)p.n_split * total_q_heads * ((tuned ? D : 32 * a.DPL) + 2));
     }
@@ -840,7 +849,7 @@ void polarquant_fused_attention_ws_cuda_c(const float* q_rotated, const uint8_t*
 
     // Head dims 64 and 128 on 16-byte boundaries (the bridge's own buffers are) have a kernel of their own.  It masks
     // indices with n_levels - 1 like the general one, so other table sizes than powers of two behave alike.
-    const bool tuned = pq::bridge_attention_fits(D, packed_k, packed_v) && (reinterpret_cast<uintptr_t>(q_rotated) & 7) == 0;
+    const bool tuned = tuned_attention(p, total_kv_heads, packed_k, packed_v) && (reinterpret_cast<uintptr_t>(q_rotated) & 7) == 0;
     size_t floats = kWsFloats;
     if (ws) floats = ws_bytes <= kWsCounterBytes ? 0 : std::min(kWsFloats, (ws_bytes - kWsCounterBytes) / sizeof(float));
     const AttnPlan a = plan_attention(p, tuned, total_q_heads, total_kv_heads, device_sms(), floats);

@@ -214,7 +214,8 @@ def test_compress_tensor_core_edges_vs_oracle(d, n, book):
 
 # edges of the kernel for head dims 64 and 128: every group width (missing heads masked), tiles of one token, slices
 @pytest.mark.parametrize("hq,hkv,s", [(1, 1, 31), (2, 2, 32), (6, 3, 129), (3, 1, 64), (7, 1, 1000), (10, 2, 513),
-                                      (20, 1, 300), (5, 5, 4099), (2, 1, 70_001)])
+                                      (20, 1, 300), (5, 5, 4099), (2, 1, 70_001),
+                                      (14, 2, 512), (14, 2, 513), (9, 1, 200), (40, 8, 1), (700, 700, 32), (700, 350, 64), (700, 350, 65), (700, 700, 65)])
 @pytest.mark.parametrize("d", [64, 128])
 def test_fused_attention_group_widths_vs_oracle(hq, hkv, s, d):
     from polarquant_kv import _ext
